@@ -98,14 +98,38 @@ extern "C" int blaze_db_create(int device, const uint8_t *residues, const uint64
             rc = BLAZE_ERR_CUDA;
         }
     } while (false);
+    if (rc == BLAZE_OK) {
+        db->h_off.swap(off);
+        rc = db_make_groups(db);
+    }
     if (rc != BLAZE_OK) {
         blaze_db_free(db);
         return rc;
     }
-    db->h_off.swap(off);
     *out = db;
     return BLAZE_OK;
 } BLAZE_ABI_CATCH
+
+int db_make_groups(blaze_db *db) {
+    const std::vector<uint64_t> &off = db->h_off;
+    // at least 16 groups for each of the 152 x 32 warps of a scan, so that they
+    // end about together (256 queries against 35 M residues: 185.5 ms, and
+    // 189.6 with 4)
+    constexpr uint64_t kGroups = 16ull * 152 * 32;
+    const uint64_t most = std::min<uint64_t>(db->total / kGroups, kGroupMaxResidues);
+    db->group_residues = static_cast<uint32_t>(most);
+    std::vector<uint32_t> &b = db->h_groups;
+    b.assign(1, db->n);
+    for (uint32_t hi = db->n; hi > 0;) {
+        uint32_t lo = hi - 1;
+        while (lo > 0 && hi - lo < kGroupMaxSubjects && off[hi] - off[lo - 1] <= most) --lo;
+        b.push_back(lo);
+        hi = lo;
+    }
+    BLAZE_CUDA_TRY(cudaMalloc(&db->d_groups, sizeof(uint32_t) * b.size()));
+    BLAZE_CUDA_TRY(cudaMemcpy(db->d_groups, b.data(), sizeof(uint32_t) * b.size(), cudaMemcpyHostToDevice));
+    return BLAZE_OK;
+}
 
 extern "C" int blaze_db_free(blaze_db *db) {
     if (!db) return BLAZE_OK;
@@ -113,6 +137,7 @@ extern "C" int blaze_db_free(blaze_db *db) {
     if (db->d_res) cudaFree(db->d_res);
     if (db->d_off) cudaFree(db->d_off);
     if (db->d_oid) cudaFree(db->d_oid);
+    if (db->d_groups) cudaFree(db->d_groups);
     delete db;
     return BLAZE_OK;
 }
@@ -334,6 +359,7 @@ struct ScanLaunch {
     int blocks, warps_per_block;
     size_t smem_bytes;
     bool tiles;  // the batched (tiled) kernel, else the single-query one
+    bool word_table;
 };
 
 struct PassLaunch {
@@ -358,7 +384,7 @@ static cudaError_t enqueue_pass(blaze_search *s, const PassLaunch &pl, unsigned 
     for (const ScanLaunch &l : pl.scans) {
         if (e != cudaSuccess) break;
         e = l.tiles ? launch_scan_batch(l.sa, l.blocks, l.warps_per_block, l.smem_bytes, s->stream)
-                       : launch_scan(l.sa, l.blocks, l.warps_per_block, l.smem_bytes, s->stream);
+                       : launch_scan(l.sa, l.word_table, l.blocks, l.warps_per_block, l.smem_bytes, s->stream);
     }
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(s->ev[2], s->stream, event_flags);
     if (e == cudaSuccess)
@@ -392,7 +418,7 @@ static int launch_pass_graph(blaze_search *s, const PassLaunch &pl) {
     put(head, sizeof(head));
     for (const ScanLaunch &l : pl.scans) {
         put(&l.sa, sizeof(ScanArgs));
-        const int64_t shape[3] = {l.blocks, l.warps_per_block, static_cast<int64_t>(l.smem_bytes)};
+        const int64_t shape[4] = {l.blocks, l.warps_per_block, static_cast<int64_t>(l.smem_bytes), l.word_table};
         put(shape, sizeof(shape));
     }
     put(pl.ga, sizeof(GappedArgs));
@@ -447,20 +473,20 @@ struct ScanPlan {
     bool tiles = false;  // batched: tiles of the plan's queries; else one query's launch
 };
 
-// Subject ranges of about `target` residues, from the longest subjects down
-// (bounds descending, n_ranges + 1 of them), uploaded once per tile size.
+// Ranges of groups of about `target` residues, from the longest subjects
+// down (n_ranges + 1 bounds), uploaded once per tile size.
 static int tile_bounds_for(blaze_search *s, uint32_t target, const uint32_t **bounds, uint32_t *n_ranges) {
     auto it = s->tile_bounds.find(target);
     if (it == s->tile_bounds.end()) {
         const std::vector<uint64_t> &off = s->db->h_off;
-        const uint32_t n = s->db->n;
-        std::vector<uint32_t> b{n};
-        for (uint32_t hi = n; hi > 0;) {
-            const uint64_t want = off[hi] > target ? off[hi] - target : 0;
-            uint32_t lo = static_cast<uint32_t>(std::lower_bound(off.begin(), off.begin() + hi, want) - off.begin());
-            if (lo >= hi) lo = hi - 1;
-            b.push_back(lo);
-            hi = lo;
+        const std::vector<uint32_t> &groups = s->db->h_groups;
+        const uint32_t n = static_cast<uint32_t>(groups.size()) - 1;
+        std::vector<uint32_t> b{0};
+        for (uint32_t lo = 0; lo < n;) {
+            uint32_t hi = lo + 1;
+            while (hi < n && off[groups[lo]] - off[groups[hi + 1]] <= target) ++hi;
+            b.push_back(hi);
+            lo = hi;
         }
         DevBuf<uint32_t> d;
         int rc = d.ensure(b.size());
@@ -520,18 +546,19 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
         ScanLaunch l;
         ScanArgs &sa = l.sa;
         std::memset(&sa, 0, sizeof(sa));  // whole bytes: the graph key compares them
+        l.word_table = lay.word_table;
         l.blocks = plan.blocks;
         l.warps_per_block = lay.warps_per_block;
         l.smem_bytes = lay.smem_bytes;
         sa.res = db->d_res;
         sa.off = db->d_off;
-        sa.n_subj = db->n;
+        sa.groups = db->d_groups;
+        sa.n_groups = static_cast<uint32_t>(db->h_groups.size()) - 1;
         sa.window = p->window;
         sa.xdrop = p->ungapped_xdrop;
         sa.diag_entries = lay.diag_entries;
         sa.diag_magic = lay.diag_magic;
         sa.diag_bytes = lay.diag_bytes;
-        sa.diag_entries_max = lay.diag_entries;
         sa.stage_bytes = lay.stage_bytes;
         sa.query_smem_bytes = lay.query_smem_bytes;
         sa.warp_smem_bytes = lay.warp_smem_bytes;
@@ -665,11 +692,17 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     constexpr size_t kSmemBudget = 220 * 1024;
     const int reg_cap = batched ? std::min(scan_batch_max_warps_by_registers(true),
                                            scan_batch_max_warps_by_registers(false))
-                                : scan_max_warps_by_registers(r.q->qlen <= static_cast<int32_t>(kQuerySmemMax));
+                                : scan_max_warps_by_registers(scan_query_in_smem(r.q->qlen, p0->window));
     const int warp_cap = s->max_warps ? std::min(reg_cap, static_cast<int>(s->max_warps)) : reg_cap;
     // layout of one single-query scan launch
-    auto layout_for = [&](int32_t max_qlen) {
-        return scan_layout(max_qlen, p0->window, s->stage_bytes, kSmemBudget, warp_cap);
+    const uint32_t stage_bytes = std::max(s->stage_bytes, db->group_residues);
+    constexpr size_t kSmemMost = 227 * 1024 - 64;  // the opt-in limit less static shared memory
+    auto layout_for = [&](int32_t qlen, uint32_t n_hits) {
+        ScanLayout l = scan_layout(qlen, p0->window, n_hits, stage_bytes, kSmemBudget, warp_cap);
+        // next to the longest tables only smaller groups are staged
+        if (l.smem_bytes > kSmemMost)
+            l = scan_layout(qlen, p0->window, n_hits, std::max(s->stage_bytes, 160u) - 160u, kSmemBudget, warp_cap);
+        return l;
     };
     // layout of one batched scan launch over queries of up to `longest`
     // residues: shared memory for all the block's warps at the longest query
@@ -677,22 +710,19 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     // each tile runs as many warps as fit for its own query
     auto batch_layout_for = [&](int32_t longest) {
         ScanLayout l{};
-        const uint32_t stage_region = (s->stage_bytes + 32u + 15u) & ~15u;
         auto warp_bytes = [&](int32_t qlen) {
-            const uint32_t e = static_cast<uint32_t>(qlen + p0->window + 3) & ~3u;
-            return static_cast<size_t>(((4u * e + 15u) & ~15u) + 2u * kDeferCap * sizeof(uint2) +
-                                       kSeedCap * sizeof(int4) + stage_region);
+            return static_cast<size_t>(scan_warp_bytes(scan_diag_bytes(qlen, p0->window), stage_bytes));
         };
         const int w = std::max(1, std::min(warp_cap, kScanMaxWarpsPerBlock));
-        l.query_smem_bytes = longest <= kQuerySmemMax ? (static_cast<uint32_t>(longest) + 15u) & ~15u : 0u;
-        const size_t regions = kScanMatBytes + kScanPresenceBytes + l.query_smem_bytes + 16u * static_cast<size_t>(w);
+        l.query_smem_bytes = scan_query_in_smem(longest, p0->window) ? (static_cast<uint32_t>(longest) + 15u) & ~15u : 0u;
+        const size_t regions = kScanMatBytes + kScanPresenceBytes + l.query_smem_bytes + kScanSlackBytes;
         l.smem_bytes = std::max(std::min(kSmemBudget, regions + static_cast<size_t>(w) * warp_bytes(longest)),
                                 regions + warp_bytes(longest));
         l.warps_per_block = w;
-        l.stage_bytes = s->stage_bytes;
-        l.diag_entries = static_cast<uint32_t>(longest + p0->window + 3) & ~3u;
+        l.stage_bytes = stage_bytes;
+        l.diag_entries = scan_diag_entries(longest, p0->window);
         l.diag_magic = static_cast<uint32_t>((1ull << 32) / l.diag_entries + 1);
-        l.diag_bytes = 4u * l.diag_entries;
+        l.diag_bytes = scan_diag_bytes(longest, p0->window);
         l.warp_smem_bytes = static_cast<uint32_t>(warp_bytes(longest));
         return l;
     };
@@ -716,7 +746,7 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
         const size_t need = batch_layout_for(qlen).smem_bytes;
         int k = 0;
         while (k < 4 && need > kSteps[k]) ++k;
-        return k + (qlen > kQuerySmemMax ? 8 : 0);  // longer queries stay in global memory: own launch
+        return k + (scan_query_in_smem(qlen, p0->window) ? 0 : 8);  // longer queries stay in global memory: own launch
     };
     // batched runs of few queries, or on a large database, launch the
     // single-query kernel once per query (a query alone fills the GPU there,
@@ -736,16 +766,17 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
         }
         ScanPlan pl;
         pl.tiles = batched && !per_query;
-        pl.lay = pl.tiles ? batch_layout_for(qlen_at(j - 1)) : layout_for(qlen_at(j - 1));
+        pl.lay = pl.tiles ? batch_layout_for(qlen_at(j - 1)) : layout_for(qlen_at(i), batched ? r.b->n_off[order[i]] : r.q->n_off);
         pl.first = i;
         pl.n = j - i;
-        if (pl.lay.smem_bytes > 227 * 1024 - 64) return BLAZE_ERR_LIMIT;  // the opt-in limit less static shared memory
+        if (pl.lay.smem_bytes > kSmemMost) return BLAZE_ERR_LIMIT;
         int per_sm = 0;
         if (pl.tiles) {
             BLAZE_CUDA_TRY(scan_batch_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.warps_per_block, pl.lay.smem_bytes,
                                                 &per_sm));
         } else {
-            BLAZE_CUDA_TRY(scan_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.warps_per_block, pl.lay.smem_bytes, &per_sm));
+            BLAZE_CUDA_TRY(scan_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.word_table, pl.lay.warps_per_block,
+                                          pl.lay.smem_bytes, &per_sm));
         }
         if (per_sm < 1) return BLAZE_ERR_LIMIT;
         pl.blocks = s->n_sm * per_sm;
@@ -787,8 +818,9 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
             d.cell_pack = r.b->d_cell_pack + static_cast<size_t>(i) * kWords;
             d.presence = r.b->d_presence + static_cast<size_t>(i) * kPresenceWords;
             d.cell_off = r.b->d_cell_off + r.b->off_off[i];
-            d.diag_entries = static_cast<uint32_t>(d.qlen + pi.window + 3) & ~3u;
+            d.diag_entries = scan_diag_entries(d.qlen, pi.window);
             d.diag_magic = static_cast<uint32_t>((1ull << 32) / d.diag_entries + 1);
+            d.diag_bytes = scan_diag_bytes(d.qlen, pi.window);
             d.index = i;
             qp[i] = d.q;
             ql[i] = d.qlen;
@@ -961,7 +993,7 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     s->last_work_count = c.work_count;
     s->last_batched = batched;
     s->last_batch = r.b;
-    s->stats.residues_scanned = c.residues;
+    s->stats.residues_scanned = db->total * nq;
     s->stats.word_hits = c.word_hits;
     s->stats.ungapped_extensions = c.extensions;
     s->stats.init_hsps = c.init_count;

@@ -30,6 +30,7 @@ static int batch_fill(blaze_batch *b, const uint8_t *residues, const uint64_t *o
     b->qlen.clear();
     b->res_off.clear();
     b->off_off.clear();
+    b->n_off.clear();
     std::vector<uint8_t> res;
     std::vector<uint32_t> cs_all(static_cast<size_t>(n_queries) * (kWords + 1));
     std::vector<uint32_t> pack_all(static_cast<size_t>(n_queries) * kWords);
@@ -48,6 +49,7 @@ static int batch_fill(blaze_batch *b, const uint8_t *residues, const uint64_t *o
         int rc = build_lookup(q, len, word_threshold, cs, &offs, &n_off);
         if (rc != BLAZE_OK) return rc;
         b->off_off.push_back(offs_all.size());
+        b->n_off.push_back(n_off);
         offs_all.insert(offs_all.end(), offs, offs + n_off);
         std::free(offs);
         pack_word_cells(cs, pack_all.data() + static_cast<size_t>(i) * kWords,

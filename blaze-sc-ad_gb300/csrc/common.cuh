@@ -20,14 +20,37 @@ constexpr int kWarp = 32;
 // Word-finder tuning (per warp of the scan kernel).
 constexpr int kDeferCap = 64;   // deferred hits per buffer (two buffers)
 constexpr int kSeedCap = 64;    // queued two-hit seeds (>= kDeferCap)
+constexpr int kChunk = 128;     // subject positions a warp looks up at a time
+// a warp's region up to its diagonal table: mbarrier, deferred hits (two
+// buffers), seeds, the chunk's words with hits
+constexpr uint32_t kScanWarpFixedBytes = 16 + 2 * kDeferCap * 4 + kSeedCap * 8 + kChunk * 8;
+constexpr uint32_t kScanSlackBytes = 144;  // a chunk's reads run past its subject, never past this
+// A group: consecutive subjects that one warp stages and scans together.
+constexpr uint32_t kGroupMaxSubjects = 31;    // their bounds are one per lane, with the end
+constexpr uint32_t kGroupMaxResidues = 2032;  // of a group of several subjects
+__host__ __device__ constexpr uint32_t scan_stage_region(uint32_t stage_bytes) { return (stage_bytes + 32u + 15u) & ~15u; }
 constexpr int kScanMaxWarpsPerBlock = 32;
 constexpr int kGappedWarpsPerBlock = 4;
 constexpr int kPresenceWords = (kWords + 31) / 32;                     // 686
 constexpr size_t kScanMatBytes = kAlphabet * kAlphabet;               // int8 matrix, 784
 constexpr size_t kScanPresenceBytes = (kPresenceWords * 4 + 15) & ~15; // 2752
-constexpr int32_t kQuerySmemMax = 8192;      // queries up to this length live in shared memory
+constexpr size_t kScanWordTabBytes = ((kWords + 1) * 2 + 15) & ~15;    // 43,920
+constexpr uint32_t kScanWordTabHits = 65535;  // hit-list entries a 16-bit word table can number
+constexpr int32_t kQuerySmemMax = 8192;      // queries up to this length live in shared memory,
+constexpr int32_t kTab16Window = 256;        // for windows up to this one: 16-bit diagonal tables
 constexpr uint32_t kScanStageBytes = 1024;   // subjects up to this length are staged
 constexpr uint32_t kMaxTileResidues = 1u << 16;  // automatic tile size at most (residues per warp)
+
+inline bool scan_query_in_smem(int32_t qlen, int32_t window) { return qlen <= kQuerySmemMax && window <= kTab16Window; }
+inline uint32_t scan_diag_entries(int32_t qlen, int32_t window) {  // >= qlen + window
+    return static_cast<uint32_t>(qlen + window + 3) & ~3u;
+}
+inline uint32_t scan_diag_bytes(int32_t qlen, int32_t window) {
+    return (scan_diag_entries(qlen, window) * (scan_query_in_smem(qlen, window) ? 2u : 4u) + 15u) & ~15u;
+}
+__host__ __device__ constexpr uint32_t scan_warp_bytes(uint32_t diag_bytes, uint32_t stage_bytes) {
+    return kScanWarpFixedBytes + diag_bytes + scan_stage_region(stage_bytes);
+}
 
 // An ungapped HSP that reached the ungapped cutoff (NCBI BlastInitHSP analog).
 struct InitHit {
@@ -69,7 +92,6 @@ struct DevCounters {
     unsigned long long extensions;
     unsigned long long gapped_ext;
     unsigned long long dp_cells;
-    unsigned long long residues;
     unsigned int overflow_subjects;  // subjects whose init hits exceeded the per-warp scratch
     unsigned int max_init_needed;    // largest init-hit count among those
     unsigned int flags;              // kFlag* bits
@@ -107,14 +129,15 @@ struct BatchQuery {
     int32_t ungapped_cutoff;
     const uint32_t *cell_start, *cell_pack, *presence;
     const uint16_t *cell_off;
-    uint32_t diag_entries, diag_magic;
+    uint32_t diag_entries, diag_magic, diag_bytes;
     uint32_t index;  // position of the query in its batch
 };
 
 struct ScanArgs {
     const uint8_t *res;        // residues, length-sorted subjects
     const uint64_t *off;       // n_subj + 1 offsets
-    uint32_t n_subj;
+    const uint32_t *groups;    // n_groups + 1 subject indices, descending: group g is [groups[g+1], groups[g])
+    uint32_t n_groups;
     const uint8_t *q;          // query residues
     int32_t qlen;
     const uint32_t *cell_start;  // kWords + 1
@@ -125,12 +148,11 @@ struct ScanArgs {
     uint32_t diag_entries;       // >= qlen + window
     uint32_t diag_magic;         // floor(2^32 / diag_entries) + 1
     uint32_t diag_bytes, stage_bytes, query_smem_bytes, warp_smem_bytes;
-    uint32_t diag_entries_max;   // largest table any query of the launch uses
     uint32_t smem_bytes;         // batched launches: dynamic shared memory of a block
     // batched launches only
     const BatchQuery *queries;   // n_queries descriptors
     uint32_t n_queries;
-    const uint32_t *tile_bounds;  // n_ranges + 1 subject indices, descending: range r is [b[r+1], b[r])
+    const uint32_t *tile_bounds;  // n_ranges + 1 group indices, ascending: range r is [b[r], b[r+1])
     uint32_t n_ranges;
     uint32_t *work_query;        // query index of each work item (nullptr: one query)
     uint32_t query_index;        // single-query launches inside a batched pass: the query's index
@@ -197,6 +219,7 @@ struct HitlistArgs {
 // Shared-memory layout of the scan kernel for one query.
 struct ScanLayout {
     uint32_t diag_entries, diag_magic, diag_bytes, stage_bytes, query_smem_bytes, warp_smem_bytes;
+    bool word_table;  // the 16-bit word table in shared memory instead of the presence bitset
     int warps_per_block;
     size_t smem_bytes;
 };
@@ -236,9 +259,10 @@ struct TracebackArgs {
 };
 
 // Launchers (scan.cu, kernels.cu, traceback.cu).
-ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t stage_bytes, size_t smem_budget, int max_warps);
-cudaError_t launch_scan(const ScanArgs &a, int n_blocks, int warps_per_block, size_t smem, cudaStream_t st);
-cudaError_t scan_occupancy(bool query_in_smem, int warps_per_block, size_t smem, int *blocks_per_sm);
+ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t n_hits, uint32_t stage_bytes, size_t smem_budget, int max_warps);
+cudaError_t launch_scan(const ScanArgs &a, bool word_table, int n_blocks, int warps_per_block, size_t smem,
+                        cudaStream_t st);
+cudaError_t scan_occupancy(bool query_in_smem, bool word_table, int warps_per_block, size_t smem, int *blocks_per_sm);
 int scan_max_warps_by_registers(bool query_in_smem);
 cudaError_t launch_gapped(const GappedArgs &a, int n_blocks, cudaStream_t st,
                           int warps_per_block = kGappedWarpsPerBlock);

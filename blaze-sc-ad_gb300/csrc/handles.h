@@ -27,7 +27,15 @@ struct blaze_db {
     std::vector<uint32_t> oid_of;  // sorted index -> OID
     std::vector<uint32_t> sorted_of;  // OID -> sorted index
     std::vector<uint64_t> h_off;   // offsets of the length-sorted copy (host)
+    // the word finder's groups, from the longest subjects down (ScanArgs::groups)
+    std::vector<uint32_t> h_groups;
+    uint32_t *d_groups = nullptr;
+    uint32_t group_residues = 0;   // the most a group of several subjects holds
 };
+
+// Cuts the length-sorted database into groups of consecutive subjects and
+// uploads their bounds (h_off must be set).
+int db_make_groups(blaze_db *db);
 
 struct blaze_query {
     int device = 0;
@@ -139,6 +147,7 @@ struct blaze_batch {
     int32_t threshold = 0;
     std::vector<int32_t> qlen;
     std::vector<uint64_t> res_off, off_off;  // per query: residues, hit lists
+    std::vector<uint32_t> n_off;             // per query: entries of its hit lists
     // device tables; a refilled batch keeps them while they are large enough
     DevBuf<uint8_t> res;
     DevBuf<uint32_t> cell_start, cell_pack, presence;

@@ -210,11 +210,14 @@ extern "C" int blaze_db_create_from_source(int device, const blaze_seq_source *s
         }
     } while (false);
     if (st) cudaStreamDestroy(st);
+    if (rc == BLAZE_OK) {
+        db->h_off.swap(off);
+        rc = db_make_groups(db);
+    }
     if (rc != BLAZE_OK) {
         blaze_db_free(db);
         return rc;
     }
-    db->h_off.swap(off);
     *out = db;
     return BLAZE_OK;
 } BLAZE_ABI_CATCH
