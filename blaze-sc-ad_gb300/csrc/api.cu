@@ -116,13 +116,15 @@ int db_make_groups(blaze_db *db) {
     // end about together (256 queries against 35 M residues: 185.5 ms, and
     // 189.6 with 4)
     constexpr uint64_t kGroups = 16ull * 152 * 32;
-    const uint64_t most = std::min<uint64_t>(db->total / kGroups, kGroupMaxResidues);
-    db->group_residues = static_cast<uint32_t>(most);
+    const uint64_t most = std::min<uint64_t>(db->total / kGroups, kGroupMaxBytes);
+    db->group_bytes = static_cast<uint32_t>(most);
     std::vector<uint32_t> &b = db->h_groups;
     b.assign(1, db->n);
     for (uint32_t hi = db->n; hi > 0;) {
         uint32_t lo = hi - 1;
-        while (lo > 0 && hi - lo < kGroupMaxSubjects && off[hi] - off[lo - 1] <= most) --lo;
+        while (lo > 0 && hi - lo < kGroupMaxSubjects &&
+               off[hi] - off[lo - 1] + kGroupSubjectBytes * (hi - lo + 1) <= most)
+            --lo;
         b.push_back(lo);
         hi = lo;
     }
@@ -695,7 +697,7 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
                                 : scan_max_warps_by_registers(scan_query_in_smem(r.q->qlen, p0->window));
     const int warp_cap = s->max_warps ? std::min(reg_cap, static_cast<int>(s->max_warps)) : reg_cap;
     // layout of one single-query scan launch
-    const uint32_t stage_bytes = std::max(s->stage_bytes, db->group_residues);
+    const uint32_t stage_bytes = std::max(s->stage_bytes, db->group_bytes);
     constexpr size_t kSmemMost = 227 * 1024 - 64;  // the opt-in limit less static shared memory
     auto layout_for = [&](int32_t qlen, uint32_t n_hits) {
         ScanLayout l = scan_layout(qlen, p0->window, n_hits, stage_bytes, kSmemBudget, warp_cap);
@@ -715,7 +717,7 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
         };
         const int w = std::max(1, std::min(warp_cap, kScanMaxWarpsPerBlock));
         l.query_smem_bytes = scan_query_in_smem(longest, p0->window) ? (static_cast<uint32_t>(longest) + 15u) & ~15u : 0u;
-        const size_t regions = kScanMatBytes + kScanPresenceBytes + l.query_smem_bytes + kScanSlackBytes;
+        const size_t regions = kScanMatBytes + kScanPresenceBytes + l.query_smem_bytes;
         l.smem_bytes = std::max(std::min(kSmemBudget, regions + static_cast<size_t>(w) * warp_bytes(longest)),
                                 regions + warp_bytes(longest));
         l.warps_per_block = w;

@@ -22,17 +22,18 @@ constexpr int kDeferCap = 64;   // deferred hits per buffer (two buffers)
 constexpr int kSeedCap = 64;    // queued two-hit seeds (>= kDeferCap)
 constexpr int kChunk = 128;     // subject positions a warp looks up at a time
 // a warp's region up to its diagonal table: mbarrier, deferred hits (two
-// buffers), seeds, the chunk's words with hits
-constexpr uint32_t kScanWarpFixedBytes = 16 + 2 * kDeferCap * 4 + kSeedCap * 8 + kChunk * 8;
-constexpr uint32_t kScanSlackBytes = 144;  // a chunk's reads run past its subject, never past this
+// buffers), seeds, words with hits
+constexpr uint32_t kScanWarpFixedBytes = 16 + 2 * kDeferCap * 4 + kSeedCap * 8 + (kChunk + 32) * 8;
+constexpr uint32_t kScanStageSlack = 144;  // zeros behind the staged subjects: a chunk's reads end there
 // A group: consecutive subjects that one warp stages and scans together.
 constexpr uint32_t kGroupMaxSubjects = 31;    // their bounds are one per lane, with the end
-constexpr uint32_t kGroupMaxResidues = 2032;  // of a group of several subjects
-__host__ __device__ constexpr uint32_t scan_stage_region(uint32_t stage_bytes) { return (stage_bytes + 32u + 15u) & ~15u; }
+constexpr uint32_t kGroupSubjectBytes = 32;   // of a subject's block beyond its residues, at most
+constexpr uint32_t kGroupMaxBytes = 2240;     // of the blocks of a group of several subjects
+__host__ __device__ constexpr uint32_t scan_stage_blocks(uint32_t stage_bytes) { return (stage_bytes + 32u + 15u) & ~15u; }
 constexpr int kScanMaxWarpsPerBlock = 32;
 constexpr int kGappedWarpsPerBlock = 4;
 constexpr int kPresenceWords = (kWords + 31) / 32;                     // 686
-constexpr size_t kScanMatBytes = kAlphabet * kAlphabet;               // int8 matrix, 784
+constexpr size_t kScanMatBytes = kAlphabet * kAlphabet * 4;           // matrix, 3,136
 constexpr size_t kScanPresenceBytes = (kPresenceWords * 4 + 15) & ~15; // 2752
 constexpr size_t kScanWordTabBytes = ((kWords + 1) * 2 + 15) & ~15;    // 43,920
 constexpr uint32_t kScanWordTabHits = 65535;  // hit-list entries a 16-bit word table can number
@@ -49,7 +50,7 @@ inline uint32_t scan_diag_bytes(int32_t qlen, int32_t window) {
     return (scan_diag_entries(qlen, window) * (scan_query_in_smem(qlen, window) ? 2u : 4u) + 15u) & ~15u;
 }
 __host__ __device__ constexpr uint32_t scan_warp_bytes(uint32_t diag_bytes, uint32_t stage_bytes) {
-    return kScanWarpFixedBytes + diag_bytes + scan_stage_region(stage_bytes);
+    return kScanWarpFixedBytes + diag_bytes + scan_stage_blocks(stage_bytes) + kScanStageSlack;
 }
 
 // An ungapped HSP that reached the ungapped cutoff (NCBI BlastInitHSP analog).

@@ -30,7 +30,7 @@ struct blaze_db {
     // the word finder's groups, from the longest subjects down (ScanArgs::groups)
     std::vector<uint32_t> h_groups;
     uint32_t *d_groups = nullptr;
-    uint32_t group_residues = 0;   // the most a group of several subjects holds
+    uint32_t group_bytes = 0;      // the most that the blocks of a group of several subjects take
 };
 
 // Cuts the length-sorted database into groups of consecutive subjects and

@@ -29,12 +29,8 @@ __device__ const int8_t g_blosum8[kAlphabet * kAlphabet] = {
 };
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kCoopSeeds = 4;  // flushes with at most this many seeds extend warp-cooperatively
-__device__ __forceinline__ unsigned lanemask_lt() {
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
+__device__ __forceinline__ unsigned lanemask_lt() { return (1u << (threadIdx.x & 31u)) - 1u; }
+__device__ __forceinline__ unsigned lanemask_le() { return 0xffffffffu >> (31u - (threadIdx.x & 31u)); }
 
 // idx mod L for idx < 2^32, with magic = floor(2^32 / L) + 1: the estimated
 // quotient is the true one or one more.
@@ -57,8 +53,8 @@ constexpr uint32_t kQueryOff = kTabOff + (WT ? kScanWordTabBytes : kScanPresence
 constexpr uint32_t kBarAt = 0;                                // the stage buffer's mbarrier
 constexpr uint32_t kDeferAt = 16;                             // two buffers of deferred hits
 constexpr uint32_t kSeedAt = kDeferAt + 2 * kDeferCap * 4;    // queued seeds
-constexpr uint32_t kListAt = kSeedAt + kSeedCap * 8;          // the chunk's words with hits
-constexpr uint32_t kDiagAt = kListAt + kChunk * 8;            // diagonal table, then the stage buffer
+constexpr uint32_t kListAt = kSeedAt + kSeedCap * 8;          // words with hits: the chunk's, and those waiting
+constexpr uint32_t kDiagAt = kListAt + (kChunk + 32) * 8;     // diagonal table, then the stage buffer
 static_assert(kDiagAt == kScanWarpFixedBytes, "a warp's region");
 
 extern __shared__ __align__(16) unsigned char smem[];
@@ -68,13 +64,23 @@ __device__ __forceinline__ uint32_t lds32(uint32_t off) { return reinterpret_cas
 __device__ __forceinline__ void sts32(uint32_t off, uint32_t v) { reinterpret_cast<uint32_t *>(smem)[off >> 2] = v; }
 __device__ __forceinline__ uint2 lds64(uint32_t off) { return reinterpret_cast<const uint2 *>(smem)[off >> 3]; }
 __device__ __forceinline__ void sts64(uint32_t off, uint2 v) { reinterpret_cast<uint2 *>(smem)[off >> 3] = v; }
-__device__ __forceinline__ int32_t score_of(uint32_t qa, uint32_t sb) {
-    return static_cast<int32_t>(reinterpret_cast<const int8_t *>(smem)[kMatOff + qa * kAlphabet + sb]);
+// The matrix holds keys: the score times 2^14, less one. A walk that sums them
+// has 2^14 x (its score) - (its length), so the largest sum it passes gives the
+// best score and, among equals, the first position that reached it.
+constexpr int kKeyBits = 14;
+constexpr int32_t kKeyMask = (1 << kKeyBits) - 1;
+constexpr int32_t kKeyedLength = 11900;  // of a walk: 11 x its length times 2^14 stays below 2^31
+static_assert(kQuerySmemMax <= kKeyedLength, "walks on keys");
+__device__ __forceinline__ int32_t key_of(uint32_t qa, uint32_t sb) {
+    return reinterpret_cast<const int32_t *>(smem + kMatOff)[qa * kAlphabet + sb];
 }
+__device__ __forceinline__ int32_t score_of(uint32_t qa, uint32_t sb) { return (key_of(qa, sb) + 1) >> kKeyBits; }
+__device__ __forceinline__ int32_t key_score(int32_t k) { return (k + kKeyMask) >> kKeyBits; }
+__device__ __forceinline__ int32_t key_length(int32_t k) { return (0 - k) & kKeyMask; }
 
 // ------------------------------------------------------------------------
-// Subject staging by the bulk-copy (TMA) engine: one elected lane arms the
-// warp's mbarrier with the byte count and issues cp.async.bulk
+// Staging by the bulk-copy (TMA) engine: one lane arms the warp's mbarrier
+// with the group's bytes, and each lane issues its subject's cp.async.bulk
 // global -> shared; the warp waits on the barrier's phase. A warp stages one
 // group at a time, just before scanning it, in one stage buffer. Waits are
 // bounded: a copy that never lands sets kFlagBadState.
@@ -101,25 +107,31 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0u;
 }
 
-// Lane 0 of the calling warp: copies `bytes` (a multiple of 16) from 16-byte
-// aligned global `src` to shared offset `dst` and completes the barrier.
+// Lane 0 of the calling warp: arms the barrier with the bytes to come.
+__device__ __forceinline__ void stage_expect(uint32_t bytes, uint32_t bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_base() + bar), "r"(bytes)
+                 : "memory");
+}
+
+// A lane copies `bytes` (a multiple of 16) from 16-byte aligned global `src`
+// to shared offset `dst`, reported to the barrier.
 __device__ __forceinline__ void bulk_stage(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     const uint32_t d = smem_base() + dst, b = smem_base() + bar;
-    // earlier generic reads of this buffer come before the async overwrite
+    // earlier generic accesses of this buffer come before the async overwrite
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(d), "l"(src), "r"(bytes), "r"(b)
                  : "memory");
 }
 
-// A group's residues, staged in shared memory, or read from global memory
-// when they are longer than the staging buffer. Positions (x) count from the
-// group's first residue.
+// A group's residues by position x: in the stage buffer, or, for a subject too
+// long for it, in global memory. In the stage buffer each subject begins in a
+// 16-byte block of its own, with zeros around it: no word with a zero letter
+// has a hit.
 template <bool STAGED>
 struct Span {
-    uint32_t off;        // shared offset of position 0 (staged)
-    const uint8_t *ptr;  // global address of position 0 (not staged)
+    uint32_t off;        // shared offset of x = 0 (staged)
+    const uint8_t *ptr;  // global address of x = 0 (not staged)
     __device__ __forceinline__ uint32_t at(int32_t x) const {
         if (STAGED) return smem[off + x];
         return __ldg(ptr + x);
@@ -186,6 +198,51 @@ __device__ __forceinline__ int32_t extend_right(const Q &q, const S &s, int32_t 
     return maxscore;
 }
 
+// The same walks on keys, for sequences of which one is at most kKeyedLength
+// long: one sum, one maximum and one comparison a position (139 M residues at
+// 300 query residues: 1.32 -> 1.29 ms).
+template <typename Q, typename S>
+__device__ __forceinline__ int32_t extend_two_hit_keyed(const Q &q, const S &s, int32_t s_left_off, int32_t s_off,
+                                                        int32_t q_off, int32_t xdrop, int32_t *hsp_q, int32_t *hsp_s,
+                                                        int32_t *hsp_len, int32_t *right_extend,
+                                                        int32_t *s_last_off) {
+    const int32_t drop = min(xdrop, (1 << (31 - kKeyBits)) - 1) << kKeyBits;
+    int32_t k = 0, m = 0;
+#pragma unroll
+    for (int32_t i = 0; i < kWordSize; ++i) {
+        k += key_of(q.at(q_off + i), s.at(s_off + i));
+        m = max(m, k);
+    }
+    const int32_t q_right = q_off + key_length(m), s_right = s_off + key_length(m);
+    k = m = 0;
+    for (int32_t i = 1, n = min(s_right, q_right); i <= n; ++i) {
+        k += key_of(q.at(q_right - i), s.at(s_right - i));
+        m = max(m, k);
+        if (m - k >= drop) break;
+    }
+    const int32_t left_d = key_length(m);
+    int32_t score = key_score(m), right_d = 0;
+    *right_extend = 0;
+    *s_last_off = s_right;
+    if (left_d >= s_right - s_left_off) {
+        *right_extend = 1;
+        k = m = score << kKeyBits;
+        int32_t i = 0;
+        for (const int32_t n = min(s.len - s_right, q.len - q_right); i < n; ++i) {
+            k += key_of(q.at(q_right + i), s.at(s_right + i));
+            m = max(m, k);
+            if (m - k >= drop || k <= 0) break;
+        }
+        right_d = key_length(m);
+        score = key_score(m);
+        *s_last_off = s_right + i;
+    }
+    *hsp_q = q_right - left_d;
+    *hsp_s = s_right - left_d;
+    *hsp_len = left_d + right_d;
+    return score;
+}
+
 template <typename Q, typename S>
 __device__ __forceinline__ int32_t extend_two_hit(const Q &q, const S &s,
                                                   int32_t s_left_off, int32_t s_off, int32_t q_off,
@@ -217,120 +274,23 @@ __device__ __forceinline__ int32_t extend_two_hit(const Q &q, const S &s,
 }
 
 // ------------------------------------------------------------------------
-// Warp-cooperative form of extend_two_hit for one seed: the 32 lanes take 32
-// consecutive positions of a walk per step. The running score is a prefix sum
-// and the running best a prefix maximum (carried between steps); the walk
-// stops at the first position whose stop test holds, and the best is the
-// first position reaching the final maximum -- exactly the positions and
-// scores of the sequential walk. Every lane returns the same values.
-
-// One X-drop walk of up to n positions; score and best start at `start`.
-// t(k) gives the score of the k-th position. Returns the best score; *best_k
-// is its position (-1 when never above start), *end the position the walk
-// stopped at (n when it ran out). right: also stop when the score drops to 0.
-template <bool RIGHT, typename F>
-__device__ __forceinline__ int32_t walk_warp(F t, int32_t n, int32_t start, int32_t xdrop, int32_t *best_k,
-                                             int32_t *end) {
-    const int lane = threadIdx.x & 31;
-    int32_t carry = start, cmax = start, bk = -1, stop_at = n;
-    for (int32_t base = 0; base < n; base += 32) {
-        const int32_t k = base + lane;
-        const bool valid = k < n;
-        int32_t S = valid ? t(k) : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t x = __shfl_up_sync(kFull, S, o);
-            if (lane >= o) S += x;
-        }
-        S += carry;
-        int32_t P = S;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t x = __shfl_up_sync(kFull, P, o);
-            if (lane >= o) P = max(P, x);
-        }
-        P = max(P, cmax);
-        const bool stop = valid && ((RIGHT && S <= 0) || P - S >= xdrop);
-        const unsigned sm = __ballot_sync(kFull, stop);
-        const int last = sm ? __ffs(sm) - 1 : min(31, n - 1 - base);
-        const int32_t m = __shfl_sync(kFull, P, last);
-        if (m > cmax) {
-            const unsigned hm = __ballot_sync(kFull, valid && lane <= last && S == m);
-            bk = base + __ffs(hm) - 1;
-            cmax = m;
-        }
-        carry = __shfl_sync(kFull, S, last);
-        if (sm) {
-            stop_at = base + last;
-            break;
-        }
-    }
-    *best_k = bk;
-    *end = stop_at;
-    return cmax;
-}
-
-template <typename Q, typename S>
-__device__ __forceinline__ int32_t extend_two_hit_warp(const Q &q, const S &s,
-                                                       int32_t s_left_off, int32_t s_off, int32_t q_off,
-                                                       int32_t xdrop, int32_t *hsp_q, int32_t *hsp_s,
-                                                       int32_t *hsp_len, int32_t *right_extend,
-                                                       int32_t *s_last_off) {
-    int32_t score = 0, left_score = 0, right_d = 0;
-#pragma unroll
-    for (int32_t i = 0; i < kWordSize; ++i) {
-        score += score_of(q.at(q_off + i), s.at(s_off + i));
-        if (score > left_score) {
-            left_score = score;
-            right_d = i + 1;
-        }
-    }
-    const int32_t q_right = q_off + right_d, s_right = s_off + right_d;
-    // left: positions k = 0 .. min(s_right, q_right) - 1 backwards from the
-    // residue pair before (q_right, s_right)
-    int32_t bk, end;
-    left_score = walk_warp<false>(
-        [&](int32_t k) { return score_of(q.at(q_right - 1 - k), s.at(s_right - 1 - k)); },
-        min(s_right, q_right), 0, xdrop, &bk, &end);
-    const int32_t left_d = bk + 1;
-    int32_t right_score = 0, rd = 0;
-    *right_extend = 0;
-    *s_last_off = s_right;
-    if (left_d >= s_right - s_left_off) {
-        *right_extend = 1;
-        int32_t bi, iend;
-        right_score = walk_warp<true>(
-            [&](int32_t i) { return score_of(q.at(q_right + i), s.at(s_right + i)); },
-            min(s.len - s_right, q.len - q_right), left_score, xdrop, &bi, &iend);
-        rd = bi + 1;
-        *s_last_off = s_right + iend;
-    }
-    *hsp_q = q_right - left_d;
-    *hsp_s = s_right - left_d;
-    *hsp_len = left_d + rd;
-    return max(left_score, right_score);
-}
-
-// ------------------------------------------------------------------------
-// Word finder state of one warp. The diagonal table holds, per diagonal
-// (x - q) mod L, either the last recorded hit (biased by window and by a
-// running base so the table never needs clearing between groups), the end of
+// Word finder state of one warp. A hit is a pair (v, q): v is the position x
+// plus `window` for each subject of the group before its own, so that hits of
+// different subjects are always more than `window` apart. The diagonal table
+// holds, per diagonal (v - q) mod L, either the last recorded hit (v plus a
+// running base, so the table never needs clearing between groups), the end of
 // a right extension with kFlag, or kPend | seed slot while that diagonal's
 // extension is queued. With L >= qlen + window two diagonals that share an
 // entry never both matter: all hits of the later one come more than `window`
 // positions after every hit of the earlier one and after the end of any
-// extension on it. Each subject of a group adds `window` to the bias, so what
-// the subjects before it left in the table is likewise out of reach; only a
-// seed still queued for an earlier subject makes a hit on its entry wait.
+// extension on it; only a seed still queued for an earlier subject makes a hit
+// on its entry wait.
 //
 // Entries are 16 bits wide for the queries kept in shared memory, which
 // leaves room for twice the warps with long queries (3,000 residues: 24
-// instead of 14 per SM, 18.4 -> 11.3 ms for 139 M residues); the
+// instead of 14 per SM, 18.4 -> 11.7 ms for 139 M residues); the
 // values then stay below 2^14: the table is cleared before a group that would
 // pass it, and moved down (rebase) inside a long subject. Otherwise 32 bits.
-//
-// Deferred hits and seeds are packed: x and the subject's number in the
-// group (or, in a group of one subject, 17 bits of x counted from xb), and q.
 template <bool QS>
 struct Tab {
     static constexpr uint32_t kFlag = QS ? 0x8000u : 0x40000000u;
@@ -353,9 +313,9 @@ struct Finder {
     uint32_t base;
     uint32_t n_init;
     uint32_t hits, extensions;  // not yet added to the counters
-    uint32_t rel;  // lane i: position of the group's subject i (i <= their number)
-    int32_t xb;    // packed positions count from here
-    uint32_t xs;   // bits of the subject's number in a packed hit
+    uint32_t ns;                // subjects of the group
+    uint32_t first, end;        // lane i < ns: subject i's positions [first, end); first is 2^31 - 1 from ns on
+    int32_t vb;                 // packed hits count v from here
 };
 
 // Per-query parameters of the word finder (one query, or the query of the
@@ -369,26 +329,16 @@ struct Ctx {
     uint32_t seed_span;  // distances from the word size on that trigger an extension
 };
 
-constexpr int kGroupBits = 5;  // of a subject's number in its group
 constexpr int32_t kPackSpan = 1 << 17;
-static_assert(kGroupMaxSubjects < 32 && (kGroupMaxResidues << kGroupBits) < kPackSpan, "packed hits");
-static_assert(kGroupMaxResidues + (kGroupMaxSubjects + 1) * kTab16Window <= Tab<true>::kMost, "16-bit entries");
+static_assert(kGroupMaxBytes + (kGroupMaxSubjects + 2) * kTab16Window <= Tab<true>::kMost, "16-bit entries");
 static_assert(kQuerySmemMax + kChunk + kTab16Window <= Tab<true>::kMost, "16-bit entries");
 
-__device__ __forceinline__ uint32_t pack_hit(const Finder &f, int32_t x, int32_t q, uint32_t subj) {
-    return ((static_cast<uint32_t>(x - f.xb) << f.xs | subj) << 15) | static_cast<uint32_t>(q);
+// A hit in 32 bits: v (17 bits from vb on) and q (at most 32,000).
+__device__ __forceinline__ uint32_t pack_hit(const Finder &f, int32_t v, int32_t q) {
+    return (static_cast<uint32_t>(v - f.vb) << 15) | static_cast<uint32_t>(q);
 }
-struct Hit {
-    int32_t x, q;
-    uint32_t subj;
-};
-__device__ __forceinline__ Hit unpack_hit(const Finder &f, uint32_t v) {
-    Hit h;
-    h.q = static_cast<int32_t>(v & 0x7fffu);
-    h.subj = (v >> 15) & ((1u << f.xs) - 1u);
-    h.x = static_cast<int32_t>(v >> (15u + f.xs)) + f.xb;
-    return h;
-}
+__device__ __forceinline__ int32_t hit_v(const Finder &f, uint32_t p) { return static_cast<int32_t>(p >> 15) + f.vb; }
+__device__ __forceinline__ int32_t hit_q(uint32_t p) { return static_cast<int32_t>(p & 0x7fffu); }
 
 __device__ __forceinline__ uint32_t defer_at(const Finder &f, uint32_t buf, int i) {
     return f.w + kDeferAt + 4u * (buf * kDeferCap + static_cast<uint32_t>(i));
@@ -397,49 +347,93 @@ __device__ __forceinline__ uint32_t defer_at(const Finder &f, uint32_t buf, int 
 __device__ __forceinline__ uint32_t seed_at(const Finder &f, int i) {
     return f.w + kSeedAt + 8u * static_cast<uint32_t>(i);
 }
-__device__ __forceinline__ uint32_t diag_of(const Ctx &c, int32_t x, int32_t q) {
-    return fast_mod(static_cast<uint32_t>(x - q + c.qlen), c.diag_entries, c.diag_magic);
-}
-// What to add to positions of the group's subject number `subj`.
-__device__ __forceinline__ uint32_t bias_of(const Finder &f, const Ctx &c, uint32_t subj) {
-    return f.base + static_cast<uint32_t>(c.window) * (subj + 1u);
+__device__ __forceinline__ uint32_t diag_of(const Ctx &c, int32_t v, int32_t q) {
+    return fast_mod(static_cast<uint32_t>(v - q + c.qlen), c.diag_entries, c.diag_magic);
 }
 __device__ __forceinline__ InitHit *scratch_of(const ScanArgs &a) {
     const unsigned long long gwarp = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     return a.scratch + gwarp * a.scratch_cap;
 }
 
-// What a hit does on its diagonal, from the entry's distance below it:
-// a flagged entry is further below than any recorded hit, a pending one
-// further still (`here` and every entry's value stay within Tab::kMost).
-struct Outcome {
-    bool set, seed, pend;
-};
+// Stores `here` in the entry for the lanes that `act` and returns, for them,
+// what the entry then holds: the smallest `here` of the lanes that share it.
+// The hardware keeps the lowest lane's store, and lanes are in hit order; the
+// loop makes sure of it.
 template <bool QS>
-__device__ __forceinline__ Outcome outcome(uint32_t here, uint32_t e, const Ctx &c) {
-    const int32_t diff = static_cast<int32_t>(here - e);
-    Outcome o;
-    // a hit far from the last one starts over, as does the first hit past
-    // the end of an extension (the wrapped distances from -kFlag on)
-    o.set = diff >= c.window || static_cast<uint32_t>(diff) >= 0u - Tab<QS>::kFlag;
-    // one at distance [wordsize, window) triggers an extension; an overlapping
-    // one, and one inside the last extension, is ignored
-    o.seed = static_cast<uint32_t>(diff - kWordSize) < c.seed_span;
-    o.pend = e >= Tab<QS>::kPend;
-    return o;
+__device__ __forceinline__ uint32_t claim(uint32_t entry, uint32_t here, bool act) {
+    uint32_t low = here;
+    __syncwarp();
+    if (act) Tab<QS>::store(entry, here);
+    __syncwarp();
+    if (act) low = Tab<QS>::load(entry);
+    while (__any_sync(kFull, low > here)) {
+        if (low > here) Tab<QS>::store(entry, here);
+        __syncwarp();
+        if (act) low = Tab<QS>::load(entry);
+        __syncwarp();
+    }
+    return low;
 }
 
-// Appends the batch's deferred hits and seeds to their queues, in lane order.
+// Runs up to 32 hits (one per lane, lanes in hit order) through the two-hit
+// logic. The entry's distance below a hit decides what it does: a flagged entry
+// is further below than any recorded hit, a pending one further still (every
+// value stays within Tab::kMost).
+//
+// About a quarter of a batch's hits share their diagonal with an earlier lane,
+// mostly the next word of the same match (1 or 2 positions on). The lanes whose
+// hits do something claim their entries; the first of a diagonal does what the
+// entry said, and leaves the others one of two cases:
+//   it is a seed: they are deferred, as every later hit is until it is extended
+//   it starts over: a hit 1 or 2 positions on is ignored, and the first of
+//     the others decides by its distance from it: the second claim
+// Behind a second hit that starts over as well (rare: it is `window` or more
+// from the first) the rest is brought again: true is returned for them.
+//
+// The kernel is bound by instruction issue (82 % at 300 query residues), and
+// this function was nearly half of it. __match_any_sync in place of the claims
+// costs few instructions, but 8.4 cycles per distinct value: 270 for a batch of
+// 32 diagonals. With the claims and full batches: 139 M residues at 300 / 1,000
+// query residues 1.26 -> 1.05 and 3.39 -> 2.70 ms.
 template <bool QS>
-__device__ __forceinline__ void queue_hits(Finder &f, bool def, bool seed, int32_t x, int32_t q, uint32_t subj,
-                                           int32_t dist, uint32_t entry) {
+__device__ __forceinline__ bool two_hit(Finder &f, const Ctx &c, bool valid, int32_t v, int32_t q) {
+    const uint32_t entry = Tab<QS>::at(f.w, diag_of(c, v, q));
+    const uint32_t here = static_cast<uint32_t>(v) + f.base;
+    const uint32_t e = valid ? Tab<QS>::load(entry) : here;  // a lane without a hit does nothing
+    int32_t dist = static_cast<int32_t>(here - e);
+    // a hit far from the last one starts over, as does the first hit past the
+    // end of an extension (the wrapped distances from -kFlag on); one at
+    // distance [wordsize, window) triggers an extension; an overlapping one,
+    // and one inside the last extension, is ignored
+    const bool near = static_cast<uint32_t>(dist - kWordSize) < c.seed_span;
+    const bool act = near || dist >= c.window || static_cast<uint32_t>(dist) >= 0u - Tab<QS>::kFlag;
+    const uint32_t low = claim<QS>(entry, here, act);
+    const bool alone = low == here;
+    bool seed = near && alone;
+    bool def = valid && e >= Tab<QS>::kPend;  // its diagonal waits for an extension
+    bool again = false;
+    if (__any_sync(kFull, !alone)) {
+        const bool behind_seed = static_cast<uint32_t>(static_cast<int32_t>(low - e) - kWordSize) < c.seed_span;
+        const int32_t df = static_cast<int32_t>(here - low);
+        def = def || (!alone && behind_seed);
+        const bool wait = !behind_seed && df >= kWordSize;
+        if (__any_sync(kFull, wait)) {
+            const uint32_t low2 = claim<QS>(entry, here, wait);
+            const bool second = static_cast<int32_t>(low2 - low) < c.window;  // the second hit is a seed
+            if (wait) {
+                dist = df;
+                seed = second && low2 == here;
+                def = second && low2 != here;
+                again = !second && low2 != here;
+            }
+        }
+    }
     const unsigned dm = __ballot_sync(kFull, def);
     const unsigned sm = __ballot_sync(kFull, seed);
     if ((dm | sm) != 0u) {
         const unsigned lt = lanemask_lt();
-        const uint32_t packed = pack_hit(f, x, q, subj);
+        const uint32_t packed = pack_hit(f, v, q);
         if (def) sts32(defer_at(f, f.sel, f.n_defer + __popc(dm & lt)), packed);
-        __syncwarp();  // a seed's entry overwrites the one its diagonal's first hit just recorded
         if (seed) {
             const int slot = f.n_seed + __popc(sm & lt);
             sts64(seed_at(f, slot), make_uint2(packed, static_cast<uint32_t>(dist)));
@@ -448,144 +442,67 @@ __device__ __forceinline__ void queue_hits(Finder &f, bool def, bool seed, int32
         f.n_defer += __popc(dm);
         f.n_seed += __popc(sm);
     }
+    __syncwarp();
+    return again;
 }
 
-// Runs up to 32 hits (one per lane, lanes in hit order) through the two-hit
-// logic. A hit whose diagonal waits on an extension is appended to the
-// deferred list. About a quarter of a batch's hits share their diagonal with
-// an earlier lane, mostly the next word of the same match (1 or 2 positions
-// on). What such a hit does follows from the diagonal's first hit in the
-// batch, so most are settled here without another pass over the table:
-//   first recorded     1-2 positions on: ignored (so are all hits between);
-//                      the second hit, 3 to window on: a seed
-//   first seeded       deferred
-//   first left the entry as it was: the entry decides for the second hit
-//                      too, and for later ones that it makes do nothing
-// Only the rest (`hard`) reread the table, one per diagonal at a time. The
-// kernel is bound by instruction issue, and one pass over the table per hit
-// of a diagonal, as before, took 11.4 warp instructions per residue at 300
-// query residues, this form 10.5 (139 M residues: 1.64 -> 1.57 ms; at 1,000
-// query residues 4.27 -> 4.06 ms).
-template <bool QS>
-__device__ __forceinline__ void process_batch(Finder &f, const Ctx &c, bool valid, int32_t x, int32_t q,
-                                              uint32_t subj, uint32_t bias) {
-    const unsigned lt = lanemask_lt();
-    const uint32_t entry = Tab<QS>::at(f.w, diag_of(c, x, q));
-    const uint32_t here = static_cast<uint32_t>(x) + bias;
-    const unsigned peers = __match_any_sync(kFull, valid ? entry : ~(threadIdx.x & 31u));
-    const uint32_t e = valid ? Tab<QS>::load(entry) : here;  // a lane without a hit does nothing
-    const unsigned lower = peers & lt;
-    const Outcome o = outcome<QS>(here, e, c);
-    const bool dup = lower != 0u;
-    bool set = o.set && !dup, seed = o.seed && !dup, def = o.pend, hard = false;
-    int32_t dist = static_cast<int32_t>(here - e);
-    const unsigned dupm = __ballot_sync(kFull, dup);
-    if (dupm != 0u) {
-        const unsigned setm = __ballot_sync(kFull, set), seedm = __ballot_sync(kFull, seed);
-        const uint32_t hf = __shfl_sync(kFull, here, __ffs(peers) - 1);
-        if (dup) {
-            const unsigned first = peers & (0u - peers);
-            const bool second = (lower & (lower - 1u)) == 0u;
-            const int32_t df = static_cast<int32_t>(here - hf);
-            if ((setm & first) != 0u) {
-                seed = second && df >= kWordSize && df < c.window;
-                hard = !seed && df >= kWordSize;
-                dist = df;
-            } else if ((seedm & first) != 0u) {
-                def = true;
-            } else if (o.set || o.seed) {
-                set = second && o.set;
-                seed = second && o.seed;
-                hard = !second;
-            }
-        }
-    }
-    if (set) Tab<QS>::store(entry, here);
-    queue_hits<QS>(f, def, seed, x, q, subj, dist, entry);
-    __syncwarp();
-    if (dupm != 0u) {
-        for (unsigned hm = __ballot_sync(kFull, hard); hm != 0u;) {
-            const bool mine = hard && (lower & hm) == 0u;
-            const uint32_t e2 = mine ? Tab<QS>::load(entry) : here;
-            const Outcome o2 = outcome<QS>(here, e2, c);
-            if (o2.set) Tab<QS>::store(entry, here);
-            queue_hits<QS>(f, o2.pend, o2.seed, x, q, subj, static_cast<int32_t>(here - e2), entry);
-            hard = hard && !mine;
-            hm = __ballot_sync(kFull, hard);
-            __syncwarp();
-        }
-    }
+// Whether the queues may not hold another batch's seeds or deferred hits.
+__device__ __forceinline__ bool queues_full(const Finder &f) {
+    return f.n_seed >= 32 || f.n_defer > kDeferCap - 32;
 }
 
 // Extends every queued seed (one lane each), settles their diagonals, keeps
-// those reaching the ungapped cutoff, then replays the deferred hits; repeats
-// until no seed and no deferred hit is left. Each replay is shorter than the
-// list it replays whenever it queues a seed, so the loop ends. Seeds of all
-// the group's subjects share a flush: a walk takes about 13 warp instructions
-// a step whether one lane or 32 take it, so what an extension costs falls with
-// the seeds it shares its flush with.
+// those reaching the ungapped cutoff, then replays the deferred hits. The
+// seeds that the replay queues wait for the next flush, unless the queues are
+// still too full for another batch or (`empty`) have to be emptied: then it
+// repeats. Each replay is shorter than the list it replays whenever it queues
+// a seed, so the loop ends. Seeds of all the group's subjects share a flush: a
+// walk takes as many warp instructions a step whether one lane or 32 take it,
+// so what an extension costs falls with the seeds it shares its flush with.
 template <bool QS, bool WT, bool ST>
 __device__ __forceinline__ void flush(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, WT> &q,
-                                      const Span<ST> &span) {
-    const int lane = threadIdx.x & 31;
+                                      const Span<ST> &span, bool empty) {
+    const uint32_t lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();
-    auto settle = [&](const Hit &h, int32_t first, int32_t rext, int32_t slast) {
-        const uint32_t bias = bias_of(f, c, h.subj);
-        Tab<QS>::store(Tab<QS>::at(f.w, diag_of(c, h.x, h.q)),
-                       rext ? (Tab<QS>::kFlag | (static_cast<uint32_t>(first + slast - (kWordSize - 1)) + bias))
-                            : (static_cast<uint32_t>(h.x) + bias));
-    };
-    auto keep = [&](uint32_t at, const Hit &h, int32_t first, int32_t hq, int32_t hs, int32_t hl, int32_t score) {
-        if (at >= a.scratch_cap) return;
-        InitHit r;
-        r.q_start = hq;
-        r.s_start = hs + first;  // positions of the span until the group is published
-        r.len = hl;
-        r.score = score;
-        r.q_trig = h.q;
-        r.s_trig = h.x;
-        scratch_of(a)[at] = r;
-    };
-    while (f.n_seed > 0 || f.n_defer > 0) {
-        // few seeds: one at a time with the whole warp on each walk
-        for (int i = 0; f.n_seed <= kCoopSeeds && i < f.n_seed; ++i) {
-            const uint2 sd = lds64(seed_at(f, i));
-            const Hit h = unpack_hit(f, sd.x);
-            Subject<ST> sub;
-            sub.span = span;
-            sub.first = __shfl_sync(kFull, f.rel, h.subj);
-            sub.len = __shfl_sync(kFull, f.rel, h.subj + 1u) - sub.first;
-            const int32_t so = h.x - sub.first;
-            int32_t hq, hs, hl, rext, slast;
-            const int32_t score = extend_two_hit_warp(q, sub, so - static_cast<int32_t>(sd.y) + kWordSize, so, h.q,
-                                                      c.xdrop, &hq, &hs, &hl, &rext, &slast);
-            if (lane == 0) {
-                settle(h, sub.first, rext, slast);
-                if (score >= c.cutoff) keep(f.n_init, h, sub.first, hq, hs, hl, score);
-            }
-            if (score >= c.cutoff) ++f.n_init;
-        }
-        // many: one lane per seed
-        for (int c0 = 0; f.n_seed > kCoopSeeds && c0 < f.n_seed; c0 += 32) {
-            const int i = c0 + lane;
-            bool pass = false;
-            int32_t hq = 0, hs = 0, hl = 0, score = 0;
+    // where subject `lane` begins in v (its 16-byte block where there are several)
+    const uint32_t v0 = f.ns > 1 ? (f.first & ~15u) + static_cast<uint32_t>(c.window) * lane : f.first;
+    do {
+        for (int c0 = 0; c0 < f.n_seed; c0 += 32) {
+            const int i = c0 + static_cast<int>(lane);
             const uint2 sd = lds64(seed_at(f, min(i, f.n_seed - 1)));
-            const Hit h = unpack_hit(f, sd.x);
+            const int32_t hv = hit_v(f, sd.x), hq = hit_q(sd.x);
+            uint32_t subj = 0;  // the last subject that begins at or before the hit
+            if (f.ns > 1) {
+#pragma unroll
+                for (uint32_t step = 16; step >= 1; step >>= 1)
+                    if (__shfl_sync(kFull, v0, subj + step) <= static_cast<uint32_t>(hv)) subj += step;
+            }
             Subject<ST> sub;
             sub.span = span;
-            sub.first = __shfl_sync(kFull, f.rel, h.subj);
-            sub.len = __shfl_sync(kFull, f.rel, h.subj + 1u) - sub.first;
+            sub.first = static_cast<int32_t>(__shfl_sync(kFull, f.first, subj));
+            sub.len = static_cast<int32_t>(__shfl_sync(kFull, f.end, subj)) - sub.first;
+            bool pass = false;
+            InitHit h{};
             if (i < f.n_seed) {
-                const int32_t so = h.x - sub.first;
+                const int32_t to_v = c.window * static_cast<int32_t>(subj) + sub.first;  // from the subject's offsets
+                const int32_t so = hv - to_v, left = so - static_cast<int32_t>(sd.y) + kWordSize;
                 int32_t rext, slast;
-                score = extend_two_hit(q, sub, so - static_cast<int32_t>(sd.y) + kWordSize, so, h.q, c.xdrop, &hq, &hs,
-                                       &hl, &rext, &slast);
-                settle(h, sub.first, rext, slast);
-                pass = score >= c.cutoff;
+                h.score = QS || sub.len <= kKeyedLength
+                              ? extend_two_hit_keyed(q, sub, left, so, hq, c.xdrop, &h.q_start, &h.s_start, &h.len,
+                                                     &rext, &slast)
+                              : extend_two_hit(q, sub, left, so, hq, c.xdrop, &h.q_start, &h.s_start, &h.len, &rext,
+                                               &slast);
+                Tab<QS>::store(Tab<QS>::at(f.w, diag_of(c, hv, hq)),
+                               rext ? Tab<QS>::kFlag | (static_cast<uint32_t>(slast - (kWordSize - 1) + to_v) + f.base)
+                                    : static_cast<uint32_t>(hv) + f.base);
+                pass = h.score >= c.cutoff;
+                h.q_trig = hq;
+                h.s_trig = so + sub.first;  // positions until the group is published
+                h.s_start += sub.first;
             }
             const unsigned pm = __ballot_sync(kFull, pass);
-            if (pass) keep(f.n_init + __popc(pm & lt), h, sub.first, hq, hs, hl, score);
+            const uint32_t at = f.n_init + __popc(pm & lt);
+            if (pass && at < a.scratch_cap) scratch_of(a)[at] = h;
             f.n_init += __popc(pm);
         }
         f.extensions += static_cast<uint32_t>(f.n_seed);
@@ -597,13 +514,14 @@ __device__ __forceinline__ void flush(Finder &f, const ScanArgs &a, const Ctx &c
             f.sel ^= 1u;
             f.n_defer = 0;
             for (int c0 = 0; c0 < n_old; c0 += 32) {
-                const int i = c0 + lane;
-                const bool v = i < n_old;
-                const Hit h = unpack_hit(f, lds32(defer_at(f, old, v ? i : 0)));
-                process_batch<QS>(f, c, v, h.x, h.q, h.subj, bias_of(f, c, h.subj));
+                const int i = c0 + static_cast<int>(lane);
+                const uint32_t p = lds32(defer_at(f, old, min(i, n_old - 1)));
+                bool again = i < n_old;
+                do again = two_hit<QS>(f, c, again, hit_v(f, p), hit_q(p));
+                while (__any_sync(kFull, again));
             }
         }
-    }
+    } while (queues_full(f) || (empty && (f.n_seed > 0 || f.n_defer > 0)));
 }
 
 // Adds the hit and extension counts to the launch's counters.
@@ -615,121 +533,159 @@ __device__ __forceinline__ void add_counts(Finder &f, const ScanArgs &a) {
     f.hits = f.extensions = 0;
 }
 
-// Whether the chunk at cb (of a subject ending at x1) needs a rebase first:
-// the values its hits and extensions can reach, or its packed positions, would
-// pass their limits. Only a group of one subject ever does.
+// Whether the chunk at cb of a group of one subject (ending at `end`) needs a
+// rebase first: the values its hits and extensions can reach, or its packed
+// hits, would pass their limits.
 template <bool QS>
-__device__ __forceinline__ bool needs_rebase(const Finder &f, const Ctx &c, int32_t x1, int32_t cb, uint32_t bias) {
-    if (QS) return static_cast<uint32_t>(min(x1, cb + kChunk + c.qlen)) + bias > Tab<QS>::kMost;
-    return cb - f.xb > kPackSpan - kChunk;
+__device__ __forceinline__ bool needs_rebase(const Finder &f, const Ctx &c, int32_t end, int32_t cb) {
+    if (QS) return static_cast<uint32_t>(min(end, cb + kChunk + c.qlen)) + f.base > Tab<QS>::kMost;
+    return cb - f.vb > kPackSpan - kChunk;
 }
 
-// Lets packed positions count from cb and (16-bit entries) moves the table
-// down so that a hit at cb has value `window`; an entry that falls below 0 is
-// more than `window` behind cb, or an extension's end behind it, and stays so
-// as 0. The queues are empty.
+// Lets packed hits count from cb and (16-bit entries) moves the table down so
+// that a hit at cb has value `window`; an entry that falls below 0 is more
+// than `window` behind cb, or an extension's end behind it, and stays so as 0.
+// The queues are empty.
 template <bool QS>
-__device__ __forceinline__ void rebase(Finder &f, const ScanArgs &a, const Ctx &c, int32_t cb, uint32_t &bias) {
-    f.xb = cb;
+__device__ __forceinline__ void rebase(Finder &f, const ScanArgs &a, const Ctx &c, int32_t cb) {
+    f.vb = cb;
     add_counts(f, a);
     if (!QS) return;
-    const uint32_t delta = static_cast<uint32_t>(cb) + bias - static_cast<uint32_t>(c.window);
+    const uint32_t delta = static_cast<uint32_t>(cb - c.window) + f.base;
     for (uint32_t i = threadIdx.x & 31; i < c.diag_entries; i += 32) {
         const uint32_t o = Tab<QS>::at(f.w, i), e = Tab<QS>::load(o), v = e & Tab<QS>::kMost;
         Tab<QS>::store(o, (e & Tab<QS>::kFlag) | (v > delta ? v - delta : 0u));
     }
     f.base -= delta;
-    bias -= delta;
     __syncwarp();
 }
 
-// 1 << n, 0 from n = 32 on
-__device__ __forceinline__ uint32_t bit_at(uint32_t n) {
+// x << n, 0 from n = 32 on
+__device__ __forceinline__ uint32_t shift_left(uint32_t x, uint32_t n) {
     uint32_t r;
-    asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(n));
+    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(n));
     return r;
 }
 
-// Word scan of a group of ns subjects: chunks of 128 positions, four
-// consecutive positions per lane. One warp prefix sum per chunk numbers the
-// chunk's hits in (subject offset, query offset) order and the words that have
-// any; each such word leaves its position and where its hits lie in the warp's
-// list. Lanes then take the hits 32 at a time: a bit mask of the hits that
-// start a word gives each lane its word by a population count.
+// Inclusive prefix sum over the warp.
+__device__ __forceinline__ uint32_t warp_prefix(uint32_t x) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+        asm volatile("{\n .reg .pred p;\n .reg .u32 t;\n shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n @p add.u32 %0, %0, t;\n}"
+            : "+r"(x)
+            : "r"(o));
+    return x;
+}
+
+// Word scan of a group: chunks of 128 positions, four consecutive positions
+// per lane. One warp prefix sum per chunk numbers the chunk's hits in (subject
+// offset, query offset) order and the words that have any; each such word
+// leaves its v and where its hits lie in the warp's list. Lanes then take the
+// hits 32 at a time: a bit mask of the hits that start a word gives each lane
+// its word by a population count. A chunk's last hits, too few for a batch,
+// wait in front of the next chunk's, so batches are full (at 300 query
+// residues a chunk brings 79 hits).
 template <bool QS, bool WT, bool ST>
 __device__ __forceinline__ void scan_span(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, WT> &q,
-                                          const Span<ST> &span, uint32_t ns) {
+                                          const Span<ST> &span, bool long_one) {
     const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t subj = 0; subj < ns; ++subj) {
-        const int32_t x0 = static_cast<int32_t>(__shfl_sync(kFull, f.rel, subj));
-        const int32_t x1 = static_cast<int32_t>(__shfl_sync(kFull, f.rel, subj + 1u));
-        const int32_t xend = x1 - (kWordSize - 1);  // words start below it
-        uint32_t bias = bias_of(f, c, subj);
-        for (int32_t cb = x0; cb < xend; cb += kChunk) {
-            if (needs_rebase<QS>(f, c, x1, cb, bias)) rebase<QS>(f, a, c, cb, bias);
-            // the queues are emptied at the group's end and before a rebase
-            // (the group's last subject is its longest: it has a chunk if any has)
-            const int32_t next = cb + kChunk;
-            const bool empty = next < xend ? needs_rebase<QS>(f, c, x1, next, bias) : subj + 1u == ns;
-            const int32_t p0 = cb + 4 * static_cast<int32_t>(lane);
-            uint32_t r[6];
+    const uint32_t list = f.w + kListAt;
+    const int32_t end = static_cast<int32_t>(__shfl_sync(kFull, f.end, f.ns - 1u));
+    const int32_t xend = end - (kWordSize - 1);  // words start below it
+    uint32_t before = 0;                         // subjects that begin before the chunk
+    uint32_t left = 0;   // hits waiting from the chunks before, fewer than a batch
+    uint32_t left_m = 0; // which of them start a word
+    uint32_t left_w = 0; // words begun before the chunk whose hits are waiting
+    // four positions of a lane lie in one subject's block
+    int32_t cb = static_cast<int32_t>(__shfl_sync(kFull, f.first, 0));
+    if (f.ns > 1) cb &= ~15;
+    for (; cb < xend; cb += kChunk) {
+        if (long_one && needs_rebase<QS>(f, c, end, cb)) rebase<QS>(f, a, c, cb);
+        // the queues are emptied at the group's end and before a rebase
+        const bool empty = cb + kChunk >= xend || (long_one && needs_rebase<QS>(f, c, end, cb + kChunk));
+        const int32_t p0 = cb + 4 * static_cast<int32_t>(lane);
+        uint32_t r[6];
 #pragma unroll
-            for (int j = 0; j < 6; ++j) r[j] = span.at(ST ? p0 + j : min(p0 + j, x1 - 1));
-            uint32_t cs[4], cnt[4], sum = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const bool v = p0 + j < xend;
-                if (WT) {
-                    const uint32_t t = kTabOff + r[j] * 1568u + r[j + 1] * 56u + r[j + 2] * 2u;
-                    cs[j] = v ? lds16(t) : 0u;
-                    cnt[j] = v ? lds16(t + 2u) - cs[j] : 0u;
-                } else {
-                    const uint32_t w = r[j] * 784u + r[j + 1] * 28u + r[j + 2];
-                    const bool present = v && ((lds32(kTabOff + 4u * (v ? w >> 5 : 0u)) >> (w & 31u)) & 1u);
-                    const uint32_t pk = present ? __ldg(c.cell_pack + w) : 0u;
-                    cs[j] = pk >> 8;
-                    cnt[j] = pk & 0xffu;
-                    if (cnt[j] == 0xffu) cnt[j] = __ldg(c.cell_start + w + 1) - cs[j];
-                }
-                sum += (cnt[j] << 8) + (cnt[j] ? 1u : 0u);  // 24 bits: 128 words of at most 32,000 hits
-            }
-            uint32_t incl = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(kFull, incl, o);
-                if (lane >= o) incl += y;
-            }
-            const uint32_t total = __shfl_sync(kFull, incl, 31) >> 8;
-            if (total == 0 && !empty) continue;
-            f.hits += total;
-            uint32_t e[4], run = (incl - sum) >> 8, slot = f.w + kListAt + 8u * ((incl - sum) & 0xffu);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                e[j] = cnt[j] ? run : 0x80000000u;  // the word's first hit
-                if (cnt[j]) {
-                    sts64(slot, make_uint2(cs[j] - run, static_cast<uint32_t>(p0 + j)));
-                    slot += 8u;
-                }
-                run += cnt[j];
-            }
-            __syncwarp();
-            uint32_t word = f.w + kListAt - 8u;  // the last word begun before the batch
-            uint32_t kb = 0;
-            do {
-                if (kb < total) {
-                    const uint32_t m = __reduce_or_sync(
-                        kFull, bit_at(e[0] - kb) | bit_at(e[1] - kb) | bit_at(e[2] - kb) | bit_at(e[3] - kb));
-                    const uint32_t k = kb + lane;
-                    const uint2 wd = lds64(word + 8u * __popc(m & (0xffffffffu >> (31u - lane))));
-                    word += 8u * __popc(m);
-                    const bool hv = k < total;
-                    const int32_t qo = hv ? static_cast<int32_t>(__ldg(c.cell_off + (wd.x + k))) : 0;
-                    process_batch<QS>(f, c, hv, static_cast<int32_t>(wd.y), qo, subj, bias);
-                }
-                kb += 32;
-                if (f.n_seed >= 32 || f.n_defer > kDeferCap - 32 || (empty && kb >= total)) flush(f, a, c, q, span);
-            } while (kb < total);
+        for (int j = 0; j < 6; ++j) r[j] = span.at(ST ? p0 + j : min(p0 + j, end - 1));
+        int32_t v0 = p0;
+        if (f.ns > 1) {
+            const uint32_t begins =
+                __reduce_or_sync(kFull, shift_left(1u, ((f.first & ~15u) - static_cast<uint32_t>(cb)) >> 2));
+            v0 += c.window * static_cast<int32_t>(before + __popc(begins & lanemask_le()) - 1u);
+            before += __popc(begins);
         }
+        uint32_t cs[4], cnt[4], has[4], sum = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const bool in = ST || p0 + j < xend;  // (zeros follow the staged residues)
+            if (WT) {
+                const uint32_t t = kTabOff + (in ? r[j] * 1568u + r[j + 1] * 56u + r[j + 2] * 2u : 0u);
+                cs[j] = lds16(t);
+                cnt[j] = lds16(t + 2u) - cs[j];
+            } else {
+                const uint32_t w = in ? r[j] * 784u + r[j + 1] * 28u + r[j + 2] : 0u;
+                const bool present = (lds32(kTabOff + 4u * (w >> 5)) >> (w & 31u)) & 1u;
+                const uint32_t pk = present ? __ldg(c.cell_pack + w) : 0u;
+                cs[j] = pk >> 8;
+                cnt[j] = pk & 0xffu;
+                if (cnt[j] == 0xffu) cnt[j] = __ldg(c.cell_start + w + 1) - cs[j];
+            }
+            has[j] = min(cnt[j], 1u);
+            sum += cnt[j] * 256u + has[j];  // 24 bits: 128 words of at most 32,000 hits
+        }
+        const uint32_t incl = warp_prefix(sum);
+        const uint32_t all = __shfl_sync(kFull, incl, 31);
+        if (all == 0 && !empty) continue;
+        f.hits += all >> 8;
+        const uint32_t total = left + (all >> 8);  // hits, the waiting ones first
+        uint32_t e[4], run = left + ((incl - sum) >> 8), slot = list + 8u * (left_w + ((incl - sum) & 0xffu));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            e[j] = run;  // the word's first hit
+            if (cnt[j]) sts64(slot, make_uint2(cs[j] - run, static_cast<uint32_t>(v0 + j)));
+            slot += 8u * has[j];
+            run += cnt[j];
+        }
+        __syncwarp();
+        // words that begin with one of the hits k0 .. k0 + 31
+        auto begins_from = [&](uint32_t k0) {
+            return __reduce_or_sync(kFull, shift_left(has[0], e[0] - k0) | shift_left(has[1], e[1] - k0) |
+                                               shift_left(has[2], e[2] - k0) | shift_left(has[3], e[3] - k0));
+        };
+        uint32_t m = begins_from(0) | left_m;
+        // the last word begun before the batch: with hits waiting, the first of the list is
+        uint32_t word = list - (left > 0 && (left_m & 1u) == 0u ? 0u : 8u);
+        uint32_t k0 = 0;  // the first hit not yet taken
+        do {
+            bool batch = k0 + 32u <= total || (empty && k0 < total);
+            if (batch) {
+                const uint32_t k = k0 + lane;
+                const uint2 wd = lds64(word + 8u * __popc(m & lanemask_le()));
+                word += 8u * __popc(m);
+                bool go = k < total;
+                const int32_t qo = go ? static_cast<int32_t>(__ldg(c.cell_off + (wd.x + k))) : 0;
+                do go = two_hit<QS>(f, c, go, static_cast<int32_t>(wd.y), qo);
+                while (__any_sync(kFull, go));
+                k0 += 32u;
+                m = begins_from(k0);
+            }
+            const bool done = empty && k0 >= total;
+            if (queues_full(f) || done) flush(f, a, c, q, span, done);
+            if (done || !batch) break;
+        } while (true);
+        // the hits left wait: their words move to the front of the list, counted from k0
+        left = k0 < total ? total - k0 : 0u;
+        left_m = m;
+        left_w = 0;
+        if (left > 0) {
+            const uint32_t from = (m & 1u) ? word + 8u : word;  // the first hit's word
+            left_w = __popc(m | 1u);
+            uint2 wd = make_uint2(0u, 0u);
+            if (lane < left_w) wd = lds64(from + 8u * lane);
+            __syncwarp();
+            if (lane < left_w) sts64(list + 8u * lane, make_uint2(wd.x + k0, wd.y));
+        }
+        __syncwarp();
     }
 }
 
@@ -793,64 +749,105 @@ __device__ __forceinline__ void publish_subject(const Finder &f, const ScanArgs 
     }
 }
 
-// A group about to be scanned: its subjects [lo, lo + ns), its residues (at
-// o0) and whether they are on their way to the stage buffer.
+// Subjects about to be scanned together: the first, its residues (at o0) and
+// whether they are on their way to the stage buffer.
 struct Group {
-    uint32_t lo, ns;
+    uint32_t lo;
     uint64_t o0;
     bool staged;
 };
 
-// Reads the bounds of group g and, when it fits and `staging` is on, starts
-// its copy to the stage buffer.
-__device__ __forceinline__ Group fetch_group(Finder &f, const ScanArgs &a, const Ctx &c, uint32_t g, bool staging) {
+// Takes the subjects [lo, hi) of a group -- or only the first, when they do
+// not fit the stage buffer or `staging` is off -- and starts their copies to
+// the stage buffer, each lane its subject's.
+__device__ __forceinline__ Group fetch_group(Finder &f, const ScanArgs &a, const Ctx &c, uint32_t lo, uint32_t hi,
+                                             bool staging) {
     const uint32_t lane = threadIdx.x & 31;
     Group r;
-    r.lo = a.groups[g + 1];
-    r.ns = a.groups[g] - r.lo;  // 1 .. kGroupMaxSubjects
-    const uint64_t mine = a.off[r.lo + min(lane, r.ns)];
+    r.lo = lo;
+    f.ns = hi - lo;  // 1 .. kGroupMaxSubjects
+    const uint64_t mine = a.off[lo + min(lane, f.ns)];
     r.o0 = __shfl_sync(kFull, mine, 0);
-    f.rel = static_cast<uint32_t>(mine - r.o0);
-    const uint32_t len = __shfl_sync(kFull, f.rel, r.ns);
-    r.staged = staging && len >= static_cast<uint32_t>(kWordSize) && len <= a.stage_bytes;
-    if (r.staged && lane == 0) {
-        const uint32_t lead = static_cast<uint32_t>(r.o0 & 15u);
-        const uint32_t bytes = (lead + len + 15u) & ~15u;  // the database is padded
-        bulk_stage(f.w + kDiagAt + c.diag_bytes, a.res + (r.o0 - lead), bytes, f.w + kBarAt);
+    const uint64_t next = __shfl_down_sync(kFull, mine, 1);
+    const uint32_t lead = static_cast<uint32_t>(mine & 15u);
+    uint32_t len = lane < f.ns ? static_cast<uint32_t>(next - mine) : 0u;
+    // a subject's block: what precedes it in its first 16 bytes, it, two zeros
+    const uint32_t block = lane < f.ns ? (lead + len + 2u + 15u) & ~15u : 0u;
+    const uint32_t to = warp_prefix(block);
+    auto fits = [&](uint32_t n) {
+        const uint32_t need = __shfl_sync(kFull, to, n - 1u);
+        return staging && need <= scan_stage_blocks(a.stage_bytes) &&
+               (n == 1u || need + static_cast<uint32_t>(c.window) * n <= kPackSpan - kChunk);
+    };
+    r.staged = fits(f.ns);
+    if (!r.staged && f.ns > 1) {
+        f.ns = 1;
+        r.staged = fits(1);
+    }
+    const bool has = lane < f.ns;
+    if (!has) len = 0u;
+    f.first = has ? (r.staged ? to - block + lead : 0u) : 0x7fffffffu;
+    f.end = f.first + len;
+    if (r.staged) {
+        const uint32_t bytes = has ? (lead + len + 15u) & ~15u : 0u;  // the database is padded
+        const uint32_t all = __reduce_add_sync(kFull, bytes);
+        if (lane == 0) stage_expect(all, f.w + kBarAt);
+        __syncwarp();
+        if (bytes) bulk_stage(f.w + kDiagAt + c.diag_bytes + to - block, a.res + (mine - lead), bytes, f.w + kBarAt);
     }
     return r;
 }
 
-// The diagonal table as empty, values from 0 on.
-template <bool QS>
-__device__ __forceinline__ void clear_table(Finder &f, const Ctx &c) {
-    for (uint32_t i = 4u * (threadIdx.x & 31); i < c.diag_bytes; i += 128u) sts32(f.w + kDiagAt + i, 0u);
-    f.base = 0;
+// Zeros around the staged subjects, and for a chunk's reads past the last.
+__device__ __forceinline__ void clear_margins(const Finder &f, uint32_t stage) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t first = stage + f.first, end = stage + f.end;
+    const uint32_t next = (end + 2u + 15u) & ~15u;  // of the block after the subject's
+    if (lane < f.ns) {
+        // whole words and then bytes up to the subject, bytes and then whole words behind it
+        for (uint32_t i = first & ~15u; i + 4u <= first; i += 4u) sts32(i, 0u);
+        for (uint32_t i = first & ~3u; i < first; ++i) smem[i] = 0;
+        for (uint32_t i = end; (i & 3u) != 0u; ++i) smem[i] = 0;
+        for (uint32_t i = (end + 3u) & ~3u; i < next; i += 4u) sts32(i, 0u);
+    }
+    const uint32_t last = __shfl_sync(kFull, next, f.ns - 1u);
+    sts32(last + 4u * lane, 0u);
+    if (lane < kScanStageSlack / 4u - 32u) sts32(last + 128u + 4u * lane, 0u);
     __syncwarp();
 }
 
-// The subjects of a fetched group for the query of `c`: finds their init hits
-// and publishes each subject's. False when the staging copy never landed.
+// The diagonal table as empty: every hit to come is `window` or more past 0.
+template <bool QS>
+__device__ __forceinline__ void clear_table(Finder &f, const Ctx &c) {
+    for (uint32_t i = 4u * (threadIdx.x & 31); i < c.diag_bytes; i += 128u) sts32(f.w + kDiagAt + i, 0u);
+    f.base = static_cast<uint32_t>(c.window);
+    __syncwarp();
+}
+
+// The fetched subjects for the query of `c`: finds their init hits and
+// publishes each subject's. False when a staging copy never landed.
 template <bool QS, bool WT>
 __device__ __forceinline__ bool process_group(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, WT> &q,
                                               const Group &g, uint32_t query_index) {
     const uint32_t lane = threadIdx.x & 31;
     f.n_init = 0;
-    f.xb = 0;
-    f.xs = g.ns > 1 ? kGroupBits : 0;
-    if (f.base + __shfl_sync(kFull, f.rel, g.ns) + static_cast<uint32_t>(c.window) * (g.ns + 1u) > Tab<QS>::kMost)
-        clear_table<QS>(f, c);
+    f.vb = 0;
+    // the values the group's hits take, with the distance to the next group's
+    const uint32_t extent = __shfl_sync(kFull, f.end, f.ns - 1u) + static_cast<uint32_t>(c.window) * f.ns;
+    if (f.base + extent > Tab<QS>::kMost) clear_table<QS>(f, c);
+    const bool long_one = QS ? f.base + extent > Tab<QS>::kMost : extent > kPackSpan - kChunk;
     if (g.staged) {
         if (!stage_wait(f, a)) return false;
         Span<true> span;
-        span.off = f.w + kDiagAt + c.diag_bytes + static_cast<uint32_t>(g.o0 & 15u);
+        span.off = f.w + kDiagAt + c.diag_bytes;
         span.ptr = nullptr;
-        scan_span(f, a, c, q, span, g.ns);
-    } else {
+        clear_margins(f, span.off);
+        scan_span(f, a, c, q, span, long_one);
+    } else {  // one subject
         Span<false> span;
         span.off = 0;
         span.ptr = a.res + g.o0;
-        scan_span(f, a, c, q, span, g.ns);
+        scan_span(f, a, c, q, span, long_one);
     }
     if (f.n_init > a.scratch_cap) {
         if (lane == 0) {
@@ -859,9 +856,9 @@ __device__ __forceinline__ bool process_group(Finder &f, const ScanArgs &a, cons
         }
     } else if (f.n_init > 0) {
         __syncwarp();  // the records in scratch were written by several lanes
-        for (uint32_t i = 0; i < g.ns; ++i) {
-            const int32_t x0 = static_cast<int32_t>(__shfl_sync(kFull, f.rel, i));
-            const int32_t x1 = static_cast<int32_t>(__shfl_sync(kFull, f.rel, i + 1u));
+        for (uint32_t i = 0; i < f.ns; ++i) {
+            const int32_t x0 = static_cast<int32_t>(__shfl_sync(kFull, f.first, i));
+            const int32_t x1 = static_cast<int32_t>(__shfl_sync(kFull, f.end, i));
             uint32_t n = 0;
             for (uint32_t i0 = 0; i0 < f.n_init; i0 += 32) {
                 const int32_t t = i0 + lane < f.n_init ? scratch_of(a)[i0 + lane].s_trig : -1;
@@ -870,7 +867,7 @@ __device__ __forceinline__ bool process_group(Finder &f, const ScanArgs &a, cons
             if (n) publish_subject(f, a, g.lo + i, x0, x1, n, query_index);
         }
     }
-    f.base += __shfl_sync(kFull, f.rel, g.ns) + static_cast<uint32_t>(c.window) * g.ns;
+    f.base += extent;
     if (f.hits >> 26) add_counts(f, a);
     __syncwarp();
     return true;
@@ -887,9 +884,9 @@ __device__ __forceinline__ void start_region(Finder &f, uint32_t w) {
     __syncwarp();
 }
 
-__device__ __forceinline__ void load_matrix8() {
+__device__ __forceinline__ void load_matrix() {
     for (int i = threadIdx.x; i < kAlphabet * kAlphabet; i += blockDim.x)
-        reinterpret_cast<int8_t *>(smem)[kMatOff + i] = g_blosum8[i];
+        reinterpret_cast<int32_t *>(smem + kMatOff)[i] = static_cast<int32_t>(g_blosum8[i]) * (1 << kKeyBits) - 1;
 }
 
 // One query against the whole database: the query's word table (or its
@@ -917,9 +914,13 @@ scan_kernel(const ScanArgs a) {
     // blocks; its copy runs while the block fills its tables
     unsigned long long t = static_cast<unsigned long long>(warp) * gridDim.x + blockIdx.x;
     Group g{};
-    if (t < a.n_groups) g = fetch_group(f, a, c, static_cast<uint32_t>(t), true);
+    uint32_t hi = 0;
+    if (t < a.n_groups) {
+        hi = a.groups[t];
+        g = fetch_group(f, a, c, a.groups[t + 1], hi, true);
+    }
     clear_table<QS>(f, c);
-    load_matrix8();
+    load_matrix();
     if (WT) {
         uint16_t *tab = reinterpret_cast<uint16_t *>(smem + kTabOff);
         for (uint32_t i = threadIdx.x; i <= kWords; i += blockDim.x) tab[i] = static_cast<uint16_t>(a.cell_start[i]);
@@ -934,9 +935,15 @@ scan_kernel(const ScanArgs a) {
     q.len = a.qlen;
     while (t < a.n_groups) {
         if (!process_group(f, a, c, q, g, a.query_index)) return;
-        if (lane == 0) t = atomicAdd(a.cursor, 1ull) + static_cast<unsigned long long>(gridDim.x) * (blockDim.x >> 5);
-        t = __shfl_sync(kFull, t, 0);
-        if (t < a.n_groups) g = fetch_group(f, a, c, static_cast<uint32_t>(t), true);
+        uint32_t lo = g.lo + f.ns;
+        if (lo == hi) {
+            if (lane == 0) t = atomicAdd(a.cursor, 1ull) + static_cast<unsigned long long>(gridDim.x) * (blockDim.x >> 5);
+            t = __shfl_sync(kFull, t, 0);
+            if (t >= a.n_groups) break;
+            lo = a.groups[t + 1];
+            hi = a.groups[t];
+        }
+        g = fetch_group(f, a, c, lo, hi, true);
     }
     add_counts(f, a);
 }
@@ -960,7 +967,7 @@ scan_batch_kernel(const ScanArgs a) {
     __shared__ uint32_t s_next;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t n_warps = blockDim.x >> 5;
-    load_matrix8();
+    load_matrix();
     const uint32_t regions = kQueryOff<false> + a.query_smem_bytes;
     Finder f{};
     const unsigned long long n_tiles = static_cast<unsigned long long>(a.n_ranges) * a.n_queries;
@@ -981,7 +988,7 @@ scan_batch_kernel(const ScanArgs a) {
             for (int i = threadIdx.x; i < bq.qlen; i += blockDim.x) smem[kQueryOff<false> + i] = bq.q[i];
         __syncthreads();
         const uint32_t warp_bytes = scan_warp_bytes(bq.diag_bytes, a.stage_bytes);
-        const uint32_t active = min(n_warps, (a.smem_bytes - kScanSlackBytes - regions) / warp_bytes);  // >= 1 (host)
+        const uint32_t active = min(n_warps, (a.smem_bytes - regions) / warp_bytes);  // >= 1 (host)
         if (warp < active) {
             Ctx c;
             c.qlen = bq.qlen;
@@ -1001,14 +1008,19 @@ scan_batch_kernel(const ScanArgs a) {
             q.ptr = bq.q;
             q.len = bq.qlen;
             const uint32_t g0 = a.tile_bounds[range], g1 = a.tile_bounds[range + 1];
-            for (;;) {
-                uint32_t k = 0;
-                if (lane == 0) k = atomicAdd(&s_next, 1u);
-                k = __shfl_sync(kFull, k, 0);
-                if (k >= g1 - g0) break;
+            for (uint32_t lo = 0, hi = 0;;) {
+                if (lo == hi) {
+                    uint32_t k = 0;
+                    if (lane == 0) k = atomicAdd(&s_next, 1u);
+                    k = __shfl_sync(kFull, k, 0);
+                    if (k >= g1 - g0) break;
+                    lo = a.groups[g0 + k + 1];
+                    hi = a.groups[g0 + k];
+                }
                 // after a copy that never landed: read this and every later
-                // group from global memory (the host reports the run as failed)
-                while (!process_group(f, a, c, q, fetch_group(f, a, c, g0 + k, staging), bq.index)) staging = false;
+                // subject from global memory (the host reports the run as failed)
+                while (!process_group(f, a, c, q, fetch_group(f, a, c, lo, hi, staging), bq.index)) staging = false;
+                lo += f.ns;
             }
             __syncwarp();
             if (lane == 0) mbar_inval(smem_base() + f.w + kBarAt);
@@ -1029,7 +1041,7 @@ ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t n_hits, uint32_t s
     l.query_smem_bytes = scan_query_in_smem(qlen, window) ? (static_cast<uint32_t>(qlen) + 15u) & ~15u : 0u;
     l.warp_smem_bytes = scan_warp_bytes(l.diag_bytes, stage_bytes);
     auto fit = [&](size_t tab) {
-        const size_t fixed = kScanMatBytes + tab + l.query_smem_bytes + kScanSlackBytes;
+        const size_t fixed = kScanMatBytes + tab + l.query_smem_bytes;
         int w = std::max(1, std::min(max_warps, kScanMaxWarpsPerBlock));
         while (w > 1 && fixed + static_cast<size_t>(w) * l.warp_smem_bytes > smem_budget) --w;
         l.warps_per_block = w;
