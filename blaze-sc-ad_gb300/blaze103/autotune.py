@@ -3,12 +3,12 @@
 For each named shape (a query-length profile, a batch size and a database
 size) it times the search over a grid of launch settings with CUDA events --
 the subject staging bound (subjects up to `stage_bytes` residues are staged in
-shared memory, longer ones are read from global memory), warps per scan block,
-residues per batched tile and the batched launch mode (tiles of many queries
-per launch, or one launch per query) -- checks that every setting returns the
-same HSPs, and writes the fastest setting per shape to ``tuning.json`` beside
-this file. ``lookup`` returns the entry of the nearest shape; ``PrelimSearch``
-applies it to batched runs unless a tuning was set explicitly.
+shared memory, longer ones are read from global memory) and warps per scan
+block -- checks that every setting returns the same HSPs, and writes the fastest
+setting per shape to ``tuning.json`` beside this file. ``lookup`` returns the
+entry of the nearest shape; ``PrelimSearch`` applies it to batched runs unless
+a tuning was set explicitly. The batched launch mode stays automatic: it goes
+by the database's longest subject, which a shape does not tell.
 
 Run on the GPU:  python blaze-sc-ad_gb300/blaze103/autotune.py [--quick]
 """
@@ -28,24 +28,17 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 TUNING_PATH = os.path.join(HERE, "tuning.json")
 
 # shapes: (kind, synthetic workload, scale of its database, queries, grid,
-# timed repetitions). Knobs: the subject staging bound, warps per scan block
-# (0: as many as registers allow), residues per warp of a batched tile (0:
-# several tiles' worth per warp) and the batched launch mode (1: tiles of
-# many queries per launch, 2: one scan launch per query).
-_SMALL_BATCH_GRID = {
-    "stage_bytes": (1024, 2048),
-    "max_warps_per_block": (16, 0),
-    "tile_residues": (0, 4096, 65536),
-    "batch_launch": (1, 2),
-}
+# timed repetitions). Knobs: the subject staging bound and warps per scan block
+# (0: as many as registers allow).
+_SMALL_BATCH_GRID = {"stage_bytes": (1024, 2048), "max_warps_per_block": (16, 0)}
 SHAPES = {
     "plain-db-scale": ("plain", "plain-db-scale", 1.0, 8,
                        {"stage_bytes": (1024, 2048, 4096), "max_warps_per_block": (8, 16, 0)}, 3),
     "batched-512": ("batched", "batched", 0.02, 512, _SMALL_BATCH_GRID, 3),
-    "batched-512-full": ("batched", "batched", 1.0, 512, {"stage_bytes": (1024, 2048), "batch_launch": (1, 2)}, 1),
+    "batched-512-full": ("batched", "batched", 1.0, 512, {"stage_bytes": (1024, 2048)}, 1),
     "batched-64": ("batched", "batched", 0.02, 64, _SMALL_BATCH_GRID, 3),
     "serving-32": ("batched", "serving", 0.01, 32, _SMALL_BATCH_GRID, 3),
-    "serving-4-large": ("batched", "serving", 0.1, 4, {"stage_bytes": (1024, 2048), "batch_launch": (1, 2)}, 3),
+    "serving-4-large": ("batched", "serving", 0.1, 4, {"stage_bytes": (1024, 2048)}, 3),
 }
 DEFAULT = {"stage_bytes": 1024, "max_warps_per_block": 0, "tile_residues": 0, "batch_launch": 0}
 

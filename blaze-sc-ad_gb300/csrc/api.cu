@@ -263,7 +263,6 @@ extern "C" int blaze_search_free(blaze_search *s) {
     cudaSetDevice(s->db->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
-    for (auto &kv : s->tile_bounds) kv.second.release();
     s->scratch.release();
     s->init_out.release();
     s->init_sorted.release();
@@ -360,12 +359,13 @@ struct ScanLaunch {
     ScanArgs sa;
     int blocks, warps_per_block;
     size_t smem_bytes;
-    bool tiles;  // the batched (tiled) kernel, else the single-query one
+    bool queue;  // the batched kernel, else the single-query one
     bool word_table;
 };
 
 struct PassLaunch {
     std::vector<ScanLaunch> scans;
+    uint32_t n_cursors;
     const GappedArgs *ga;
     bool batched;
     bool split;  // the gapped stage as prep, lane-parallel DP and finishing kernels
@@ -381,11 +381,11 @@ constexpr uint32_t kGappedSplitMinQueries = 16;
 static cudaError_t enqueue_pass(blaze_search *s, const PassLaunch &pl, unsigned event_flags) {
     cudaError_t e = cudaMemsetAsync(s->d_cnt, 0, sizeof(DevCounters), s->stream);
     if (e == cudaSuccess)
-        e = cudaMemsetAsync(s->cursors.p, 0, sizeof(unsigned long long) * pl.scans.size(), s->stream);
+        e = cudaMemsetAsync(s->cursors.p, 0, sizeof(unsigned long long) * pl.n_cursors, s->stream);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(s->ev[1], s->stream, event_flags);
     for (const ScanLaunch &l : pl.scans) {
         if (e != cudaSuccess) break;
-        e = l.tiles ? launch_scan_batch(l.sa, l.blocks, l.warps_per_block, l.smem_bytes, s->stream)
+        e = l.queue ? launch_scan_batch(l.sa, l.word_table, l.blocks, l.warps_per_block, l.smem_bytes, s->stream)
                        : launch_scan(l.sa, l.word_table, l.blocks, l.warps_per_block, l.smem_bytes, s->stream);
     }
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(s->ev[2], s->stream, event_flags);
@@ -471,41 +471,8 @@ struct ScanPlan {
     ScanLayout lay;
     int blocks = 0;
     uint32_t first = 0, n = 1;
-    uint32_t tile_residues = 0;
-    bool tiles = false;  // batched: tiles of the plan's queries; else one query's launch
+    bool queue = false;  // the batched kernel over the plan's queries; else one query's launch
 };
-
-// Ranges of groups of about `target` residues, from the longest subjects
-// down (n_ranges + 1 bounds), uploaded once per tile size.
-static int tile_bounds_for(blaze_search *s, uint32_t target, const uint32_t **bounds, uint32_t *n_ranges) {
-    auto it = s->tile_bounds.find(target);
-    if (it == s->tile_bounds.end()) {
-        const std::vector<uint64_t> &off = s->db->h_off;
-        const std::vector<uint32_t> &groups = s->db->h_groups;
-        const uint32_t n = static_cast<uint32_t>(groups.size()) - 1;
-        std::vector<uint32_t> b{0};
-        for (uint32_t lo = 0; lo < n;) {
-            uint32_t hi = lo + 1;
-            while (hi < n && off[groups[lo]] - off[groups[hi + 1]] <= target) ++hi;
-            b.push_back(hi);
-            lo = hi;
-        }
-        DevBuf<uint32_t> d;
-        int rc = d.ensure(b.size());
-        if (rc != BLAZE_OK) return rc;
-        cudaError_t e = cudaMemcpy(d.p, b.data(), sizeof(uint32_t) * b.size(), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) {
-            d.release();
-            BLAZE_CUDA_TRY(e);
-        }
-        s->stats.h2d_bytes += sizeof(uint32_t) * b.size();
-        it = s->tile_bounds.emplace(target, d).first;
-        s->tile_ranges[target] = static_cast<uint32_t>(b.size() - 1);
-    }
-    *bounds = it->second.p;
-    *n_ranges = s->tile_ranges[target];
-    return BLAZE_OK;
-}
 
 // One pass of both stages; fills s->h_cnt.
 static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPlan> &plans) {
@@ -538,11 +505,12 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
     // rows start 8-byte aligned (the DP reads and writes column pairs)
     const size_t dp_stride = (static_cast<size_t>(std::max<uint32_t>(db->max_len, 1)) + 3) & ~size_t{1};
     if ((rc = s->dp.ensure(gapped_warps * 2 * dp_stride)) != BLAZE_OK) return rc;
-    if ((rc = s->cursors.ensure(plans.size())) != BLAZE_OK) return rc;
+    if ((rc = s->cursors.ensure(nq)) != BLAZE_OK) return rc;
 
     PassLaunch pl;
     pl.batched = batched;
     pl.split = split;
+    pl.n_cursors = nq;
     for (const ScanPlan &plan : plans) {
         const ScanLayout &lay = plan.lay;
         ScanLaunch l;
@@ -572,9 +540,9 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
         sa.work = s->work.p;
         sa.work_cap = work_cap;
         sa.cnt = s->d_cnt;
-        sa.cursor = s->cursors.p + pl.scans.size();
-        l.tiles = plan.tiles;
-        if (batched && !plan.tiles) {
+        sa.cursor = s->cursors.p + plan.first;
+        l.queue = plan.queue;
+        if (batched && !plan.queue) {
             // one query of the batch with the single-query kernel; its work
             // items carry the query's batch index
             const uint32_t i = r.border[plan.first];
@@ -592,10 +560,6 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
         } else if (batched) {
             sa.queries = s->bq.p + plan.first;
             sa.n_queries = plan.n;
-            // a tile is one block's work: tile_residues per warp
-            const uint32_t block_tile = static_cast<uint32_t>(std::min<uint64_t>(
-                static_cast<uint64_t>(plan.tile_residues) * static_cast<uint64_t>(lay.warps_per_block), 1u << 31));
-            if ((rc = tile_bounds_for(s, block_tile, &sa.tile_bounds, &sa.n_ranges)) != BLAZE_OK) return rc;
             sa.work_query = s->work_query.p;
         } else {
             const blaze_query *q = r.q;
@@ -699,38 +663,29 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     // layout of one single-query scan launch
     const uint32_t stage_bytes = std::max(s->stage_bytes, db->group_bytes);
     constexpr size_t kSmemMost = 227 * 1024 - 64;  // the opt-in limit less static shared memory
-    auto layout_for = [&](int32_t qlen, uint32_t n_hits) {
-        ScanLayout l = scan_layout(qlen, p0->window, n_hits, stage_bytes, kSmemBudget, warp_cap);
+    auto layout_for = [&](int32_t qlen, uint32_t n_hits, int warps) {
+        ScanLayout l = scan_layout(qlen, p0->window, n_hits, stage_bytes, kSmemBudget, warps);
         // next to the longest tables only smaller groups are staged
         if (l.smem_bytes > kSmemMost)
-            l = scan_layout(qlen, p0->window, n_hits, std::max(s->stage_bytes, 160u) - 160u, kSmemBudget, warp_cap);
+            l = scan_layout(qlen, p0->window, n_hits, std::max(s->stage_bytes, 576u) - 576u, kSmemBudget, warps);
         return l;
     };
     // layout of one batched scan launch over queries of up to `longest`
     // residues: shared memory for all the block's warps at the longest query
     // when that fits the budget, else the whole budget (at least one warp);
-    // each tile runs as many warps as fit for its own query
-    auto batch_layout_for = [&](int32_t longest) {
-        ScanLayout l{};
-        auto warp_bytes = [&](int32_t qlen) {
-            return static_cast<size_t>(scan_warp_bytes(scan_diag_bytes(qlen, p0->window), stage_bytes));
-        };
-        const int w = std::max(1, std::min(warp_cap, kScanMaxWarpsPerBlock));
-        l.query_smem_bytes = scan_query_in_smem(longest, p0->window) ? (static_cast<uint32_t>(longest) + 15u) & ~15u : 0u;
-        const size_t regions = kScanMatBytes + kScanPresenceBytes + l.query_smem_bytes;
-        l.smem_bytes = std::max(std::min(kSmemBudget, regions + static_cast<size_t>(w) * warp_bytes(longest)),
-                                regions + warp_bytes(longest));
-        l.warps_per_block = w;
-        l.stage_bytes = stage_bytes;
-        l.diag_entries = scan_diag_entries(longest, p0->window);
-        l.diag_magic = static_cast<uint32_t>((1ull << 32) / l.diag_entries + 1);
-        l.diag_bytes = scan_diag_bytes(longest, p0->window);
-        l.warp_smem_bytes = static_cast<uint32_t>(warp_bytes(longest));
+    // the block runs as many warps as fit for each query
+    auto batch_layout_for = [&](int32_t longest, bool word_table) {
+        ScanLayout l = layout_for(longest, UINT32_MAX, 1);
+        const size_t regions = l.smem_bytes - l.warp_smem_bytes + (word_table ? kScanWordTabBytes - kScanPresenceBytes : 0);
+        l.word_table = word_table;
+        l.warps_per_block = std::max(1, std::min(warp_cap, kScanMaxWarpsPerBlock));
+        l.smem_bytes = std::max(std::min(kSmemBudget, regions + static_cast<size_t>(l.warps_per_block) * l.warp_smem_bytes),
+                                regions + l.warp_smem_bytes);
         return l;
     };
-    // Batched: one scan launch for the queries whose residues fit the
-    // block's shared-memory copy and one for any longer ones (their tiles
-    // size the warps' tables per query).
+    // Batched: the queries in length order, one scan launch for those that
+    // take the same kernel (the query in shared memory or not, its word table
+    // or not).
     std::vector<uint32_t> order(nq);
     std::iota(order.begin(), order.end(), 0u);
     if (batched)
@@ -738,66 +693,44 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
                          [&](uint32_t a, uint32_t b) { return r.b->qlen[a] < r.b->qlen[b]; });
     auto qlen_at = [&](uint32_t k) { return batched ? r.b->qlen[order[k]] : r.q->qlen; };
     std::vector<ScanPlan> plans;
-    // A launch's shared memory fixes the SM's L1 share for all of it, and the
-    // L1 keeps the word tables the finder reads per position; so batched
-    // queries are grouped by the shared-memory step (of the SM's carve-out
-    // choices) that all the block's warps need for them, each group one launch
-    // sized for its longest query -- what a single-query launch does per query.
-    auto smem_step = [&](int32_t qlen) {
-        constexpr size_t kSteps[] = {100u << 10, 132u << 10, 164u << 10, 196u << 10};
-        const size_t need = batch_layout_for(qlen).smem_bytes;
-        int k = 0;
-        while (k < 4 && need > kSteps[k]) ++k;
-        return k + (scan_query_in_smem(qlen, p0->window) ? 0 : 8);  // longer queries stay in global memory: own launch
+    auto query_layout = [&](uint32_t k) {
+        return layout_for(qlen_at(k), batched ? r.b->n_off[order[k]] : r.q->n_off, warp_cap);
     };
-    // batched runs of few queries, or on a large database, launch the
-    // single-query kernel once per query (a query alone fills the GPU there,
-    // and that kernel is the faster per residue); the tiles pay off where
-    // many per-query launches would each be short
-    constexpr uint64_t kPerQueryLaunchResidues = 1ull << 27;
-    constexpr uint32_t kPerQueryLaunchQueries = 16;
-    const bool per_query = batched && (s->batch_launch == 2 ||
-                                       (s->batch_launch == 0 && (db->total >= kPerQueryLaunchResidues ||
-                                                                 nq <= kPerQueryLaunchQueries)));
+    // A batch runs as one launch whose blocks go from query to query where a
+    // query's own pass would end in a wait for its longest subjects, that is
+    // where one of them is more than a warp's share of the residues: 16 queries
+    // of 2,000 to 5,000 residues against 10.7 M residues with subjects of up to
+    // 35,000 scan in 14.4 ms instead of 104.2. Otherwise one launch per query
+    // is the faster (256 queries against 35 M residues 117.2 ms and 120.1).
+    const uint64_t share = db->total / (static_cast<uint64_t>(s->n_sm) * kScanMaxWarpsPerBlock);
+    const bool per_query = batched && (s->batch_launch == 2 || (s->batch_launch == 0 && (nq == 1 || db->max_len < share)));
     r.border = order;
     for (uint32_t i = 0; i < nq;) {
         uint32_t j = i + 1;
-        if (batched && !per_query) {
-            const int step = smem_step(qlen_at(i));
-            while (j < nq && smem_step(qlen_at(j)) == step) ++j;
-        }
         ScanPlan pl;
-        pl.tiles = batched && !per_query;
-        pl.lay = pl.tiles ? batch_layout_for(qlen_at(j - 1)) : layout_for(qlen_at(i), batched ? r.b->n_off[order[i]] : r.q->n_off);
+        pl.lay = query_layout(i);
+        pl.queue = batched && !per_query;
+        if (pl.queue) {
+            const bool smem = pl.lay.query_smem_bytes != 0, table = pl.lay.word_table;
+            for (; j < nq; ++j) {
+                const ScanLayout l = query_layout(j);
+                if ((l.query_smem_bytes != 0) != smem || l.word_table != table) break;
+            }
+            pl.lay = batch_layout_for(qlen_at(j - 1), table);
+        }
         pl.first = i;
         pl.n = j - i;
         if (pl.lay.smem_bytes > kSmemMost) return BLAZE_ERR_LIMIT;
         int per_sm = 0;
-        if (pl.tiles) {
-            BLAZE_CUDA_TRY(scan_batch_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.warps_per_block, pl.lay.smem_bytes,
-                                                &per_sm));
+        if (pl.queue) {
+            BLAZE_CUDA_TRY(scan_batch_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.word_table, pl.lay.warps_per_block,
+                                                pl.lay.smem_bytes, &per_sm));
         } else {
             BLAZE_CUDA_TRY(scan_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.word_table, pl.lay.warps_per_block,
                                           pl.lay.smem_bytes, &per_sm));
         }
         if (per_sm < 1) return BLAZE_ERR_LIMIT;
         pl.blocks = s->n_sm * per_sm;
-        if (pl.tiles) {
-            if (s->tile_residues) {
-                pl.tile_residues = s->tile_residues;
-            } else {
-                // about 16 tiles per block (its warps wait for the last one
-                // at each tile's end, so larger tiles waste less), at most
-                // kMaxTileResidues per warp; a power of two so that few
-                // distinct bound tables exist
-                const uint64_t per_block = db->total * pl.n / (16ull * static_cast<uint64_t>(pl.blocks));
-                uint64_t t = std::max<uint64_t>(per_block / static_cast<uint64_t>(pl.lay.warps_per_block), 1);
-                t = std::min<uint64_t>(t, kMaxTileResidues);
-                uint32_t pow2 = 1;
-                while (static_cast<uint64_t>(pow2) * 2 <= t) pow2 *= 2;
-                pl.tile_residues = pow2;
-            }
-        }
         plans.push_back(pl);
         i = j;
     }
@@ -1062,7 +995,6 @@ extern "C" int blaze_search_set_tuning(blaze_search *s, const blaze_tuning *t) t
     s->launch_mode = t->launch_mode;
     s->batch_launch = t->batch_launch;
     s->stage_bytes = t->stage_bytes ? t->stage_bytes : kScanStageBytes;
-    s->tile_residues = t->tile_residues;
     s->max_warps = t->max_warps_per_block;
     return BLAZE_OK;
 } BLAZE_ABI_CATCH

@@ -40,7 +40,6 @@ constexpr uint32_t kScanWordTabHits = 65535;  // hit-list entries a 16-bit word 
 constexpr int32_t kQuerySmemMax = 8192;      // queries up to this length live in shared memory,
 constexpr int32_t kTab16Window = 256;        // for windows up to this one: 16-bit diagonal tables
 constexpr uint32_t kScanStageBytes = 1024;   // subjects up to this length are staged
-constexpr uint32_t kMaxTileResidues = 1u << 16;  // automatic tile size at most (residues per warp)
 
 inline bool scan_query_in_smem(int32_t qlen, int32_t window) { return qlen <= kQuerySmemMax && window <= kTab16Window; }
 inline uint32_t scan_diag_entries(int32_t qlen, int32_t window) {  // >= qlen + window
@@ -153,8 +152,6 @@ struct ScanArgs {
     // batched launches only
     const BatchQuery *queries;   // n_queries descriptors
     uint32_t n_queries;
-    const uint32_t *tile_bounds;  // n_ranges + 1 group indices, ascending: range r is [b[r], b[r+1])
-    uint32_t n_ranges;
     uint32_t *work_query;        // query index of each work item (nullptr: one query)
     uint32_t query_index;        // single-query launches inside a batched pass: the query's index
     InitHit *scratch;          // per warp: scratch_cap records
@@ -164,7 +161,7 @@ struct ScanArgs {
     WorkItem *work;
     unsigned long long work_cap;
     DevCounters *cnt;
-    unsigned long long *cursor;  // this launch's work cursor (zeroed before the pass)
+    unsigned long long *cursor;  // the launch's work cursor, batched: one per query (zeroed before the pass)
 };
 
 struct GappedArgs {
@@ -270,8 +267,10 @@ cudaError_t launch_gapped(const GappedArgs &a, int n_blocks, cudaStream_t st,
 cudaError_t launch_hitlist(const HitlistArgs &a, uint32_t n_select, int n_sm, cudaStream_t st);
 constexpr int kTracebackWarpsPerBlock = 4;
 cudaError_t launch_traceback(const TracebackArgs &a, int n_blocks, cudaStream_t st);
-cudaError_t launch_scan_batch(const ScanArgs &a, int n_blocks, int warps_per_block, size_t smem, cudaStream_t st);
-cudaError_t scan_batch_occupancy(bool query_in_smem, int warps_per_block, size_t smem, int *blocks_per_sm);
+cudaError_t launch_scan_batch(const ScanArgs &a, bool word_table, int n_blocks, int warps_per_block, size_t smem,
+                              cudaStream_t st);
+cudaError_t scan_batch_occupancy(bool query_in_smem, bool word_table, int warps_per_block, size_t smem,
+                                 int *blocks_per_sm);
 int scan_batch_max_warps_by_registers(bool query_in_smem);
 cudaError_t gapped_occupancy(int *blocks_per_sm);
 // The gapped stage as prep, lane-parallel DP and finishing kernels (batched

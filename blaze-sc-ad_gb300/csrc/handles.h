@@ -96,10 +96,6 @@ struct blaze_search {
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     // launch shape (blaze_search_set_tuning)
     uint32_t stage_bytes = kScanStageBytes;
-    uint32_t tile_residues = 0;  // 0: automatic
-    // residue-balanced subject ranges of batched tiles, per tile size
-    std::map<uint32_t, DevBuf<uint32_t>> tile_bounds;
-    std::map<uint32_t, uint32_t> tile_ranges;
     uint32_t max_warps = 0;
     uint32_t launch_mode = 0;
     uint32_t batch_launch = 0;  // blaze_tuning.batch_launch
@@ -113,7 +109,7 @@ struct blaze_search {
     DevBuf<const uint8_t *> bqptr;
     DevBuf<int32_t> bqlen, bcut;
     DevBuf<uint32_t> work_query;
-    DevBuf<unsigned long long> cursors;  // one work cursor per scan launch of a pass
+    DevBuf<unsigned long long> cursors;  // the scan's work cursors, one per query
     // per-query finishing on the device: reap score, max_hsps, published
     // lists per query, and the hit-list selection's segments
     DevBuf<int32_t> bsmin, bmaxh, sel_limit;

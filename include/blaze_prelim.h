@@ -264,8 +264,7 @@ int blaze_search_traceback_batch_results(const blaze_search *s, blaze_batch_alig
 
 /* ---------------------------------------------------------------------
  * Batched form: many queries of uneven length against the database in one
- * persistent launch per stage. Warps pull (query, subject range) tiles from a
- * device work queue, longest subjects first, queries interleaved. All
+ * pass. Each query has a cursor over the database, longest subjects first. All
  * queries of a batch share word_threshold, window, X-drops and gap costs;
  * cutoffs and E-value statistics are per query (params[i]).
  */
@@ -295,10 +294,8 @@ int blaze_search_batch_results(const blaze_search *s, blaze_batch_hsp *out, uint
                                uint64_t *n_hsps);
 
 /* Launch shape of the word finder (0 = library default): subjects up to
- * stage_bytes residues are staged in shared memory; a batched tile is one
- * block's work for one query: consecutive subjects of about tile_residues
- * residues per warp of the block (a longer subject is a tile of its own; 0:
- * sized so that every warp gets several tiles' worth); max_warps_per_block
+ * stage_bytes residues are staged in shared memory; tile_residues has no effect
+ * (the batched form needs no tile size); max_warps_per_block
  * caps the block. */
 typedef struct blaze_tuning {
     uint32_t stage_bytes;
@@ -310,11 +307,11 @@ typedef struct blaze_tuning {
      * The graph is captured once and replayed while the launch arguments stay
      * the same (updated in place when they change). */
     uint32_t launch_mode;
-    /* Batched runs: 0: automatic (one scan launch per query for batches of
-     * at most 16 queries or databases from 2^27 residues on, where a query
-     * alone fills the GPU; tiles of many queries per launch otherwise);
-     * 1: tiles always; 2: one launch per query always. Results are
-     * identical either way. */
+    /* Batched runs: 0: automatic (one scan launch for the whole batch where a
+     * subject is longer than a warp's share of the database, so that the
+     * queries do not wait for their longest subjects one after another; one
+     * launch per query otherwise); 1: one launch for the batch always; 2: one
+     * launch per query always. Results are identical either way. */
     uint32_t batch_launch;
 } blaze_tuning;
 int blaze_search_set_tuning(blaze_search *s, const blaze_tuning *t);
@@ -327,9 +324,8 @@ int blaze_search_set_tuning(blaze_search *s, const blaze_tuning *t);
  * the in-flight batches (word tables plus a per-query allowance for seed and
  * HSP buffers) stays within memory_budget, so batches overlap on the GPU.
  * Each query's HSP lists are handed back when its batch completes. On a
- * database of 2^27 residues or more (unless tuning.batch_launch forces
- * tiles), where a batched run launches the word finder once per query and a
- * query alone fills the GPU, batches take at most 4 queries and run on the
+ * database of 2^27 residues or more (unless tuning.batch_launch is 1), where
+ * a query alone fills the GPU, batches take at most 4 queries and run on the
  * GPU one at a time (the workers' host work still overlaps): batching saves
  * nothing there, and concurrent whole-GPU launches only contend.
  */
