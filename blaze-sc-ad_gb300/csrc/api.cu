@@ -8,6 +8,7 @@
 #include <cstring>
 #include <map>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "handles.h"
@@ -253,6 +254,8 @@ extern "C" int blaze_search_create(blaze_db *db, blaze_search **out) try {
     if (const char *v = std::getenv("BLAZE_INITIAL_INIT_CAP")) s->init_cap = std::max(1, std::atoi(v));
     if (const char *v = std::getenv("BLAZE_INITIAL_OUT_CAP")) s->out_cap = std::max(1, std::atoi(v));
     if (const char *v = std::getenv("BLAZE_INITIAL_WORK_CAP")) s->work_cap = std::max(1, std::atoi(v));
+    // likewise the pass size from which the gapped stage runs one lane per DP
+    if (const char *v = std::getenv("BLAZE_LANE_DP_SLOTS")) s->lane_dp_slots = std::strtoull(v, nullptr, 10);
     if (const char *v = std::getenv("BLAZE_INITIAL_TRACEBACK_CAP")) s->tb_dir_cap = std::max(64, std::atoi(v));
     *out = s;
     return BLAZE_OK;
@@ -265,10 +268,7 @@ extern "C" int blaze_search_free(blaze_search *s) {
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
     s->scratch.release();
     s->init_out.release();
-    s->init_sorted.release();
-    s->dtask.release();
-    s->dres.release();
-    s->sorted.release();
+    s->gapped_ws.release();
     s->work.release();
     s->saved.release();
     s->out.release();
@@ -368,15 +368,11 @@ struct PassLaunch {
     uint32_t n_cursors;
     const GappedArgs *ga;
     bool batched;
-    bool split;  // the gapped stage as prep, lane-parallel DP and finishing kernels
 };
 
-// Batched passes of at least this many queries run the gapped stage with one
-// lane per DP: they hold enough DPs (thousands per SM) for its throughput,
-// while a pass of one or a few queries finishes sooner with a warp per
-// subject (a lane's DP takes too long for a pass that gives each lane one or
-// two of them).
-constexpr uint32_t kGappedSplitMinQueries = 16;
+// Batched passes of at least this many queries may hold so many init hits
+// (kLaneDpSlots) that one lane per DP is the faster; only the device knows.
+constexpr uint32_t kLaneDpMinQueries = 16;
 
 static cudaError_t enqueue_pass(blaze_search *s, const PassLaunch &pl, unsigned event_flags) {
     cudaError_t e = cudaMemsetAsync(s->d_cnt, 0, sizeof(DevCounters), s->stream);
@@ -389,9 +385,7 @@ static cudaError_t enqueue_pass(blaze_search *s, const PassLaunch &pl, unsigned 
                        : launch_scan(l.sa, l.word_table, l.blocks, l.warps_per_block, l.smem_bytes, s->stream);
     }
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(s->ev[2], s->stream, event_flags);
-    if (e == cudaSuccess)
-        e = pl.split ? launch_gapped_split(*pl.ga, s->gapped_blocks, s->n_sm, s->stream)
-                     : launch_gapped(*pl.ga, s->gapped_blocks, s->stream);
+    if (e == cudaSuccess) e = launch_gapped_split(*pl.ga, s->gapped_blocks, s->n_sm, s->stream);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(s->ev[3], s->stream, event_flags);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(s->h_cnt, s->d_cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, s->stream);
@@ -416,7 +410,7 @@ static int launch_pass_graph(blaze_search *s, const PassLaunch &pl) {
         const auto *c = static_cast<const unsigned char *>(p);
         key.insert(key.end(), c, c + n);
     };
-    const int64_t head[3] = {pl.batched, pl.split, s->gapped_blocks};
+    const int64_t head[2] = {pl.batched, s->gapped_blocks};
     put(head, sizeof(head));
     for (const ScanLaunch &l : pl.scans) {
         put(&l.sa, sizeof(ScanArgs));
@@ -486,18 +480,15 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
     const size_t work_cap = batched ? s->work_cap : std::max<uint32_t>(db->n, 1);
     int rc;
     if ((rc = s->scratch.ensure(scan_warps * s->scratch_cap)) != BLAZE_OK) return rc;
-    if ((rc = s->sorted.ensure(gapped_warps * s->scratch_cap)) != BLAZE_OK) return rc;
     if ((rc = s->saved.ensure(gapped_warps * s->scratch_cap)) != BLAZE_OK) return rc;
     if ((rc = s->init_out.ensure(s->init_cap)) != BLAZE_OK) return rc;
     if ((rc = s->work.ensure(work_cap)) != BLAZE_OK) return rc;
     if ((rc = s->out.ensure(s->out_cap)) != BLAZE_OK) return rc;
     const uint32_t nq = batched ? r.b->n : 1u;
-    const bool split = batched && nq >= kGappedSplitMinQueries;
-    if (split) {  // per init-hit slot: ordered init hit, DP task, two DP results
-        if ((rc = s->init_sorted.ensure(s->init_cap)) != BLAZE_OK) return rc;
-        if ((rc = s->dtask.ensure(s->init_cap)) != BLAZE_OK) return rc;
-        if ((rc = s->dres.ensure(2 * s->init_cap)) != BLAZE_OK) return rc;
-    }
+    // the gapped stage's arrays, per init-hit slot: ordered init hit, DP task,
+    // two DP results, DP order, DPs left
+    const size_t slot_bytes = sizeof(InitHit) + sizeof(DpTask) + 2 * sizeof(int4) + 2 * sizeof(uint32_t);
+    if ((rc = s->gapped_ws.ensure(s->init_cap * slot_bytes)) != BLAZE_OK) return rc;
     if ((rc = s->groups.ensure(s->out_cap)) != BLAZE_OK) return rc;  // a published list holds >= 1 HSP
     if ((rc = s->qkept.ensure(nq)) != BLAZE_OK) return rc;
     if (batched && (rc = s->work_query.ensure(work_cap)) != BLAZE_OK) return rc;
@@ -509,7 +500,6 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
 
     PassLaunch pl;
     pl.batched = batched;
-    pl.split = split;
     pl.n_cursors = nq;
     for (const ScanPlan &plan : plans) {
         const ScanLayout &lay = plan.lay;
@@ -585,7 +575,6 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
     ga.init_cap = s->init_cap;
     ga.n_subj = db->n;
     ga.n_queries = nq;
-    ga.sorted = s->sorted.p;
     ga.saved = s->saved.p;
     ga.cap = s->scratch_cap;
     ga.dp = s->dp.p;
@@ -599,11 +588,17 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
     ga.groups = s->groups.p;
     ga.qkept = s->qkept.p;
     ga.cnt = s->d_cnt;
-    if (split) {
-        ga.init_sorted = s->init_sorted.p;
-        ga.dtask = s->dtask.p;
-        ga.dres = s->dres.p;
-    }
+    unsigned char *ws = s->gapped_ws.p;
+    auto take = [&](auto *&p, size_t n) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(ws);
+        ws += n * sizeof(*p);
+    };
+    take(ga.dres, 2 * s->init_cap);
+    take(ga.dtask, s->init_cap);
+    take(ga.init_sorted, s->init_cap);
+    take(ga.dorder, s->init_cap);
+    take(ga.dleft, s->init_cap);
+    ga.lane_slots = batched && nq >= kLaneDpMinQueries ? s->lane_dp_slots : ~0ull;
     if (batched) {
         ga.work_query = s->work_query.p;
         ga.batch_q = s->bqptr.p;
@@ -622,7 +617,7 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
     BLAZE_CUDA_TRY(cudaMemsetAsync(s->qkept.p, 0, sizeof(uint32_t) * nq, s->stream));
     const bool graph = s->launch_mode == 2 || (s->launch_mode == 0 && batched);
     if ((rc = graph ? launch_pass_graph(s, pl) : launch_pass_direct(s, pl)) != BLAZE_OK) return rc;
-    s->stats.kernel_launches += static_cast<uint32_t>(pl.scans.size()) + 1;
+    s->stats.kernel_launches += static_cast<uint32_t>(pl.scans.size()) + (ga.lane_slots == ~0ull ? 2u : 4u);
     s->stats.d2h_bytes += sizeof(DevCounters);
     BLAZE_CUDA_TRY(cudaStreamSynchronize(s->stream));
     return BLAZE_OK;

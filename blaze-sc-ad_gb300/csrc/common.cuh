@@ -65,7 +65,7 @@ struct WorkItem {
     uint64_t first;    // first record in the init-hit array
 };
 
-// One init hit's gapped extension for the lane-parallel DP: the subject, the
+// One init hit's gapped extension as a DP task: the subject, the
 // query (batched: its index) and the gapped start point. Written by the prep
 // kernel at the init hit's slot; valid = 0 for an init hit that is skipped.
 struct DpTask {
@@ -73,7 +73,9 @@ struct DpTask {
     int32_t slen;
     uint32_t query;
     int32_t q_off, s_off;
-    int32_t valid, pad;
+    int32_t valid;
+    int32_t rank;  // of its init hit in its item (0: the best)
+    uint64_t item;
 };
 
 // A finished gapped HSP as the device writes it (subject = sorted index).
@@ -98,7 +100,8 @@ struct DevCounters {
     unsigned int pad;
     unsigned long long group_count;  // subject HSP lists published (GroupDesc records)
     unsigned long long next_prep;    // gapped prep-kernel work cursor
-    unsigned long long next_dp;      // lane DP task cursor
+    unsigned long long next_dp;      // DP task cursor
+    unsigned long long n_first, n_rest;  // DP tasks: items' best init hits, the others
 };
 
 // One subject's HSP list in the gapped stage's output, after the preliminary
@@ -194,10 +197,13 @@ struct GappedArgs {
     GroupDesc *groups;       // one per published list (null: none written)
     uint32_t *qkept;         // per query: lists published (null: not counted)
     DevCounters *cnt;
-    // the three-kernel form (launch_gapped_split), per init-hit slot
+    // the form by DP tasks (launch_gapped_split), per init-hit slot
     InitHit *init_sorted;    // each item's init hits in processing order
     DpTask *dtask;
     int4 *dres;              // per slot: left and right DP (best, row, column, cells; cells -1: not run)
+    uint32_t *dorder;        // slots in DP order: items' best from the front, the others from the back
+    uint32_t *dleft;         // at an item's first slot: its DPs still to end
+    unsigned long long lane_slots;  // from this many slots on one lane per DP, else one warp
 };
 
 // Hit-list selection: queries that keep more subjects than their
@@ -273,9 +279,8 @@ cudaError_t scan_batch_occupancy(bool query_in_smem, bool word_table, int warps_
                                  int *blocks_per_sm);
 int scan_batch_max_warps_by_registers(bool query_in_smem);
 cudaError_t gapped_occupancy(int *blocks_per_sm);
-// The gapped stage as prep, lane-parallel DP and finishing kernels (batched
-// passes of many queries); n_blocks as for launch_gapped, the DP kernel
-// fills n_sm SMs. Results equal launch_gapped's.
+// The gapped stage as DP tasks; n_blocks as for launch_gapped, the lane DP
+// kernel fills n_sm SMs. Results equal launch_gapped's.
 cudaError_t launch_gapped_split(const GappedArgs &a, int n_blocks, int n_sm, cudaStream_t st);
 
 // Host helpers (host.cpp).

@@ -14,6 +14,9 @@ using namespace blaze;
 
 constexpr uint32_t kMaxSubjectLength = (1u << 28) - 64;  // diagonal table encoding limit
 constexpr int32_t kMaxQueryLength = 32000;                // diagonal table must fit shared memory
+// init hits of a pass from which the gapped stage runs one lane per DP (893,000
+// of them: 18.5 ms, and 20.4 with a warp per DP; 130,000: 5.7 and 3.1 ms)
+constexpr unsigned long long kLaneDpSlots = 600000;
 constexpr uint32_t kInitialScratchCap = 1024;             // init hits per subject before a rerun
 
 struct blaze_db {
@@ -77,18 +80,17 @@ struct blaze_search {
     // per-run capacities
     uint32_t scratch_cap = kInitialScratchCap;
     unsigned long long init_cap = 0, out_cap = 0;
-    DevBuf<InitHit> scratch, init_out, sorted;
+    DevBuf<InitHit> scratch, init_out;
     DevBuf<WorkItem> work;
     DevBuf<DevHsp> saved, out;
     DevBuf<int32_t> dp;
-    DevBuf<InitHit> init_sorted;
-    DevBuf<DpTask> dtask;
-    DevBuf<int4> dres;
+    DevBuf<unsigned char> gapped_ws;  // the gapped stage's arrays per init-hit slot
     DevCounters *d_cnt = nullptr;
     DevCounters *h_cnt = nullptr;  // pinned
     DevHsp *h_out = nullptr;       // pinned
     size_t h_out_n = 0;
     int gapped_blocks = 0;
+    unsigned long long lane_dp_slots = kLaneDpSlots;
     std::vector<blaze_hsp> results;
     blaze_stats stats{};
     unsigned long long last_init_count = 0, last_work_count = 0;

@@ -2,11 +2,15 @@
 // (sm_103a). Integer work only: no tensor cores, no floating point. (The
 // word finder, two-hit and ungapped stage is scan.cu.)
 //
-//   gapped_kernel  one warp per work item: orders the init hits, skips those
-//                  contained in kept HSPs, runs the left and right score-only
-//                  X-drop DP row-parallel across the warp, then purges common
-//                  endpoints, sorts the subject's HSP list and keeps what the
-//                  preliminary reap and max_hsps keep.
+//   gapped_prep_kernel, gapped_warp_dp_kernel (or, for passes of very many init
+//   hits, gapped_dp_kernel and gapped_finish_kernel)
+//                  order each work item's init hits, run the left and right
+//                  score-only X-drop DPs as independent tasks, then skip the
+//                  init hits contained in kept HSPs, purge common endpoints,
+//                  sort the subject's HSP list and keep what the preliminary
+//                  reap and max_hsps keep.
+//   gapped_kernel  the same, one warp per work item, for the allocation-free
+//                  entry point.
 //   hitlist_*      per query, the hitlist_size best subject lists (radix
 //                  select on the device).
 //
@@ -218,6 +222,152 @@ __device__ int32_t xdrop_dp(const uint8_t *__restrict__ A, const uint8_t *__rest
     return best;
 }
 
+// The same DP with the band in registers: a window of 128 columns, two halves
+// of 64, lane i holding H and E of columns w0 + 2i and w0 + 2i + 1 of each. The
+// second half is computed only in rows whose band reaches into it; the window
+// moves right when the band outgrows its first half. Row letter k is
+// Q[dir * k], column letter k is S[dir * k].
+//
+// H of every dead cell is -inf, and E of a dead cell is at most its H was, so
+// nothing outside the band can come back into it from the left or from a stale
+// E; only the band's end is tested. Returns false when the band does not fit
+// the window (nothing is then returned).
+//
+// Bound by instruction issue (80 %): a row takes about 120 warp instructions,
+// with the rows in global memory (xdrop_dp) it waits for its stores and loads
+// as well. Gapped stage of 139 M residues at 300 / 1,000 / 3,000 query residues:
+// 0.51 -> 0.24, 1.37 -> 0.71, 3.79 -> 2.03 ms.
+constexpr int kDpWindow = 128;
+__device__ __forceinline__ bool xdrop_dp_window(const uint8_t *__restrict__ Q, const uint8_t *__restrict__ S,
+                                                int32_t dir, int32_t M, int32_t N, int32_t gap_open,
+                                                int32_t gap_extend, int32_t xdrop, const int32_t *mat,
+                                                int32_t *best_out, int32_t *a_best, int32_t *b_best,
+                                                int32_t *cells) {
+    const int lane = threadIdx.x & 31;
+    const int32_t goe = gap_open + gap_extend, ge = gap_extend;
+    if (xdrop < goe) xdrop = goe;
+    *best_out = *a_best = *b_best = *cells = 0;
+    if (M <= 0 || N <= 0) return true;
+    int32_t bsize = 1 + min(N, (xdrop - goe) / ge + 1);
+    if (bsize > kDpWindow) return false;
+    int32_t w0 = 0;
+    auto letter = [&](int32_t b) { return b >= 1 && b <= N ? static_cast<int32_t>(S[dir * b]) : 0; };
+    int32_t h[4], e[4], l[4];  // per half: the lane's two columns
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int32_t b = 64 * (j >> 1) + 2 * lane + (j & 1);
+        l[j] = letter(b);
+        h[j] = b >= bsize ? kNeg : b == 0 ? 0 : -goe - (b - 1) * ge;
+        e[j] = b >= bsize ? kNeg : h[j] - goe;
+    }
+    int32_t best = 0, first = 0, ab = 0, bb = 0, n_cells = 0;
+    int32_t rows = 0;  // lane i: the matrix row of row letter (a - 1) rounded down to 32, plus i + 1
+    for (int32_t a = 1; a <= M; ++a) {
+        const int32_t ai = (a - 1) & 31;
+        if (ai == 0) rows = a + lane <= M ? kAlphabet * static_cast<int32_t>(Q[dir * (a + lane)]) : 0;
+        const int32_t *row = mat + __shfl_sync(kFull, rows, ai);
+        n_cells += bsize - first;
+        int32_t carry_p = kNeg, carry_h = kNeg;  // into the second half
+        int32_t lo = INT32_MAX, hi = -1;         // the first and last live column
+        // half s of the row
+        auto half = [&](int s, int32_t &h0, int32_t &h1, int32_t &e0, int32_t &e1, int32_t l0, int32_t l1) {
+            const int32_t b0 = w0 + 64 * s + 2 * lane, b1 = b0 + 1, gb = ge * b0;
+            const bool in0 = b0 < bsize, in1 = b1 < bsize;
+            int32_t hprev = __shfl_up_sync(kFull, h1, 1);
+            if (lane == 0) hprev = carry_h;
+            int32_t d0 = __viaddmax_s32(hprev, row[l0], e0), d1 = __viaddmax_s32(h0, row[l1], e1);
+            if (!in0) d0 = kNeg;
+            if (!in1) d1 = kNeg;
+            // row gap: prefix maximum of D + ge * column over the columns before each
+            const int32_t p0 = d0 + gb, p1 = d1 + gb + ge;
+            int32_t incl = max(p0, p1);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) incl = max(incl, __shfl_up_sync(kFull, incl, o));  // lanes < o get their own
+            int32_t excl = __shfl_up_sync(kFull, incl, 1);
+            if (lane == 0) excl = kNeg;
+            if (s) excl = max(excl, carry_p);
+            const int32_t open = ge - goe - gb;
+            int32_t H0 = __viaddmax_s32(excl, open, d0), H1 = __viaddmax_s32(max(excl, p0), open - ge, d1);
+            if (!in0) H0 = kNeg;
+            if (!in1) H1 = kNeg;
+            const int32_t top = max(H0, H1), cm = __reduce_max_sync(kFull, top);
+            int32_t thr0 = best - xdrop, thr1 = thr0;  // live from there on
+            if (cm > best) {
+                int32_t t = top;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) t = max(t, __shfl_up_sync(kFull, t, o));
+                t = __shfl_up_sync(kFull, t, 1);
+                if (lane > 0) thr0 = max(thr0, t - xdrop);
+                thr1 = max(thr0, H0 - xdrop);
+                const unsigned m0 = __ballot_sync(kFull, H0 == cm), m1 = __ballot_sync(kFull, H1 == cm);
+                const int fl = __ffs(m0 | m1) - 1;
+                ab = a;
+                bb = w0 + 64 * s + 2 * fl + ((m0 >> fl) & 1u ? 0 : 1);
+                best = cm;
+            }
+            const bool alive0 = H0 >= thr0, alive1 = H1 >= thr1;
+            lo = min(lo, __reduce_min_sync(kFull, alive0 ? b0 : alive1 ? b1 : INT32_MAX));
+            hi = max(hi, __reduce_max_sync(kFull, alive1 ? b1 : alive0 ? b0 : -1));
+            // live cells hand on; dead ones keep their E
+            if (s == 0) carry_h = __shfl_sync(kFull, h1, 31);
+            if (alive0) e0 = __viaddmax_s32(H0, -goe, e0 - ge);
+            if (alive1) e1 = __viaddmax_s32(H1, -goe, e1 - ge);
+            h0 = alive0 ? H0 : kNeg;
+            h1 = alive1 ? H1 : kNeg;
+            carry_p = max(carry_p, __shfl_sync(kFull, incl, 31));
+        };
+        half(0, h[0], h[1], e[0], e[1], l[0], l[1]);
+        if (bsize > w0 + 64) half(1, h[2], h[3], e[2], e[3], l[2], l[3]);
+        if (hi < 0) break;
+        first = lo;
+        const int32_t from = hi + 1;  // columns from here on are outside, or the row gap's
+        int32_t n_ext = 0, F = 0;
+        if (from == bsize && bsize <= N) {
+            F = carry_p - goe + ge - ge * bsize;
+            const int32_t room = F - (best - xdrop);
+            if (room >= 0) n_ext = min(N - bsize + 1, ge == 1 ? room + 1 : room / ge + 1);
+        }
+        bsize = from + n_ext;
+        if (bsize <= N) ++bsize;  // the next column, -inf so far
+        // move the window when the band leaves its first half (unless that
+        // gains little) or the window itself
+        const int32_t behind = first - w0, reach = bsize - w0;
+        if (reach > 64 && (behind >= 16 || reach > kDpWindow || (behind >= 4 && reach - behind < 64))) {
+            const int32_t by = min(behind >> 1, 31);
+            w0 += 2 * by;
+            if (bsize - w0 > kDpWindow) return false;
+            const int src = (lane + by) & 31;
+            const bool same = lane + by < 32;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int32_t hl = __shfl_sync(kFull, h[j], src), hh = __shfl_sync(kFull, h[j + 2], src);
+                const int32_t el = __shfl_sync(kFull, e[j], src), eh = __shfl_sync(kFull, e[j + 2], src);
+                h[j] = same ? hl : hh;
+                e[j] = same ? el : eh;
+                h[j + 2] = same ? hh : kNeg;
+                e[j + 2] = same ? eh : kNeg;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) l[j] = letter(w0 + 64 * (j >> 1) + 2 * lane + (j & 1));
+        }
+        if (n_ext > 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int32_t t = w0 + 64 * (j >> 1) + 2 * lane + (j & 1) - from;
+                if (t >= 0 && t < n_ext) {
+                    h[j] = F - t * ge;
+                    e[j] = h[j] - goe;
+                }
+            }
+        }
+    }
+    *cells = n_cells;
+    *best_out = best;
+    *a_best = ab;
+    *b_best = bb;
+    return true;
+}
+
 __device__ __forceinline__ int cmp_start(const DevHsp &a, const DevHsp &b) {
     if (a.q_start != b.q_start) return a.q_start < b.q_start ? -1 : 1;
     if (a.s_start != b.s_start) return a.s_start < b.s_start ? -1 : 1;
@@ -418,8 +568,8 @@ __device__ __forceinline__ unsigned long long work_items(const GappedArgs &a) {
     return n_work;
 }
 
-// The whole gapped stage in one kernel, one warp per work item (single
-// queries, small batches and the allocation-free entry point).
+// The whole gapped stage in one kernel, one warp per work item (the
+// allocation-free entry point).
 __global__ void __launch_bounds__(kGappedWarpsPerBlock * 32)
 gapped_kernel(const GappedArgs a) {
     __shared__ int32_t mat[kAlphabet * kAlphabet];
@@ -576,24 +726,26 @@ gapped_kernel(const GappedArgs a) {
 }
 
 // ------------------------------------------------------------------------
-// The gapped stage in three kernels, for batched passes of many queries:
+// The gapped stage as tasks, two DPs per init hit:
 //
-//   gapped_prep_kernel    one warp per work item: orders its init hits into
-//                         the pass-wide init_sorted array (same slots as the
-//                         scan wrote them) and writes one DP task per init
-//                         hit (its gapped start point);
-//   gapped_dp_kernel      one LANE per X-drop DP (the left and the right one
-//                         of every init hit): each lane runs the sequential
-//                         banded X-drop of the oracle on its own task, rows of
-//                         the warp's 32 tasks in step, its DP row in a
-//                         shared-memory ring of kDpRing columns; a task whose
-//                         band gets wider than the ring is left to the
-//                         finishing kernel;
-//   gapped_finish_kernel  one warp per work item: walks the ordered init
-//                         hits, skips those inside kept HSPs (so the DPs of
-//                         skipped init hits, computed ahead, go unused),
-//                         takes the DP results (running the warp-parallel DP
-//                         for a task the lane kernel left), and publishes.
+//   gapped_prep_kernel     one warp per work item: orders its init hits into
+//                          the pass-wide init_sorted array (same slots as the
+//                          scan wrote them) and writes one DP task per init
+//                          hit (its gapped start point);
+//   gapped_warp_dp_kernel  one warp per X-drop DP; the warp that ends an
+//                          item's last DP finishes it: walks the ordered init
+//                          hits, skips those inside kept HSPs (so the DPs of
+//                          skipped init hits, computed ahead, go unused), and
+//                          publishes.
+//
+// Passes of very many init hits (lane_slots) run their DPs with one LANE each:
+//
+//   gapped_dp_kernel       each lane runs the sequential banded X-drop of the
+//                          oracle on its own task, rows of the warp's 32 tasks
+//                          in step, its DP row in a shared-memory ring of
+//                          kDpRing columns; a task whose band gets wider than
+//                          the ring is left to the finishing kernel;
+//   gapped_finish_kernel   one warp per work item finishes it.
 //
 // Every DP is independent of the others (containment only decides which
 // results are used), so the results are exactly those of gapped_kernel.
@@ -630,13 +782,27 @@ gapped_prep_kernel(const GappedArgs a) {
             d.q_off = 0;
             d.s_off = 0;
             d.valid = init_hit_inside(u, it) ? 1 : 0;
-            d.pad = 0;
+            d.rank = static_cast<int32_t>(k);
+            d.item = t;
+            if (!d.valid) atomicOr(&a.cnt->flags, kFlagBadInitHit);
             if (d.valid) {
                 d.q_off = gapped_start(it.qres, it.sub, u.q_start, u.s_start, u.len, mat);
                 d.s_off = d.q_off + (u.s_start - u.q_start);
             }
             a.dtask[wi.first + k] = d;
+            a.dres[2ull * (wi.first + k)].w = a.dres[2ull * (wi.first + k) + 1].w = -1;  // not run
         }
+        // the item's best init hit among the first ones, the others among the rest
+        unsigned long long fpos = 0, rpos = 0;
+        if (lane == 0) {
+            fpos = atomicAdd(&a.cnt->n_first, 1ull);
+            if (it.n > 1) rpos = atomicAdd(&a.cnt->n_rest, static_cast<unsigned long long>(it.n - 1u));
+            a.dleft[wi.first] = 2u * it.n;
+        }
+        fpos = __shfl_sync(kFull, fpos, 0);
+        rpos = __shfl_sync(kFull, rpos, 0);
+        for (uint32_t k = lane; k < it.n; k += 32)
+            a.dorder[k == 0 ? fpos : a.init_cap - rpos - k] = static_cast<uint32_t>(wi.first + k);
     }
 }
 
@@ -673,6 +839,24 @@ struct DpLane {
     int32_t row, first, bsize, best, ab, bb, cells, thr, rowoff;
 };
 
+// Init-hit slots of the pass (two DPs each): none when the scan overflowed.
+__device__ __forceinline__ unsigned long long dp_slots(const GappedArgs &a) {
+    unsigned long long n = *reinterpret_cast<volatile unsigned long long *>(&a.cnt->init_count);
+    if (n > a.init_cap) n = a.init_cap;
+    return work_items(a) == 0 ? 0ull : n;
+}
+
+// A task record is checked before use (every slot is written by the prep
+// kernel; a stale one from another pass must not send reads astray).
+__device__ __forceinline__ bool dp_task_ok(const GappedArgs &a, const DpTask &k, uint64_t total, const uint8_t **q,
+                                           int32_t *qlen) {
+    if (!k.valid || k.query >= a.n_queries) return false;
+    *q = a.work_query ? a.batch_q[k.query] : a.q;
+    *qlen = a.work_query ? a.batch_qlen[k.query] : a.qlen;
+    return k.s_base <= total && static_cast<uint64_t>(k.slen) <= total - k.s_base && k.q_off >= 0 && k.q_off < *qlen &&
+           k.s_off >= 0 && k.s_off < k.slen && static_cast<uint32_t>(k.slen) + 2u <= a.dp_stride;
+}
+
 __device__ __forceinline__ void dp_lane_start(DpLane &L, unsigned long long t, const GappedArgs &a,
                                               const DpConsts &c, uint32_t *R) {
 #define RS(x) R[((x) & (kDpRing - 1)) * 32]
@@ -680,13 +864,9 @@ __device__ __forceinline__ void dp_lane_start(DpLane &L, unsigned long long t, c
     L.has = false;
     const DpTask k = a.dtask[t >> 1];
     const bool left = (t & 1ull) == 0;
-    const uint8_t *q = a.work_query ? a.batch_q[k.query] : a.q;
-    const int32_t qlen = a.work_query ? a.batch_qlen[k.query] : a.qlen;
-    const uint64_t total = a.off[a.n_subj];
-    // a record is checked before use (every slot is written by the prep
-    // kernel; a stale one from another pass must not send reads astray)
-    if (!k.valid || k.query >= a.n_queries || k.s_base > total || static_cast<uint64_t>(k.slen) > total - k.s_base ||
-        k.q_off < 0 || k.q_off >= qlen || k.s_off < 0 || k.s_off >= k.slen) {
+    const uint8_t *q = nullptr;
+    int32_t qlen = 0;
+    if (!dp_task_ok(a, k, a.off[a.n_subj], &q, &qlen)) {
         if (k.valid) atomicOr(&a.cnt->flags, kFlagBadState);
         a.dres[t] = make_int4(0, 0, 0, 0);
         return;
@@ -820,6 +1000,8 @@ __global__ void __launch_bounds__(kDpWarpsPerBlock * 32)
 gapped_dp_kernel(const GappedArgs a) {
     __shared__ int32_t mat[kAlphabet * kAlphabet];
     extern __shared__ __align__(16) uint32_t dp_smem[];
+    const unsigned long long slots = dp_slots(a), n = 2ull * slots;
+    if (slots < a.lane_slots) return;  // gapped_warp_dp_kernel takes the pass
     load_matrix(mat);
     __syncthreads();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -829,13 +1011,6 @@ gapped_dp_kernel(const GappedArgs a) {
     c.goe = a.gap_open + a.gap_extend;
     c.xdrop = a.xdrop < c.goe ? c.goe : a.xdrop;
     c.bsize0 = 1 + (c.xdrop - c.goe) / c.ge + 1;
-    unsigned long long n_init = 0;
-    {
-        n_init = *reinterpret_cast<volatile unsigned long long *>(&a.cnt->init_count);
-        if (n_init > a.init_cap) n_init = a.init_cap;
-        if (work_items(a) == 0) n_init = 0;
-    }
-    const unsigned long long n = 2ull * n_init;
     unsigned long long next = 0, cur;
     if (lane == 0) next = atomicAdd(&a.cnt->next_dp, 32ull);
     cur = __shfl_sync(kFull, next, 0);
@@ -863,9 +1038,151 @@ gapped_dp_kernel(const GappedArgs a) {
     }
 }
 
+// The left or right DP from a gapped start point by the whole warp: the band
+// in registers, or in the warp's DP rows when it outgrows them (best, row,
+// column, cells).
+__device__ __forceinline__ int4 warp_dp(const GappedArgs &a, const uint8_t *q, int32_t qlen, const uint8_t *s,
+                                        int32_t slen, int32_t q_off, int32_t s_off, bool left, const int32_t *mat,
+                                        int32_t *Hb, int32_t *Eb) {
+    int4 r;
+    const uint8_t *Q = q + q_off + (left ? 1 : 0), *S = s + s_off + (left ? 1 : 0);
+    const int32_t M = left ? q_off + 1 : qlen - q_off - 1, N = left ? s_off + 1 : slen - s_off - 1;
+    if (!xdrop_dp_window(Q, S, left ? -1 : 1, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, &r.x, &r.y, &r.z, &r.w)) {
+        unsigned long long cells = 0;
+        r.x = left ? xdrop_dp<true>(q, s, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, Hb, Eb, &r.y, &r.z, &cells)
+                   : xdrop_dp<false>(Q, S, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, Hb, Eb, &r.y, &r.z, &cells);
+        r.w = static_cast<int32_t>(min(cells, 0x7fffffffull));
+    }
+    return r;
+}
+
+// Walks the item's ordered init hits, skips those inside kept HSPs, takes the
+// DP results -- running the DP of one that the lane kernel left (cells -1) --
+// and publishes.
+__device__ __forceinline__ void finish_item(const GappedArgs &a, const Item &it, DevHsp *saved, int32_t *Hb,
+                                            int32_t *Eb, const int32_t *mat, unsigned long long &cells,
+                                            unsigned long long &n_ext) {
+    const int lane = threadIdx.x & 31;
+    const InitHit *sorted = a.init_sorted + it.wi.first;
+    const DpTask *tasks = a.dtask + it.wi.first;
+    const int4 *res = a.dres + 2ull * it.wi.first;
+    int nsaved = 0;
+    for (uint32_t k = 0; k < it.n; ++k) {
+        const InitHit u = sorted[k];
+        if (!init_hit_inside(u, it)) {
+            if (lane == 0) atomicOr(&a.cnt->flags, kFlagBadInitHit);
+            continue;
+        }
+        if (contained(u, saved, nsaved, lane)) continue;
+        const int32_t q_off = tasks[k].q_off;
+        const int32_t s_off = q_off + (u.s_start - u.q_start);
+        int4 r[2];
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            r[side] = __ldcg(res + 2 * k + side);  // another SM's result: not from L1
+            if (r[side].w < 0) r[side] = warp_dp(a, it.qres, it.qlen, it.sub, it.slen, q_off, s_off, side == 0, mat, Hb, Eb);
+            cells += static_cast<unsigned long long>(r[side].w);
+        }
+        ++n_ext;
+        const int32_t score = r[0].x + r[1].x;
+        if (score >= it.cutoff) {
+            if (lane == 0)
+                saved[nsaved] = make_hsp(it.wi.subject, score, q_off, s_off, r[0].y, r[0].z, r[1].y, r[1].z);
+            ++nsaved;
+        }
+        __syncwarp();
+    }
+    publish(a, it, saved, nsaved, lane);
+}
+
+// Whether the task's init hit lies inside the HSP of its item's best one, as
+// far as that is known by now: the finishing kernel then skips it.
+__device__ __forceinline__ bool inside_first(const GappedArgs &a, unsigned long long slot, const DpTask &k) {
+    if (k.rank == 0) return false;
+    const unsigned long long f = slot - static_cast<unsigned long long>(k.rank);
+    const volatile int32_t *l = reinterpret_cast<const volatile int32_t *>(a.dres + 2 * f), *r = l + 4;
+    if (l[3] < 0 || r[3] < 0) return false;
+    __threadfence();  // the rest of a result is written before its last field
+    const DpTask t = a.dtask[f];
+    if (!t.valid) return false;
+    const InitHit u = a.init_sorted[slot];
+    const DevHsp g = make_hsp(0, l[0] + r[0], t.q_off, t.s_off, l[1], l[2], r[1], r[2]);
+    return g.score >= (a.work_query ? a.batch_cutoff[t.query] : a.cutoff) && u.score <= g.score &&
+           g.q_start <= u.q_start && u.q_start + u.len <= g.q_end && g.s_start <= u.s_start &&
+           u.s_start + u.len <= g.s_end;
+}
+
+// The DP tasks with one warp per DP; the warp that ends an item's last one also
+// finishes the item. The best init hits' tasks come first, so that most of the
+// others that lie inside their HSPs need no DP. (A kernel with a warp per item
+// that runs its DPs one after another, as gapped_kernel does, lasts as long as
+// its longest item: 4,999 query residues against 50,000 subjects of up to 35,000
+// took it 8.4 ms, this form takes 1.05.)
+__global__ void __launch_bounds__(kGappedWarpsPerBlock * 32)
+gapped_warp_dp_kernel(const GappedArgs a) {
+    __shared__ int32_t mat[kAlphabet * kAlphabet];
+    const unsigned long long slots = dp_slots(a);
+    if (slots >= a.lane_slots) return;
+    load_matrix(mat);
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const unsigned long long gwarp = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    int32_t *Hb = a.dp + gwarp * 2ull * a.dp_stride;
+    int32_t *Eb = Hb + a.dp_stride;
+    DevHsp *saved = a.saved + gwarp * a.cap;
+    unsigned long long cells = 0, n_ext = 0;
+    const unsigned long long n_first = slots ? a.cnt->n_first : 0ull, n = slots ? 2ull * (n_first + a.cnt->n_rest) : 0ull;
+    const uint64_t total = a.off[a.n_subj];
+    for (;;) {
+        unsigned long long t = 0;
+        if (lane == 0) t = atomicAdd(&a.cnt->next_dp, 1ull);
+        t = __shfl_sync(kFull, t, 0);
+        if (t >= n) break;
+        const unsigned long long i = t >> 1;
+        const unsigned long long slot = a.dorder[i < n_first ? i : a.init_cap - 1ull - (i - n_first)];
+        if (slot >= a.init_cap) continue;  // cannot happen
+        const DpTask k = a.dtask[slot];
+        const bool left = (t & 1ull) == 0;
+        const uint8_t *q = nullptr;
+        int32_t qlen = 0;
+        if (!dp_task_ok(a, k, total, &q, &qlen)) {
+            if (k.valid && lane == 0) atomicOr(&a.cnt->flags, kFlagBadState);
+            continue;
+        }
+        if (!inside_first(a, slot, k)) {
+            const int4 r = warp_dp(a, q, qlen, a.res + k.s_base, k.slen, k.q_off, k.s_off, left, mat, Hb, Eb);
+            if (lane == 0) {
+                volatile int32_t *o = reinterpret_cast<volatile int32_t *>(a.dres + 2 * slot + (left ? 0 : 1));
+                o[0] = r.x;
+                o[1] = r.y;
+                o[2] = r.z;
+                __threadfence();
+                o[3] = r.w;
+            }
+        }
+        // the item's last DP finishes it
+        unsigned rest = 0;
+        if (lane == 0) {
+            __threadfence();
+            rest = atomicSub(&a.dleft[slot - static_cast<unsigned long long>(k.rank)], 1u);
+            __threadfence();
+        }
+        if (__shfl_sync(kFull, rest, 0) == 1u) {
+            Item it;
+            if (read_item(a, k.item, it, lane)) finish_item(a, it, saved, Hb, Eb, mat, cells, n_ext);
+        }
+        __syncwarp();
+    }
+    if (lane == 0 && n_ext > 0) {
+        atomicAdd(&a.cnt->dp_cells, cells);
+        atomicAdd(&a.cnt->gapped_ext, n_ext);
+    }
+}
+
 __global__ void __launch_bounds__(kGappedWarpsPerBlock * 32)
 gapped_finish_kernel(const GappedArgs a) {
     __shared__ int32_t mat[kAlphabet * kAlphabet];
+    if (dp_slots(a) < a.lane_slots) return;  // gapped_warp_dp_kernel finished the items
     load_matrix(mat);
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -881,44 +1198,7 @@ gapped_finish_kernel(const GappedArgs a) {
         t = __shfl_sync(kFull, t, 0);
         if (t >= n_work) break;
         Item it;
-        if (!read_item(a, t, it, lane)) continue;  // flagged by the prep kernel already
-        const InitHit *sorted = a.init_sorted + it.wi.first;
-        const DpTask *tasks = a.dtask + it.wi.first;
-        const int4 *res = a.dres + 2ull * it.wi.first;
-        int nsaved = 0;
-        for (uint32_t k = 0; k < it.n; ++k) {
-            const InitHit u = sorted[k];
-            if (!init_hit_inside(u, it)) {
-                if (lane == 0) atomicOr(&a.cnt->flags, kFlagBadInitHit);
-                continue;
-            }
-            if (contained(u, saved, nsaved, lane)) continue;
-            const int32_t q_off = tasks[k].q_off;
-            const int32_t s_off = q_off + (u.s_start - u.q_start);
-            const int4 rl = res[2 * k], rr = res[2 * k + 1];
-            int32_t left = rl.x, al = rl.y, bl = rl.z, right = rr.x, ar = rr.y, br = rr.z;
-            if (rl.w < 0) {
-                left = xdrop_dp<true>(it.qres, it.sub, q_off + 1, s_off + 1, a.gap_open, a.gap_extend, a.xdrop, mat, Hb,
-                                      Eb, &al, &bl, &cells);
-            } else {
-                cells += static_cast<unsigned long long>(rl.w);
-            }
-            if (rr.w < 0) {
-                ar = br = 0;
-                right = xdrop_dp<false>(it.qres + q_off, it.sub + s_off, it.qlen - q_off - 1, it.slen - s_off - 1,
-                                        a.gap_open, a.gap_extend, a.xdrop, mat, Hb, Eb, &ar, &br, &cells);
-            } else {
-                cells += static_cast<unsigned long long>(rr.w);
-            }
-            ++n_ext;
-            const int32_t score = left + right;
-            if (score >= it.cutoff) {
-                if (lane == 0) saved[nsaved] = make_hsp(it.wi.subject, score, q_off, s_off, al, bl, ar, br);
-                ++nsaved;
-            }
-            __syncwarp();
-        }
-        publish(a, it, saved, nsaved, lane);
+        if (read_item(a, t, it, lane)) finish_item(a, it, saved, Hb, Eb, mat, cells, n_ext);  // else flagged before
     }
     if (lane == 0) {
         atomicAdd(&a.cnt->dp_cells, cells);
@@ -1024,15 +1304,22 @@ cudaError_t launch_gapped_split(const GappedArgs &a, int n_blocks, int n_sm, cud
     gapped_prep_kernel<<<n_blocks, kGappedWarpsPerBlock * 32, 0, st>>>(a);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    gapped_dp_kernel<<<n_sm * std::max(per_sm_of[dev], 1), kDpWarpsPerBlock * 32, ring_bytes, st>>>(a);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    gapped_finish_kernel<<<n_blocks, kGappedWarpsPerBlock * 32, 0, st>>>(a);
+    if (a.lane_slots != ~0ull) {
+        gapped_dp_kernel<<<n_sm * std::max(per_sm_of[dev], 1), kDpWarpsPerBlock * 32, ring_bytes, st>>>(a);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    gapped_warp_dp_kernel<<<n_blocks, kGappedWarpsPerBlock * 32, 0, st>>>(a);
+    if (a.lane_slots != ~0ull) {
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        gapped_finish_kernel<<<n_blocks, kGappedWarpsPerBlock * 32, 0, st>>>(a);
+    }
     return cudaGetLastError();
 }
 
 cudaError_t gapped_occupancy(int *blocks_per_sm) {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, gapped_kernel,
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, gapped_warp_dp_kernel,
                                                          kGappedWarpsPerBlock * 32, 0);
 }
 
