@@ -153,29 +153,32 @@ extern "C" int blaze_db_info(const blaze_db *db, uint64_t *total, uint32_t *n, u
     return BLAZE_OK;
 }
 
-// A query's word tables on the host: cell_start (kWords + 1 prefix offsets),
-// the packed cells (start << 8 | min(count, 255); 255: look at cell_start),
-// the word-presence bitset and the hit lists (query offsets).
+// Where a query's residues (with 64 zero bytes behind them) and its lookup's
+// tables lie in one device buffer.
 struct QueryTables {
-    std::vector<uint32_t> cs, pack, pres;
-    uint16_t *offs = nullptr;  // malloc'd by build_lookup
-    uint32_t n_off = 0;
-    ~QueryTables() { std::free(offs); }
+    size_t res_bytes, cs, pack, pres, off, bytes;
+    QueryTables(int32_t length, uint32_t n_off) {
+        auto up = [](size_t x) { return (x + 15) & ~size_t{15}; };
+        res_bytes = up(static_cast<size_t>(length) + 64);
+        cs = res_bytes;
+        pack = up(cs + sizeof(uint32_t) * (kWords + 1));
+        pres = up(pack + sizeof(uint32_t) * kWords);
+        off = up(pres + sizeof(uint32_t) * kPresenceWords);
+        bytes = off + sizeof(uint16_t) * std::max<uint32_t>(n_off, 1);
+    }
+    void point(blaze_query &q, unsigned char *p) const {
+        q.d_q = p;
+        q.d_cell_start = reinterpret_cast<uint32_t *>(p + cs);
+        q.d_cell_pack = reinterpret_cast<uint32_t *>(p + pack);
+        q.d_presence = reinterpret_cast<uint32_t *>(p + pres);
+        q.d_cell_off = reinterpret_cast<uint16_t *>(p + off);
+    }
 };
 
-static int query_tables(const uint8_t *query, int32_t length, int32_t word_threshold, QueryTables &t) {
-    t.cs.assign(kWords + 1, 0u);
-    int rc = build_lookup(query, length, word_threshold, t.cs.data(), &t.offs, &t.n_off);
-    if (rc != BLAZE_OK) return rc;
-    t.pack.resize(kWords);
-    t.pres.resize(kPresenceWords);
-    pack_word_cells(t.cs.data(), t.pack.data(), t.pres.data());
-    return BLAZE_OK;
-}
-
-static uint64_t query_upload_bytes(int32_t length, uint32_t n_off) {
-    return static_cast<uint64_t>(length) + sizeof(uint32_t) * (2 * kWords + 1 + kPresenceWords) +
-           sizeof(uint16_t) * n_off;
+// The query's lookup, built on the device from its residues.
+static cudaError_t build_lookup(const blaze_query &q, cudaStream_t st) {
+    return launch_lookup(LookupQuery{q.d_q, q.qlen, q.d_cell_start, q.d_cell_pack, q.d_presence, q.d_cell_off}, nullptr,
+                         1, q.threshold, st);
 }
 
 extern "C" int blaze_query_create(const blaze_db *db, const uint8_t *query, int32_t length,
@@ -185,26 +188,23 @@ extern "C" int blaze_query_create(const blaze_db *db, const uint8_t *query, int3
     if (length > kMaxQueryLength) return BLAZE_ERR_LIMIT;
     if (!valid_residues(query, static_cast<uint64_t>(length))) return BLAZE_ERR_INVALID_ARG;
     BLAZE_CUDA_TRY(cudaSetDevice(db->device));
-    QueryTables t;
-    int rc = query_tables(query, length, word_threshold, t);
-    if (rc != BLAZE_OK) return rc;
+    const uint32_t n_off = lookup_hits(query, length, word_threshold);
+    const QueryTables t(length, n_off);
+    std::vector<uint8_t> res(t.res_bytes, 0);
+    std::memcpy(res.data(), query, length);
     auto *q = new blaze_query();
     q->device = db->device;
     q->qlen = length;
     q->threshold = word_threshold;
-    q->n_off = t.n_off;
-    cudaError_t e = cudaMalloc(&q->d_q, static_cast<size_t>(length) + 64);
-    if (e == cudaSuccess) e = cudaMalloc(&q->d_cell_start, sizeof(uint32_t) * (kWords + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&q->d_cell_off, sizeof(uint16_t) * std::max<uint32_t>(t.n_off, 1));
-    if (e == cudaSuccess) e = cudaMalloc(&q->d_cell_pack, sizeof(uint32_t) * kWords);
-    if (e == cudaSuccess) e = cudaMalloc(&q->d_presence, sizeof(uint32_t) * kPresenceWords);
-    if (e == cudaSuccess) e = cudaMemcpy(q->d_cell_pack, t.pack.data(), sizeof(uint32_t) * kWords, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(q->d_presence, t.pres.data(), sizeof(uint32_t) * kPresenceWords, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(q->d_q, query, length, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(q->d_q + length, 0, 64);
-    if (e == cudaSuccess) e = cudaMemcpy(q->d_cell_start, t.cs.data(), sizeof(uint32_t) * (kWords + 1), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && t.n_off) e = cudaMemcpy(q->d_cell_off, t.offs, sizeof(uint16_t) * t.n_off, cudaMemcpyHostToDevice);
-    q->upload_bytes = query_upload_bytes(length, t.n_off);
+    q->n_off = n_off;
+    q->upload_bytes = t.res_bytes;
+    cudaError_t e = cudaMalloc(&q->d_tables, t.bytes);
+    if (e == cudaSuccess) {
+        t.point(*q, q->d_tables);
+        e = cudaMemcpy(q->d_q, res.data(), t.res_bytes, cudaMemcpyHostToDevice);
+    }
+    if (e == cudaSuccess) e = build_lookup(*q, nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // searches run on streams of their own
     if (e != cudaSuccess) {
         last_cuda_error(e);
         blaze_query_free(q);
@@ -217,11 +217,7 @@ extern "C" int blaze_query_create(const blaze_db *db, const uint8_t *query, int3
 extern "C" int blaze_query_free(blaze_query *q) {
     if (!q) return BLAZE_OK;
     cudaSetDevice(q->device);
-    if (q->d_q) cudaFree(q->d_q);
-    if (q->d_cell_start) cudaFree(q->d_cell_start);
-    if (q->d_cell_pack) cudaFree(q->d_cell_pack);
-    if (q->d_presence) cudaFree(q->d_presence);
-    if (q->d_cell_off) cudaFree(q->d_cell_off);
+    if (q->d_tables) cudaFree(q->d_tables);
     delete q;
     return BLAZE_OK;
 }
@@ -289,11 +285,7 @@ extern "C" int blaze_search_free(blaze_search *s) {
     s->seg_idx.release();
     s->sel_q.release();
     s->seg_keys.release();
-    s->qt_res.release();
-    s->qt_cs.release();
-    s->qt_pack.release();
-    s->qt_pres.release();
-    s->qt_off.release();
+    s->qt.release();
     if (s->h_stage) cudaFreeHost(s->h_stage);
     s->tb_items.release();
     s->tb_out.release();
@@ -1052,10 +1044,10 @@ extern "C" int blaze_search_init_hits(blaze_search *s, blaze_init_hit *out, uint
     return k == n_init ? BLAZE_OK : BLAZE_ERR_INTERNAL;
 } BLAZE_ABI_CATCH
 
-// One call with host buffers: the query's tables go into buffers the search
-// context keeps (grown on demand), copied from pinned staging on the
-// search's stream ahead of the kernels -- no allocation and no device-wide
-// synchronisation per query once warm.
+// One call with host buffers: the query's residues go through pinned staging
+// into a buffer the search context keeps (grown on demand), and its lookup is
+// built there on the search's stream ahead of the kernels -- no allocation and
+// no device-wide synchronisation per query once warm.
 extern "C" int blaze_prelim_search(blaze_search *s, const uint8_t *query, int32_t length,
                                    const blaze_params *p, blaze_hsp *out, uint64_t capacity,
                                    uint64_t *n_hsps) try {
@@ -1065,43 +1057,20 @@ extern "C" int blaze_prelim_search(blaze_search *s, const uint8_t *query, int32_
     int rc = check_params(p);
     if (rc != BLAZE_OK) return rc;
     BLAZE_CUDA_TRY(cudaSetDevice(s->db->device));
-    QueryTables t;
-    if ((rc = query_tables(query, length, p->word_threshold, t)) != BLAZE_OK) return rc;
-    // pinned staging: residues (+ 64 zero bytes), cell_start, packed cells, presence, hit lists
-    const size_t b_q = (static_cast<size_t>(length) + 64 + 15) & ~size_t{15};
-    const size_t b_cs = sizeof(uint32_t) * (kWords + 1), b_pack = sizeof(uint32_t) * kWords;
-    const size_t b_pres = sizeof(uint32_t) * kPresenceWords, b_off = sizeof(uint16_t) * t.n_off;
-    const size_t o_cs = b_q, o_pack = (o_cs + b_cs + 15) & ~size_t{15}, o_pres = o_pack + b_pack,
-                 o_off = (o_pres + b_pres + 15) & ~size_t{15};
-    if ((rc = ensure_pinned(s->h_stage, s->h_stage_n, o_off + b_off)) != BLAZE_OK) return rc;
-    unsigned char *h = s->h_stage;
-    std::memcpy(h, query, length);
-    std::memset(h + length, 0, b_q - static_cast<size_t>(length));
-    std::memcpy(h + o_cs, t.cs.data(), b_cs);
-    std::memcpy(h + o_pack, t.pack.data(), b_pack);
-    std::memcpy(h + o_pres, t.pres.data(), b_pres);
-    if (b_off) std::memcpy(h + o_off, t.offs, b_off);
-    if ((rc = s->qt_res.ensure(b_q)) != BLAZE_OK) return rc;
-    if ((rc = s->qt_cs.ensure(kWords + 1)) != BLAZE_OK) return rc;
-    if ((rc = s->qt_pack.ensure(kWords)) != BLAZE_OK) return rc;
-    if ((rc = s->qt_pres.ensure(kPresenceWords)) != BLAZE_OK) return rc;
-    if ((rc = s->qt_off.ensure(std::max<uint32_t>(t.n_off, 1))) != BLAZE_OK) return rc;
-    BLAZE_CUDA_TRY(cudaMemcpyAsync(s->qt_res.p, h, b_q, cudaMemcpyHostToDevice, s->stream));
-    BLAZE_CUDA_TRY(cudaMemcpyAsync(s->qt_cs.p, h + o_cs, b_cs, cudaMemcpyHostToDevice, s->stream));
-    BLAZE_CUDA_TRY(cudaMemcpyAsync(s->qt_pack.p, h + o_pack, b_pack, cudaMemcpyHostToDevice, s->stream));
-    BLAZE_CUDA_TRY(cudaMemcpyAsync(s->qt_pres.p, h + o_pres, b_pres, cudaMemcpyHostToDevice, s->stream));
-    if (b_off) BLAZE_CUDA_TRY(cudaMemcpyAsync(s->qt_off.p, h + o_off, b_off, cudaMemcpyHostToDevice, s->stream));
-    blaze_query q;  // views of the search's buffers; not freed
+    blaze_query q;  // a view of the search's buffer; not freed
     q.device = s->db->device;
     q.qlen = length;
     q.threshold = p->word_threshold;
-    q.n_off = t.n_off;
-    q.upload_bytes = query_upload_bytes(length, t.n_off);
-    q.d_q = s->qt_res.p;
-    q.d_cell_start = s->qt_cs.p;
-    q.d_cell_pack = s->qt_pack.p;
-    q.d_presence = s->qt_pres.p;
-    q.d_cell_off = s->qt_off.p;
+    q.n_off = lookup_hits(query, length, p->word_threshold);
+    const QueryTables t(length, q.n_off);
+    q.upload_bytes = t.res_bytes;
+    if ((rc = ensure_pinned(s->h_stage, s->h_stage_n, t.res_bytes)) != BLAZE_OK) return rc;
+    std::memcpy(s->h_stage, query, length);
+    std::memset(s->h_stage + length, 0, t.res_bytes - static_cast<size_t>(length));
+    if ((rc = s->qt.ensure(t.bytes)) != BLAZE_OK) return rc;
+    t.point(q, s->qt.p);
+    BLAZE_CUDA_TRY(cudaMemcpyAsync(q.d_q, s->h_stage, t.res_bytes, cudaMemcpyHostToDevice, s->stream));
+    BLAZE_CUDA_TRY(build_lookup(q, s->stream));
     RunSpec r;
     r.q = &q;
     r.p = p;

@@ -1,6 +1,6 @@
-// batch.cu -- query batches of the batched form: every query's word tables
-// built on the host and uploaded into one set of device arrays (refilled in
-// place by the serving loop).
+// batch.cu -- query batches of the batched form: every query's residues and
+// word tables in one set of device arrays (refilled in place by the serving
+// loop).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -19,10 +19,10 @@ static int check_batch_input(const uint8_t *residues, const uint64_t *offsets, u
     return BLAZE_OK;
 }
 
-// Builds the word tables of every query on the host and uploads them into
-// the batch's device buffers, growing those only when they are too small
-// (so that a refilled batch allocates nothing once it has seen its largest
-// load). Copies go on `stream` (0: synchronous).
+// Uploads every query's residues and builds their lookups on the device, in
+// the batch's buffers, growing those only when they are too small (so that a
+// refilled batch allocates nothing once it has seen its largest load). The work
+// goes on `stream` (null: the default one) and is done on return.
 static int batch_fill(blaze_batch *b, const uint8_t *residues, const uint64_t *offsets, uint32_t n_queries,
                       int32_t word_threshold, cudaStream_t stream) {
     b->n = n_queries;
@@ -32,10 +32,7 @@ static int batch_fill(blaze_batch *b, const uint8_t *residues, const uint64_t *o
     b->off_off.clear();
     b->n_off.clear();
     std::vector<uint8_t> res;
-    std::vector<uint32_t> cs_all(static_cast<size_t>(n_queries) * (kWords + 1));
-    std::vector<uint32_t> pack_all(static_cast<size_t>(n_queries) * kWords);
-    std::vector<uint32_t> pres_all(static_cast<size_t>(n_queries) * kPresenceWords, 0u);
-    std::vector<uint16_t> offs_all;
+    uint64_t n_offs = 0;
     for (uint32_t i = 0; i < n_queries; ++i) {
         const int32_t len = static_cast<int32_t>(offsets[i + 1] - offsets[i]);
         const uint8_t *q = residues + offsets[i];
@@ -43,51 +40,44 @@ static int batch_fill(blaze_batch *b, const uint8_t *residues, const uint64_t *o
         b->res_off.push_back(res.size());
         res.insert(res.end(), q, q + len);
         res.resize((res.size() + 63) & ~static_cast<size_t>(63), 0);  // 64-byte separation
-        uint32_t *cs = cs_all.data() + static_cast<size_t>(i) * (kWords + 1);
-        uint16_t *offs = nullptr;
-        uint32_t n_off = 0;
-        int rc = build_lookup(q, len, word_threshold, cs, &offs, &n_off);
-        if (rc != BLAZE_OK) return rc;
-        b->off_off.push_back(offs_all.size());
-        b->n_off.push_back(n_off);
-        offs_all.insert(offs_all.end(), offs, offs + n_off);
-        std::free(offs);
-        pack_word_cells(cs, pack_all.data() + static_cast<size_t>(i) * kWords,
-                        pres_all.data() + static_cast<size_t>(i) * kPresenceWords);
+        b->off_off.push_back(n_offs);
+        b->n_off.push_back(lookup_hits(q, len, word_threshold));
+        n_offs += b->n_off.back();
     }
     res.resize(res.size() + 64, 0);
-    if (offs_all.empty()) offs_all.push_back(0);
     // a refill grows by half again so that slowly rising loads settle
     const size_t slack = stream ? 2 : 1;
     auto grow = [&](auto &buf, size_t want) {
         return want <= buf.n ? BLAZE_OK : buf.ensure(want + (slack - 1) * want / 2);
     };
     int rc = grow(b->res, res.size());
-    if (rc == BLAZE_OK) rc = grow(b->cell_start, cs_all.size());
-    if (rc == BLAZE_OK) rc = grow(b->cell_pack, pack_all.size());
-    if (rc == BLAZE_OK) rc = grow(b->presence, pres_all.size());
-    if (rc == BLAZE_OK) rc = grow(b->cell_off, offs_all.size());
+    if (rc == BLAZE_OK) rc = grow(b->cell_start, static_cast<size_t>(n_queries) * (kWords + 1));
+    if (rc == BLAZE_OK) rc = grow(b->cell_pack, static_cast<size_t>(n_queries) * kWords);
+    if (rc == BLAZE_OK) rc = grow(b->presence, static_cast<size_t>(n_queries) * kPresenceWords);
+    if (rc == BLAZE_OK) rc = grow(b->cell_off, std::max<uint64_t>(n_offs, 1));
+    if (rc == BLAZE_OK) rc = grow(b->lookups, n_queries);
     if (rc != BLAZE_OK) return rc;
     b->d_res = b->res.p;
     b->d_cell_start = b->cell_start.p;
     b->d_cell_pack = b->cell_pack.p;
     b->d_presence = b->presence.p;
     b->d_cell_off = b->cell_off.p;
-    auto put = [&](void *dst, const void *src, size_t bytes) {
-        return stream ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream)
-                      : cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
-    };
-    cudaError_t e = put(b->d_res, res.data(), res.size());
-    if (e == cudaSuccess) e = put(b->d_cell_start, cs_all.data(), sizeof(uint32_t) * cs_all.size());
-    if (e == cudaSuccess) e = put(b->d_cell_pack, pack_all.data(), sizeof(uint32_t) * pack_all.size());
-    if (e == cudaSuccess) e = put(b->d_presence, pres_all.data(), sizeof(uint32_t) * pres_all.size());
-    if (e == cudaSuccess) e = put(b->d_cell_off, offs_all.data(), sizeof(uint16_t) * offs_all.size());
-    // the host arrays die with this frame: the copies must have read them
-    if (e == cudaSuccess && stream) e = cudaStreamSynchronize(stream);
-    b->upload_bytes = res.size() + sizeof(uint32_t) * (cs_all.size() + pack_all.size() + pres_all.size()) +
-                      sizeof(uint16_t) * offs_all.size();
+    std::vector<LookupQuery> lookups(n_queries);
+    for (uint32_t i = 0; i < n_queries; ++i)
+        lookups[i] = LookupQuery{b->d_res + b->res_off[i], b->qlen[i],
+                                 b->d_cell_start + static_cast<size_t>(i) * (kWords + 1),
+                                 b->d_cell_pack + static_cast<size_t>(i) * kWords,
+                                 b->d_presence + static_cast<size_t>(i) * kPresenceWords, b->d_cell_off + b->off_off[i]};
+    cudaError_t e = cudaMemcpyAsync(b->d_res, res.data(), res.size(), cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(b->lookups.p, lookups.data(), sizeof(LookupQuery) * n_queries, cudaMemcpyHostToDevice,
+                            stream);
+    if (e == cudaSuccess) e = launch_lookup(LookupQuery{}, b->lookups.p, n_queries, word_threshold, stream);
+    // the host arrays die with this frame, and searches run on other streams
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    b->upload_bytes = res.size() + sizeof(LookupQuery) * n_queries;
     b->device_bytes = b->res.n + sizeof(uint32_t) * (b->cell_start.n + b->cell_pack.n + b->presence.n) +
-                      sizeof(uint16_t) * b->cell_off.n;
+                      sizeof(uint16_t) * b->cell_off.n + sizeof(LookupQuery) * b->lookups.n;
     if (e != cudaSuccess) {
         last_cuda_error(e);
         return e == cudaErrorMemoryAllocation ? BLAZE_ERR_OUT_OF_MEMORY : BLAZE_ERR_CUDA;
@@ -134,6 +124,7 @@ extern "C" int blaze_batch_free(blaze_batch *b) {
     b->cell_pack.release();
     b->presence.release();
     b->cell_off.release();
+    b->lookups.release();
     delete b;
     return BLAZE_OK;
 }

@@ -136,6 +136,17 @@ struct BatchQuery {
     uint32_t index;  // position of the query in its batch
 };
 
+// A query's word lookup on the device: where its residues are and its tables
+// go (cell_start: kWords + 1 prefix offsets; cell_pack: start << 8 | min(count,
+// 255), 255 sends the kernel to cell_start; presence: kPresenceWords; cell_off:
+// lookup_hits query offsets).
+struct LookupQuery {
+    const uint8_t *q;
+    int32_t qlen;
+    uint32_t *cell_start, *cell_pack, *presence;
+    uint16_t *cell_off;
+};
+
 struct ScanArgs {
     const uint8_t *res;        // residues, length-sorted subjects
     const uint64_t *off;       // n_subj + 1 offsets
@@ -283,15 +294,14 @@ cudaError_t gapped_occupancy(int *blocks_per_sm);
 // kernel fills n_sm SMs. Results equal launch_gapped's.
 cudaError_t launch_gapped_split(const GappedArgs &a, int n_blocks, int n_sm, cudaStream_t st);
 
+// The lookups of n queries: `many` (a device array), or `one` when it is null.
+cudaError_t launch_lookup(const LookupQuery &one, const LookupQuery *many, uint32_t n, int32_t threshold,
+                          cudaStream_t st);
+
 // Host helpers (host.cpp).
 extern const int32_t kBlosum62[kAlphabet][kAlphabet];
-// Word lookup of a query: cell_start[kWords + 1], offsets ascending per cell.
-int build_lookup(const uint8_t *query, int32_t qlen, int32_t threshold,
-                 uint32_t *cell_start, uint16_t **offsets, uint32_t *n_offsets);
-// The scan kernel's per-word tables from cell_start: packed cells
-// (start << 8 | min(count, 255); 255 sends the kernel to cell_start) and the
-// word-presence bitset (kPresenceWords words, overwritten).
-void pack_word_cells(const uint32_t *cell_start, uint32_t *pack, uint32_t *presence);
+// Entries of a query's hit lists (its word lookup's size), without building it.
+uint32_t lookup_hits(const uint8_t *query, int32_t qlen, int32_t threshold);
 int default_params(int32_t qlen, uint64_t db_len, uint32_t db_n, double evalue,
                    blaze_params *out);
 

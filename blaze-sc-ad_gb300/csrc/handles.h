@@ -45,6 +45,7 @@ struct blaze_query {
     int32_t qlen = 0;
     int32_t threshold = 0;
     uint64_t upload_bytes = 0;  // host->device bytes of the tables
+    unsigned char *d_tables = nullptr;  // one allocation (null: another object's): QueryTables
     uint8_t *d_q = nullptr;
     uint32_t *d_cell_start = nullptr;
     uint32_t *d_cell_pack = nullptr;
@@ -121,10 +122,8 @@ struct blaze_search {
     GroupDesc *h_groups = nullptr;  // pinned
     size_t h_groups_n = 0;
     // query tables of the one-call entry point, reused across calls
-    DevBuf<uint8_t> qt_res;
-    DevBuf<uint32_t> qt_cs, qt_pack, qt_pres;
-    DevBuf<uint16_t> qt_off;
-    unsigned char *h_stage = nullptr;  // pinned staging of those tables
+    DevBuf<unsigned char> qt;
+    unsigned char *h_stage = nullptr;  // pinned staging of its residues
     size_t h_stage_n = 0;
     std::vector<blaze_batch_hsp> batch_results;
     // traceback stage
@@ -150,6 +149,7 @@ struct blaze_batch {
     DevBuf<uint8_t> res;
     DevBuf<uint32_t> cell_start, cell_pack, presence;
     DevBuf<uint16_t> cell_off;
+    DevBuf<LookupQuery> lookups;
     uint8_t *d_res = nullptr;
     uint32_t *d_cell_start = nullptr, *d_cell_pack = nullptr, *d_presence = nullptr;
     uint16_t *d_cell_off = nullptr;

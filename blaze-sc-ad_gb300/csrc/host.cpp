@@ -18,98 +18,45 @@ const int32_t kBlosum62[kAlphabet][kAlphabet] = {
 
 namespace {
 
-// Neighbourhood of every three-letter word for one threshold, in CSR form:
-// words v with score(w, v) >= threshold, plus w itself
-// (BLAZE_ncbi/prelim_stage.cpp:135-155 enumerates the same set; :378-383
-// keeps the exact word). Computed once per threshold and cached.
-struct Neighbourhood {
-    std::vector<uint32_t> start;  // kWords + 1
-    std::vector<uint16_t> words;  // word index < 21952 fits 16 bits
-};
-
+// Size of every three-letter word's neighbourhood for one threshold: the words
+// v with score(w, v) >= threshold, and w itself (BLAZE_ncbi/
+// prelim_stage.cpp:135-155 enumerates the same set; :378-383 keeps the exact
+// word). Computed once per threshold and cached.
 std::mutex g_nb_mutex;
-std::map<int32_t, Neighbourhood *> g_nb_cache;
+std::map<int32_t, std::vector<uint16_t>> g_nb_cache;
 
-const Neighbourhood *neighbourhood(int32_t threshold) {
+const std::vector<uint16_t> &neighbourhood_sizes(int32_t threshold) {
     std::lock_guard<std::mutex> lock(g_nb_mutex);
     auto it = g_nb_cache.find(threshold);
     if (it != g_nb_cache.end()) return it->second;
-    auto *nb = new Neighbourhood();
-    nb->start.resize(kWords + 1);
+    std::vector<uint16_t> size(kWords);
     int32_t row_max[kAlphabet];
     for (int a = 0; a < kAlphabet; ++a)
         row_max[a] = *std::max_element(kBlosum62[a], kBlosum62[a] + kAlphabet);
     for (int w = 0; w < kWords; ++w) {
-        nb->start[w] = static_cast<uint32_t>(nb->words.size());
         const int x = w / 784, y = (w / 28) % 28, z = w % 28;
-        bool self_added = false;
+        uint32_t n = kBlosum62[x][x] + kBlosum62[y][y] + kBlosum62[z][z] < threshold ? 1 : 0;
         for (int a = 0; a < kAlphabet; ++a) {
             const int32_t s0 = kBlosum62[x][a];
             if (s0 + row_max[y] + row_max[z] < threshold) continue;
             for (int b = 0; b < kAlphabet; ++b) {
                 const int32_t s1 = s0 + kBlosum62[y][b];
                 if (s1 + row_max[z] < threshold) continue;
-                for (int c = 0; c < kAlphabet; ++c) {
-                    if (s1 + kBlosum62[z][c] >= threshold) {
-                        const int v = a * 784 + b * 28 + c;
-                        nb->words.push_back(static_cast<uint16_t>(v));
-                        if (v == w) self_added = true;
-                    }
-                }
+                for (int c = 0; c < kAlphabet; ++c) n += s1 + kBlosum62[z][c] >= threshold ? 1u : 0u;
             }
         }
-        if (!self_added) {
-            // keep cells sorted by word index: insert w at its place
-            auto first = nb->words.begin() + nb->start[w];
-            nb->words.insert(std::upper_bound(first, nb->words.end(), static_cast<uint16_t>(w)),
-                             static_cast<uint16_t>(w));
-        }
+        size[w] = static_cast<uint16_t>(n);  // at most 21,952
     }
-    nb->start[kWords] = static_cast<uint32_t>(nb->words.size());
-    g_nb_cache[threshold] = nb;
-    return nb;
+    return g_nb_cache.emplace(threshold, std::move(size)).first->second;
 }
 
 }  // namespace
 
-int build_lookup(const uint8_t *query, int32_t qlen, int32_t threshold, uint32_t *cell_start,
-                 uint16_t **offsets, uint32_t *n_offsets) {
-    const Neighbourhood *nb = neighbourhood(threshold);
-    const int32_t nwords = qlen >= kWordSize ? qlen - kWordSize + 1 : 0;
-    std::vector<uint32_t> count(kWords + 1, 0);
-    std::vector<int32_t> word_of(static_cast<size_t>(std::max(nwords, 1)));
-    for (int32_t i = 0; i < nwords; ++i) {
-        const int w = query[i] * 784 + query[i + 1] * 28 + query[i + 2];
-        word_of[i] = w;
-        for (uint32_t k = nb->start[w]; k < nb->start[w + 1]; ++k) count[nb->words[k]]++;
-    }
-    uint32_t acc = 0;
-    for (int v = 0; v < kWords; ++v) {
-        cell_start[v] = acc;
-        acc += count[v];
-    }
-    cell_start[kWords] = acc;
-    *n_offsets = acc;
-    auto *out = static_cast<uint16_t *>(std::malloc(sizeof(uint16_t) * std::max<uint32_t>(acc, 1)));
-    if (!out) return BLAZE_ERR_OUT_OF_MEMORY;
-    std::vector<uint32_t> cursor(cell_start, cell_start + kWords);
-    // query offsets are visited in increasing order, so every cell ends up sorted
-    for (int32_t i = 0; i < nwords; ++i) {
-        const int w = word_of[i];
-        for (uint32_t k = nb->start[w]; k < nb->start[w + 1]; ++k)
-            out[cursor[nb->words[k]]++] = static_cast<uint16_t>(i);
-    }
-    *offsets = out;
-    return BLAZE_OK;
-}
-
-void pack_word_cells(const uint32_t *cell_start, uint32_t *pack, uint32_t *presence) {
-    std::memset(presence, 0, sizeof(uint32_t) * kPresenceWords);
-    for (int w = 0; w < kWords; ++w) {
-        const uint32_t cnt = cell_start[w + 1] - cell_start[w];
-        pack[w] = (cell_start[w] << 8) | std::min<uint32_t>(cnt, 255u);
-        if (cnt) presence[w >> 5] |= 1u << (w & 31);
-    }
+uint32_t lookup_hits(const uint8_t *query, int32_t qlen, int32_t threshold) {
+    const std::vector<uint16_t> &size = neighbourhood_sizes(threshold);
+    uint32_t n = 0;
+    for (int32_t i = 0; i + kWordSize <= qlen; ++i) n += size[query[i] * 784 + query[i + 1] * 28 + query[i + 2]];
+    return n;
 }
 
 // Karlin-Altschul constants of BLOSUM62 (published NCBI table values).
