@@ -67,39 +67,43 @@ lookup_count_kernel(const LookupQuery one, const LookupQuery *many, int32_t thre
 }
 
 // One block per query: starts, packed cells (start << 8 | min(count, 255)) and
-// the presence bitset from the counts.
+// the presence bitset from the counts. A warp takes 22 rows of 32 consecutive
+// words, so every access is coalesced and a row's presence is a ballot (a run
+// of words per thread instead took 38 us for one query).
 __global__ void __launch_bounds__(1024) lookup_tables_kernel(const LookupQuery one, const LookupQuery *many) {
-    __shared__ uint16_t count[kWords];  // at most 32,000 offsets
+    constexpr uint32_t kRows = (kPresenceWords + 31) / 32;
+    static_assert(kRows * 1024 >= kWords);
     __shared__ uint32_t warp_sum[32];
     const LookupQuery lq = many ? many[blockIdx.x] : one;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    for (uint32_t w = tid; w < kWords; w += 1024u) count[w] = static_cast<uint16_t>(lq.cell_start[w]);
-    __syncthreads();
-    constexpr uint32_t kEach = (kWords + 1023) / 1024;
-    const uint32_t w0 = min(tid * kEach, static_cast<uint32_t>(kWords)), w1 = min(w0 + kEach, static_cast<uint32_t>(kWords));
-    uint32_t sum = 0;
-    for (uint32_t w = w0; w < w1; ++w) sum += count[w];
-    uint32_t incl = sum;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t w0 = warp * kRows * 32u + lane;
+    uint32_t n[kRows], sum = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= static_cast<uint32_t>(o)) incl += x;
+    for (uint32_t k = 0; k < kRows; ++k) {
+        n[k] = w0 + k * 32u < kWords ? lq.cell_start[w0 + k * 32u] : 0u;
+        sum += n[k];
     }
-    if (lane == 31u) warp_sum[warp] = incl;
-    __syncthreads();
-    uint32_t start = incl - sum;
-    for (uint32_t i = 0; i < warp; ++i) start += warp_sum[i];
-    for (uint32_t w = w0; w < w1; ++w) {
-        const uint32_t n = count[w];
-        lq.cell_start[w] = start;
-        lq.cell_pack[w] = (start << 8) | min(n, 255u);
-        start += n;
-    }
-    if (tid == 1023u) lq.cell_start[kWords] = start;
-    for (uint32_t p = tid; p < kPresenceWords; p += 1024u) {
-        uint32_t bits = 0;
-        for (uint32_t k = 0; k < 32u && p * 32u + k < kWords; ++k) bits |= (count[p * 32u + k] ? 1u : 0u) << k;
-        lq.presence[p] = bits;
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0u) warp_sum[warp] = sum;
+    __syncthreads();  // also: every count is read before a start replaces it
+    uint32_t start = __reduce_add_sync(0xffffffffu, lane < warp ? warp_sum[lane] : 0u);
+    if (warp == 31u && lane == 0u) lq.cell_start[kWords] = start + sum;
+#pragma unroll
+    for (uint32_t k = 0; k < kRows; ++k) {
+        uint32_t incl = n[k];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= static_cast<uint32_t>(o)) incl += x;
+        }
+        const uint32_t w = w0 + k * 32u, at = start + incl - n[k];
+        const uint32_t bits = __ballot_sync(0xffffffffu, n[k] != 0u);
+        if (w < kWords) {
+            lq.cell_start[w] = at;
+            lq.cell_pack[w] = (at << 8) | min(n[k], 255u);
+        }
+        if (lane == 0u && w / 32u < kPresenceWords) lq.presence[w / 32u] = bits;
+        start += __shfl_sync(0xffffffffu, incl, 31);
     }
 }
 
