@@ -129,8 +129,21 @@ int db_make_groups(blaze_db *db) {
         b.push_back(lo);
         hi = lo;
     }
+    // A subject alone in its group is cut in pieces of a warp's share of the
+    // residues (with what precedes it in its first 16 bytes), other groups are
+    // one piece. (4,000 residues against 500 subjects: 0.21 ms with pieces of
+    // 128, 0.35 of 512, 0.52 of 2,240.)
+    const uint64_t piece = std::min<uint64_t>(std::max<uint64_t>(db->total / (152 * 32), kPieceLeast), kPieceMost);
+    std::vector<uint32_t> pieces(1, 0u);
+    for (size_t g = 0; g + 1 < b.size(); ++g) {
+        const uint64_t len = b[g] - b[g + 1] == 1 ? off[b[g]] - off[b[g + 1]] : 0;
+        pieces.push_back(pieces.back() + std::max<uint32_t>(1u, static_cast<uint32_t>((len + 15 + piece - 1) / piece)));
+    }
+    db->n_pieces = pieces.back();
     BLAZE_CUDA_TRY(cudaMalloc(&db->d_groups, sizeof(uint32_t) * b.size()));
     BLAZE_CUDA_TRY(cudaMemcpy(db->d_groups, b.data(), sizeof(uint32_t) * b.size(), cudaMemcpyHostToDevice));
+    BLAZE_CUDA_TRY(cudaMalloc(&db->d_pieces, sizeof(uint32_t) * pieces.size()));
+    BLAZE_CUDA_TRY(cudaMemcpy(db->d_pieces, pieces.data(), sizeof(uint32_t) * pieces.size(), cudaMemcpyHostToDevice));
     return BLAZE_OK;
 }
 
@@ -141,6 +154,7 @@ extern "C" int blaze_db_free(blaze_db *db) {
     if (db->d_off) cudaFree(db->d_off);
     if (db->d_oid) cudaFree(db->d_oid);
     if (db->d_groups) cudaFree(db->d_groups);
+    if (db->d_pieces) cudaFree(db->d_pieces);
     delete db;
     return BLAZE_OK;
 }
@@ -264,6 +278,7 @@ extern "C" int blaze_search_free(blaze_search *s) {
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
     s->scratch.release();
     s->init_out.release();
+    s->band_state.release();
     s->gapped_ws.release();
     s->work.release();
     s->saved.release();
@@ -372,6 +387,8 @@ static cudaError_t enqueue_pass(blaze_search *s, const PassLaunch &pl, unsigned 
         e = cudaMemsetAsync(s->cursors.p, 0, sizeof(unsigned long long) * pl.n_cursors, s->stream);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(s->ev[1], s->stream, event_flags);
     for (const ScanLaunch &l : pl.scans) {
+        if (e == cudaSuccess && l.sa.pieces)
+            e = cudaMemsetAsync(s->band_state.p, 0, sizeof(BandState) * l.sa.n_groups, s->stream);
         if (e != cudaSuccess) break;
         e = l.queue ? launch_scan_batch(l.sa, l.word_table, l.blocks, l.warps_per_block, l.smem_bytes, s->stream)
                        : launch_scan(l.sa, l.word_table, l.blocks, l.warps_per_block, l.smem_bytes, s->stream);
@@ -458,6 +475,8 @@ struct ScanPlan {
     int blocks = 0;
     uint32_t first = 0, n = 1;
     bool queue = false;  // the batched kernel over the plan's queries; else one query's launch
+    bool bands = false;  // one query's launch in bands
+    uint32_t extra_bands = 0;
 };
 
 // One pass of both stages; fills s->h_cnt.
@@ -479,8 +498,11 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
     const uint32_t nq = batched ? r.b->n : 1u;
     // the gapped stage's arrays, per init-hit slot: ordered init hit, DP task,
     // two DP results, DP order, DPs left
-    const size_t slot_bytes = sizeof(InitHit) + sizeof(DpTask) + 2 * sizeof(int4) + 2 * sizeof(uint32_t);
+    constexpr size_t slot_bytes = sizeof(InitHit) + sizeof(DpTask) + 2 * sizeof(int4) + 2 * sizeof(uint32_t);
     if ((rc = s->gapped_ws.ensure(s->init_cap * slot_bytes)) != BLAZE_OK) return rc;
+    const size_t n_groups = db->h_groups.size() - 1;
+    for (const ScanPlan &plan : plans)
+        if (plan.bands && (rc = s->band_state.ensure(n_groups)) != BLAZE_OK) return rc;
     if ((rc = s->groups.ensure(s->out_cap)) != BLAZE_OK) return rc;  // a published list holds >= 1 HSP
     if ((rc = s->qkept.ensure(nq)) != BLAZE_OK) return rc;
     if (batched && (rc = s->work_query.ensure(work_cap)) != BLAZE_OK) return rc;
@@ -505,7 +527,19 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
         sa.res = db->d_res;
         sa.off = db->d_off;
         sa.groups = db->d_groups;
-        sa.n_groups = static_cast<uint32_t>(db->h_groups.size()) - 1;
+        sa.n_groups = static_cast<uint32_t>(n_groups);
+        sa.n_items = sa.n_groups;
+        if (plan.bands) {
+            sa.pieces = db->d_pieces;
+            sa.extra_bands = plan.extra_bands;
+            sa.n_items = db->n_pieces + sa.n_groups * plan.extra_bands;
+            sa.band_state = s->band_state.p;
+            // a hit takes two records at most; the gapped stage's arrays lie idle
+            // meanwhile
+            static_assert(slot_bytes >= 2 * sizeof(InitHit));
+            sa.fragments = reinterpret_cast<InitHit *>(s->gapped_ws.p);
+            sa.fragment_cap = std::min<unsigned long long>(2 * s->init_cap, UINT32_MAX - 1);
+        }
         sa.window = p->window;
         sa.xdrop = p->ungapped_xdrop;
         sa.diag_entries = lay.diag_entries;
@@ -650,11 +684,12 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     // layout of one single-query scan launch
     const uint32_t stage_bytes = std::max(s->stage_bytes, db->group_bytes);
     constexpr size_t kSmemMost = 227 * 1024 - 64;  // the opt-in limit less static shared memory
-    auto layout_for = [&](int32_t qlen, uint32_t n_hits, int warps) {
-        ScanLayout l = scan_layout(qlen, p0->window, n_hits, stage_bytes, kSmemBudget, warps);
+    auto layout_for = [&](int32_t qlen, uint32_t n_hits, int warps, uint32_t band_entries = 0) {
+        ScanLayout l = scan_layout(qlen, p0->window, n_hits, stage_bytes, kSmemBudget, warps, band_entries);
         // next to the longest tables only smaller groups are staged
         if (l.smem_bytes > kSmemMost)
-            l = scan_layout(qlen, p0->window, n_hits, std::max(s->stage_bytes, 576u) - 576u, kSmemBudget, warps);
+            l = scan_layout(qlen, p0->window, n_hits, std::max(s->stage_bytes, 576u) - 576u, kSmemBudget, warps,
+                            band_entries);
         return l;
     };
     // layout of one batched scan launch over queries of up to `longest`
@@ -680,9 +715,20 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
                          [&](uint32_t a, uint32_t b) { return r.b->qlen[a] < r.b->qlen[b]; });
     auto qlen_at = [&](uint32_t k) { return batched ? r.b->qlen[order[k]] : r.q->qlen; };
     std::vector<ScanPlan> plans;
-    auto query_layout = [&](uint32_t k) {
-        return layout_for(qlen_at(k), batched ? r.b->n_off[order[k]] : r.q->n_off, warp_cap);
+    auto query_layout = [&](uint32_t k, uint32_t band_entries = 0) {
+        return layout_for(qlen_at(k), batched ? r.b->n_off[order[k]] : r.q->n_off, warp_cap, band_entries);
     };
+    // One query's launch runs in bands of diagonals
+    // - where a subject is longer than a warp's share of the residues, so that
+    //   the launch would end in a wait for it: such subjects are cut in pieces.
+    //   300 and 4,999 residues against 17.5 M with subjects of up to 35,000:
+    //   0.81 -> 0.29 and 10.46 -> 2.83 ms; but 103 against 140 M, longest 5,000
+    //   (a share is 28,700), 0.62 -> 0.70;
+    // - for the longest queries, with a table of one band's diagonals: tables of
+    //   a whole query would leave few warps an SM. 8,000 / 12,345 / 30,000
+    //   residues against 140 M: 42.0 -> 37.5, 172 -> 62 and 1,520 -> 230 ms; at
+    //   5,000 (14 warps without) 19.9 -> 24.0, since every band looks up its
+    //   words again. Such queries of a batch have launches of their own too.
     // A batch runs as one launch whose blocks go from query to query where a
     // query's own pass would end in a wait for its longest subjects, that is
     // where one of them is more than a warp's share of the residues: 16 queries
@@ -691,19 +737,36 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     // is the faster (256 queries against 35 M residues 117.2 ms and 120.1).
     const uint64_t share = db->total / (static_cast<uint64_t>(s->n_sm) * kScanMaxWarpsPerBlock);
     const bool per_query = batched && (s->batch_launch == 2 || (s->batch_launch == 0 && (nq == 1 || db->max_len < share)));
+    const bool has_pieces = db->n_pieces + 1 > db->h_groups.size();
+    auto narrow_layout = [&](uint32_t k) { return query_layout(k, scan_band_entries(qlen_at(k))); };
+    auto is_narrow = [&](uint32_t k) {  // (a group's bands have to be staged as one)
+        return qlen_at(k) > kBandQuery && p0->window <= kTab16Window && db->n > 0 &&
+               narrow_layout(k).stage_bytes >= db->group_bytes;
+    };
     r.border = order;
     for (uint32_t i = 0; i < nq;) {
         uint32_t j = i + 1;
         ScanPlan pl;
         pl.lay = query_layout(i);
-        pl.queue = batched && !per_query;
+        const bool narrow = is_narrow(i);
+        pl.queue = batched && !per_query && (!narrow || s->batch_launch == 1);
+        const bool banded = narrow || (has_pieces && db->max_len > share && p0->window <= kTab16Window);
         if (pl.queue) {
             const bool smem = pl.lay.query_smem_bytes != 0, table = pl.lay.word_table;
             for (; j < nq; ++j) {
                 const ScanLayout l = query_layout(j);
-                if ((l.query_smem_bytes != 0) != smem || l.word_table != table) break;
+                if ((l.query_smem_bytes != 0) != smem || l.word_table != table || is_narrow(j) != narrow) break;
             }
             pl.lay = batch_layout_for(qlen_at(j - 1), table);
+        } else if (banded) {
+            if (narrow) {
+                pl.lay = narrow_layout(i);
+                // a group's diagonals: its positions, the windows between its
+                // subjects and the query
+                const uint32_t reach = static_cast<uint32_t>(qlen_at(i) + p0->window * static_cast<int32_t>(kGroupMaxSubjects));
+                pl.extra_bands = (reach + pl.lay.diag_entries - 1) / pl.lay.diag_entries;
+            }
+            pl.bands = true;
         }
         pl.first = i;
         pl.n = j - i;
@@ -713,8 +776,8 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
             BLAZE_CUDA_TRY(scan_batch_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.word_table, pl.lay.warps_per_block,
                                                 pl.lay.smem_bytes, &per_sm));
         } else {
-            BLAZE_CUDA_TRY(scan_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.word_table, pl.lay.warps_per_block,
-                                          pl.lay.smem_bytes, &per_sm));
+            BLAZE_CUDA_TRY(scan_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.word_table, pl.bands,
+                                          pl.lay.warps_per_block, pl.lay.smem_bytes, &per_sm));
         }
         if (per_sm < 1) return BLAZE_ERR_LIMIT;
         pl.blocks = s->n_sm * per_sm;

@@ -37,11 +37,23 @@ constexpr size_t kScanMatBytes = kAlphabet * kAlphabet * 4;           // matrix,
 constexpr size_t kScanPresenceBytes = (kPresenceWords * 4 + 15) & ~15; // 2752
 constexpr size_t kScanWordTabBytes = ((kWords + 1) * 2 + 15) & ~15;    // 43,920
 constexpr uint32_t kScanWordTabHits = 65535;  // hit-list entries a 16-bit word table can number
-constexpr int32_t kQuerySmemMax = 8192;      // queries up to this length live in shared memory,
+constexpr int32_t kQuerySmemMax = 11776;      // queries up to this length live in shared memory,
+constexpr int32_t kBandQuerySmemMax = 14336;  // in bands this one,
 constexpr int32_t kTab16Window = 256;        // for windows up to this one: 16-bit diagonal tables
+// Diagonals of a band where its table holds no more, by the width of its
+// entries: 12,345 residues against 140 M with 16-bit tables of 2,240 / 3,360 /
+// 4,480 / 6,720 entries 70.5 / 62.2 / 64.8 / 78.4 ms, 16,000 with 32-bit ones
+// 120 / 130 / 147 / 173
+constexpr uint32_t kBandEntries16 = 3360, kBandEntries32 = 2240;
+static_assert(kBandEntries32 >= kGroupMaxBytes && kBandEntries16 >= kGroupMaxBytes, "a group is one piece");
+constexpr uint32_t kPieceLeast = 128, kPieceMost = kGroupMaxBytes;  // residues of a long subject's piece
+constexpr int32_t kBandQuery = 7000;         // longer queries take such tables
 constexpr uint32_t kScanStageBytes = 1024;   // subjects up to this length are staged
 
-inline bool scan_query_in_smem(int32_t qlen, int32_t window) { return qlen <= kQuerySmemMax && window <= kTab16Window; }
+inline bool scan_query_in_smem(int32_t qlen, int32_t window, bool bands = false) {
+    return qlen <= (bands ? kBandQuerySmemMax : kQuerySmemMax) && window <= kTab16Window;
+}
+inline uint32_t scan_band_entries(int32_t qlen) { return qlen <= kBandQuerySmemMax ? kBandEntries16 : kBandEntries32; }
 inline uint32_t scan_diag_entries(int32_t qlen, int32_t window) {  // >= qlen + window
     return static_cast<uint32_t>(qlen + window + 3) & ~3u;
 }
@@ -84,6 +96,13 @@ struct DevHsp {
     int32_t score, q_start, q_end, s_start, s_end, q_gs, s_gs;
 };
 
+// The bands of one group of a scan launch: its fragments of init hits (index + 1
+// of the last one's record, 0: none) and the bands that are done. Zeroed before
+// the launch.
+struct BandState {
+    unsigned int head, done;
+};
+
 // Device counters of one run; zeroed before every run.
 struct DevCounters {
     unsigned long long init_count;   // init hits published
@@ -101,6 +120,7 @@ struct DevCounters {
     unsigned long long group_count;  // subject HSP lists published (GroupDesc records)
     unsigned long long next_prep;    // gapped prep-kernel work cursor
     unsigned long long next_dp;      // DP task cursor
+    unsigned long long fragments;    // records taken in ScanArgs::fragments
     unsigned long long n_first, n_rest;  // DP tasks: items' best init hits, the others
 };
 
@@ -152,6 +172,15 @@ struct ScanArgs {
     const uint64_t *off;       // n_subj + 1 offsets
     const uint32_t *groups;    // n_groups + 1 subject indices, descending: group g is [groups[g+1], groups[g])
     uint32_t n_groups;
+    // a single-query launch in bands (null: without): prefix sums over the groups
+    // of their pieces; the bands of a group beyond one per piece; per group
+    // state; fragments of init hits
+    const uint32_t *pieces;
+    uint32_t extra_bands;
+    uint32_t n_items;          // groups, or bands
+    BandState *band_state;
+    InitHit *fragments;
+    unsigned long long fragment_cap;
     const uint8_t *q;          // query residues
     int32_t qlen;
     const uint32_t *cell_start;  // kWords + 1
@@ -159,7 +188,7 @@ struct ScanArgs {
     const uint32_t *presence;    // kPresenceWords: bit w set when word w has hits
     const uint16_t *cell_off;    // query offsets per cell, ascending
     int32_t window, xdrop, cutoff;
-    uint32_t diag_entries;       // >= qlen + window
+    uint32_t diag_entries;       // >= qlen + window, or the diagonals of a band
     uint32_t diag_magic;         // floor(2^32 / diag_entries) + 1
     uint32_t diag_bytes, stage_bytes, query_smem_bytes, warp_smem_bytes;
     uint32_t smem_bytes;         // batched launches: dynamic shared memory of a block
@@ -274,10 +303,11 @@ struct TracebackArgs {
 };
 
 // Launchers (scan.cu, kernels.cu, traceback.cu).
-ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t n_hits, uint32_t stage_bytes, size_t smem_budget, int max_warps);
+ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t n_hits, uint32_t stage_bytes, size_t smem_budget,
+                       int max_warps, uint32_t band_entries = 0);
 cudaError_t launch_scan(const ScanArgs &a, bool word_table, int n_blocks, int warps_per_block, size_t smem,
                         cudaStream_t st);
-cudaError_t scan_occupancy(bool query_in_smem, bool word_table, int warps_per_block, size_t smem, int *blocks_per_sm);
+cudaError_t scan_occupancy(bool query_in_smem, bool word_table, bool bands, int warps_per_block, size_t smem, int *blocks_per_sm);
 int scan_max_warps_by_registers(bool query_in_smem);
 cudaError_t launch_gapped(const GappedArgs &a, int n_blocks, cudaStream_t st,
                           int warps_per_block = kGappedWarpsPerBlock);

@@ -33,6 +33,8 @@ struct blaze_db {
     // the word finder's groups, from the longest subjects down (ScanArgs::groups)
     std::vector<uint32_t> h_groups;
     uint32_t *d_groups = nullptr;
+    uint32_t *d_pieces = nullptr;  // prefix sums of the groups' pieces (ScanArgs::pieces)
+    uint32_t n_pieces = 0;
     uint32_t group_bytes = 0;      // the most that the blocks of a group of several subjects take
 };
 
@@ -82,6 +84,7 @@ struct blaze_search {
     uint32_t scratch_cap = kInitialScratchCap;
     unsigned long long init_cap = 0, out_cap = 0;
     DevBuf<InitHit> scratch, init_out;
+    DevBuf<BandState> band_state;
     DevBuf<WorkItem> work;
     DevBuf<DevHsp> saved, out;
     DevBuf<int32_t> dp;

@@ -70,7 +70,6 @@ __device__ __forceinline__ void sts64(uint32_t off, uint2 v) { reinterpret_cast<
 constexpr int kKeyBits = 14;
 constexpr int32_t kKeyMask = (1 << kKeyBits) - 1;
 constexpr int32_t kKeyedLength = 11900;  // of a walk: 11 x its length times 2^14 stays below 2^31
-static_assert(kQuerySmemMax <= kKeyedLength, "walks on keys");
 __device__ __forceinline__ int32_t key_of(uint32_t qa, uint32_t sb) {
     return reinterpret_cast<const int32_t *>(smem + kMatOff)[qa * kAlphabet + sb];
 }
@@ -329,9 +328,20 @@ struct Ctx {
     uint32_t seed_span;  // distances from the word size on that trigger an extension
 };
 
+// The diagonals of a group that a warp takes: those with v - q + (query length)
+// in [first, end). A group is cut into bands where its warp would be the last
+// one running, or where a table of the query's whole length plus the window
+// would leave few warps on an SM. State is kept per diagonal, so bands are
+// independent; a word's hits in a band are one run of its ascending hit list.
+struct Band {
+    int32_t first, end;
+    bool all;  // the only band
+};
+
 constexpr int32_t kPackSpan = 1 << 17;
+static_assert(kQuerySmemMax <= kKeyedLength, "walks on keys");
 static_assert(kGroupMaxBytes + (kGroupMaxSubjects + 2) * kTab16Window <= Tab<true>::kMost, "16-bit entries");
-static_assert(kQuerySmemMax + kChunk + kTab16Window <= Tab<true>::kMost, "16-bit entries");
+static_assert(kBandQuerySmemMax + kChunk + kTab16Window <= Tab<true>::kMost, "16-bit entries");
 
 // A hit in 32 bits: v (17 bits from vb on) and q (at most 32,000).
 __device__ __forceinline__ uint32_t pack_hit(const Finder &f, int32_t v, int32_t q) {
@@ -459,7 +469,7 @@ __device__ __forceinline__ bool queues_full(const Finder &f) {
 // a seed, so the loop ends. Seeds of all the group's subjects share a flush: a
 // walk takes as many warp instructions a step whether one lane or 32 take it,
 // so what an extension costs falls with the seeds it shares its flush with.
-template <bool QS, bool WT, bool ST>
+template <bool QS, bool WT, bool BANDS, bool ST>
 __device__ __forceinline__ void flush(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, WT> &q,
                                       const Span<ST> &span, bool empty) {
     const uint32_t lane = threadIdx.x & 31;
@@ -487,7 +497,7 @@ __device__ __forceinline__ void flush(Finder &f, const ScanArgs &a, const Ctx &c
                 const int32_t to_v = c.window * static_cast<int32_t>(subj) + sub.first;  // from the subject's offsets
                 const int32_t so = hv - to_v, left = so - static_cast<int32_t>(sd.y) + kWordSize;
                 int32_t rext, slast;
-                h.score = QS || sub.len <= kKeyedLength
+                h.score = (QS && !BANDS) || min(c.qlen, sub.len) <= kKeyedLength
                               ? extend_two_hit_keyed(q, sub, left, so, hq, c.xdrop, &h.q_start, &h.s_start, &h.len,
                                                      &rext, &slast)
                               : extend_two_hit(q, sub, left, so, hq, c.xdrop, &h.q_start, &h.s_start, &h.len, &rext,
@@ -577,6 +587,37 @@ __device__ __forceinline__ uint32_t warp_prefix(uint32_t x) {
     return x;
 }
 
+// The parts of the cells at v0 .. v0 + 3 (from cs on, cnt offsets each) on the
+// band's diagonals: offsets q with v + qlen - q in [band.first, band.end). The
+// eight lower bounds are searched in step, so that their loads overlap.
+__device__ __forceinline__ void clip_cells(const Ctx &c, const Band &band, int32_t v0, uint32_t *cs, uint32_t *cnt) {
+    const int32_t from = v0 + c.qlen - band.end + 1, to = v0 + c.qlen - band.first + 1;  // q in [from + j, to + j)
+    const bool clip = from + 3 > 0 || to < c.qlen;
+    const uint32_t most = max(max(cnt[0], cnt[1]), max(cnt[2], cnt[3]));
+    const uint32_t all = __reduce_max_sync(kFull, clip ? most : 0u);
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        lo[j] = 0u;
+        hi[j] = clip ? 0u : cnt[j];
+    }
+    for (uint32_t step = all ? 0x80000000u >> __clz(static_cast<int>(all)) : 0u; step != 0u; step >>= 1) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint16_t *off = c.cell_off + cs[j];
+            if (lo[j] + step <= cnt[j] && static_cast<int32_t>(__ldg(off + (lo[j] + step - 1u))) < from + j) lo[j] += step;
+            if (hi[j] + step <= cnt[j] && static_cast<int32_t>(__ldg(off + (hi[j] + step - 1u))) < to + j) hi[j] += step;
+        }
+    }
+    if (all) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            cs[j] += lo[j];
+            cnt[j] = hi[j] - lo[j];
+        }
+    }
+}
+
 // Word scan of a group: chunks of 128 positions, four consecutive positions
 // per lane. One warp prefix sum per chunk numbers the chunk's hits in (subject
 // offset, query offset) order and the words that have any; each such word
@@ -585,20 +626,25 @@ __device__ __forceinline__ uint32_t warp_prefix(uint32_t x) {
 // its word by a population count. A chunk's last hits, too few for a batch,
 // wait in front of the next chunk's, so batches are full (at 300 query
 // residues a chunk brings 79 hits).
-template <bool QS, bool WT, bool ST>
+template <bool QS, bool WT, bool BANDS, bool ST>
 __device__ __forceinline__ void scan_span(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, WT> &q,
-                                          const Span<ST> &span, bool long_one) {
+                                          const Span<ST> &span, bool long_one, const Band &band) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t list = f.w + kListAt;
     const int32_t end = static_cast<int32_t>(__shfl_sync(kFull, f.end, f.ns - 1u));
-    const int32_t xend = end - (kWordSize - 1);  // words start below it
+    int32_t xend = end - (kWordSize - 1);        // words start below it
     uint32_t before = 0;                         // subjects that begin before the chunk
     uint32_t left = 0;   // hits waiting from the chunks before, fewer than a batch
     uint32_t left_m = 0; // which of them start a word
     uint32_t left_w = 0; // words begun before the chunk whose hits are waiting
     // four positions of a lane lie in one subject's block
     int32_t cb = static_cast<int32_t>(__shfl_sync(kFull, f.first, 0));
-    if (f.ns > 1) cb &= ~15;
+    if (f.ns > 1) {
+        cb &= ~15;
+    } else if (BANDS && !band.all) {  // the positions that have a hit on the band's diagonals
+        cb += max(0, band.first - c.qlen - cb) & ~(kChunk - 1);
+        xend = min(xend, band.end - 1);
+    }
     for (; cb < xend; cb += kChunk) {
         if (long_one && needs_rebase<QS>(f, c, end, cb)) rebase<QS>(f, a, c, cb);
         // the queues are emptied at the group's end and before a rebase
@@ -630,6 +676,10 @@ __device__ __forceinline__ void scan_span(Finder &f, const ScanArgs &a, const Ct
                 cnt[j] = pk & 0xffu;
                 if (cnt[j] == 0xffu) cnt[j] = __ldg(c.cell_start + w + 1) - cs[j];
             }
+        }
+        if (BANDS && !band.all) clip_cells(c, band, v0, cs, cnt);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
             has[j] = min(cnt[j], 1u);
             sum += cnt[j] * 256u + has[j];  // 24 bits: 128 words of at most 32,000 hits
         }
@@ -670,7 +720,7 @@ __device__ __forceinline__ void scan_span(Finder &f, const ScanArgs &a, const Ct
                 m = begins_from(k0);
             }
             const bool done = empty && k0 >= total;
-            if (queues_full(f) || done) flush(f, a, c, q, span, done);
+            if (queues_full(f) || done) flush<QS, WT, BANDS>(f, a, c, q, span, done);
             if (done || !batch) break;
         } while (true);
         // the hits left wait: their words move to the front of the list, counted from k0
@@ -824,48 +874,138 @@ __device__ __forceinline__ void clear_table(Finder &f, const Ctx &c) {
     __syncwarp();
 }
 
-// The fetched subjects for the query of `c`: finds their init hits and
-// publishes each subject's. False when a staging copy never landed.
-template <bool QS, bool WT>
-__device__ __forceinline__ bool process_group(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, WT> &q,
-                                              const Group &g, uint32_t query_index) {
+// Publishes the init hits in this warp's scratch, each subject's as one block.
+__device__ __forceinline__ void publish_group(const Finder &f, const ScanArgs &a, uint32_t lo, uint32_t query_index) {
     const uint32_t lane = threadIdx.x & 31;
+    __syncwarp();  // the records in scratch were written by several lanes
+    for (uint32_t i = 0; i < f.ns; ++i) {
+        const int32_t x0 = static_cast<int32_t>(__shfl_sync(kFull, f.first, i));
+        const int32_t x1 = static_cast<int32_t>(__shfl_sync(kFull, f.end, i));
+        uint32_t n = 0;
+        for (uint32_t i0 = 0; i0 < f.n_init; i0 += 32) {
+            const int32_t t = i0 + lane < f.n_init ? scratch_of(a)[i0 + lane].s_trig : -1;
+            n += __popc(__ballot_sync(kFull, t >= x0 && t < x1));
+        }
+        if (n) publish_subject(f, a, lo + i, x0, x1, n, query_index);
+    }
+}
+
+// More init hits than the warp's scratch holds: the run is repeated with more.
+__device__ __forceinline__ void scratch_overflow(const ScanArgs &a, uint32_t n) {
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&a.cnt->overflow_subjects, 1u);
+        atomicMax(&a.cnt->max_init_needed, n);
+    }
+}
+
+// A band of group `g` is done: leaves its init hits (positions in the group,
+// which every band counts alike) as a fragment -- a record with the next
+// fragment and the number of hits, and the hits -- in the group's list. True
+// for the group's last band to finish, whose warp then has all of the group's
+// hits in its scratch.
+__device__ __forceinline__ bool merge_bands(Finder &f, const ScanArgs &a, uint32_t g, uint32_t n_bands) {
+    const uint32_t lane = threadIdx.x & 31;
+    BandState *st = a.band_state + g;
+    if (f.n_init > a.scratch_cap) {
+        scratch_overflow(a, f.n_init);
+    } else if (f.n_init > 0) {
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(&a.cnt->fragments, static_cast<unsigned long long>(f.n_init + 1u));
+        at = __shfl_sync(kFull, at, 0);
+        if (at + f.n_init + 1u <= a.fragment_cap) {
+            __syncwarp();
+            for (uint32_t i = lane; i < f.n_init; i += 32) a.fragments[at + 1u + i] = scratch_of(a)[i];
+            __syncwarp();
+            if (lane == 0) {
+                InitHit head{};
+                head.len = static_cast<int32_t>(f.n_init);
+                head.q_start = static_cast<int32_t>(atomicExch(&st->head, static_cast<unsigned int>(at + 1u)));
+                a.fragments[at] = head;
+            }
+        } else if (lane == 0) {
+            atomicOr(&a.cnt->flags, kFlagInitArrayFull);
+            atomicAdd(&a.cnt->init_count, static_cast<unsigned long long>(f.n_init));
+        }
+    }
+    uint32_t done = 0;
+    __syncwarp();
+    if (lane == 0) {
+        __threadfence();  // the fragment before the count
+        done = atomicAdd(&st->done, 1u) + 1u;
+        __threadfence();
+    }
+    done = __shfl_sync(kFull, done, 0);
+    if (done != n_bands) return false;
+    uint32_t n = 0;
+    const InitHit *frag = a.fragments;
+    for (uint32_t next = __ldcg(&st->head); next != 0u;) {
+        const uint32_t at = next - 1u, m = static_cast<uint32_t>(__ldcg(&frag[at].len));
+        for (uint32_t i = lane; i < m && n + i < a.scratch_cap; i += 32) {
+            const int32_t *w = reinterpret_cast<const int32_t *>(frag + at + 1u + i);
+            scratch_of(a)[n + i] = InitHit{__ldcg(w), __ldcg(w + 1), __ldcg(w + 2), __ldcg(w + 3), __ldcg(w + 4), __ldcg(w + 5)};
+        }
+        n += m;
+        next = static_cast<uint32_t>(__ldcg(&frag[at].q_start));
+    }
+    f.n_init = n;
+    return true;
+}
+
+// A launch's item t: its group, which of the group's bands, and of how many.
+// Without bands an item is a group. With them group g's items begin at
+// pieces[g] + g x extra_bands: one per piece of its residues (ScanArgs::pieces)
+// and the extra ones.
+struct Item {
+    uint32_t group, band, n_bands;
+};
+template <bool BANDS>
+__device__ __forceinline__ Item item_at(const ScanArgs &a, uint32_t t) {
+    if (!BANDS) return Item{t, 0u, 1u};
+    uint32_t lo = 0, hi = a.n_groups;  // the last group that begins at or before t is in [lo, hi)
+    while (hi - lo > 1u) {
+        // the lanes try 32 groups spread over [lo, hi), the first of them lo
+        const uint32_t step = (hi - lo + 31u) / 32u, g = lo + step * (threadIdx.x & 31u);
+        const bool begun = g < hi && a.pieces[g] + g * a.extra_bands <= t;
+        const uint32_t k = __popc(__ballot_sync(kFull, begun)) - 1u;
+        hi = min(hi, lo + step * (k + 1u));
+        lo += step * k;
+    }
+    return Item{lo, t - (a.pieces[lo] + lo * a.extra_bands), a.pieces[lo + 1u] - a.pieces[lo] + a.extra_bands};
+}
+
+// The fetched subjects for the query of `c`: finds the item's init hits and
+// publishes each subject's. False when a staging copy never landed.
+template <bool QS, bool WT, bool BANDS>
+__device__ __forceinline__ bool process_group(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, WT> &q,
+                                              const Group &g, uint32_t query_index, const Item &it) {
     f.n_init = 0;
     f.vb = 0;
     // the values the group's hits take, with the distance to the next group's
     const uint32_t extent = __shfl_sync(kFull, f.end, f.ns - 1u) + static_cast<uint32_t>(c.window) * f.ns;
     if (f.base + extent > Tab<QS>::kMost) clear_table<QS>(f, c);
     const bool long_one = QS ? f.base + extent > Tab<QS>::kMost : extent > kPackSpan - kChunk;
+    Band b{0, INT32_MAX, !BANDS || it.n_bands == 1u};
+    if (!b.all) {  // equal bands over the diagonals, [0, extent + qlen)
+        const unsigned long long span = static_cast<unsigned long long>(extent) + static_cast<uint32_t>(c.qlen);
+        b.first = static_cast<int32_t>(span * it.band / it.n_bands);
+        b.end = static_cast<int32_t>(span * (it.band + 1u) / it.n_bands);
+    }
     if (g.staged) {
         if (!stage_wait(f, a)) return false;
         Span<true> span;
         span.off = f.w + kDiagAt + c.diag_bytes;
         span.ptr = nullptr;
         clear_margins(f, span.off);
-        scan_span(f, a, c, q, span, long_one);
+        scan_span<QS, WT, BANDS>(f, a, c, q, span, long_one, b);
     } else {  // one subject
         Span<false> span;
         span.off = 0;
         span.ptr = a.res + g.o0;
-        scan_span(f, a, c, q, span, long_one);
+        scan_span<QS, WT, BANDS>(f, a, c, q, span, long_one, b);
     }
-    if (f.n_init > a.scratch_cap) {
-        if (lane == 0) {
-            atomicAdd(&a.cnt->overflow_subjects, 1u);
-            atomicMax(&a.cnt->max_init_needed, f.n_init);
-        }
-    } else if (f.n_init > 0) {
-        __syncwarp();  // the records in scratch were written by several lanes
-        for (uint32_t i = 0; i < f.ns; ++i) {
-            const int32_t x0 = static_cast<int32_t>(__shfl_sync(kFull, f.first, i));
-            const int32_t x1 = static_cast<int32_t>(__shfl_sync(kFull, f.end, i));
-            uint32_t n = 0;
-            for (uint32_t i0 = 0; i0 < f.n_init; i0 += 32) {
-                const int32_t t = i0 + lane < f.n_init ? scratch_of(a)[i0 + lane].s_trig : -1;
-                n += __popc(__ballot_sync(kFull, t >= x0 && t < x1));
-            }
-            if (n) publish_subject(f, a, g.lo + i, x0, x1, n, query_index);
-        }
+    if (b.all || merge_bands(f, a, it.group, it.n_bands)) {
+        if (f.n_init > a.scratch_cap) scratch_overflow(a, f.n_init);
+        else if (f.n_init > 0) publish_group(f, a, g.lo, query_index);
     }
     f.base += extent;
     if (f.hits >> 26) add_counts(f, a);
@@ -907,7 +1047,7 @@ __device__ __forceinline__ void load_query_tables(const uint32_t *cell_start, co
 // One query against the whole database: the query's word table (or its
 // word-presence bitset) and the query itself when short enough live in shared
 // memory; warps pull groups, longest subjects first.
-template <bool QS, bool WT>
+template <bool QS, bool WT, bool BANDS>
 __global__ void __launch_bounds__(kScanMaxWarpsPerBlock * 32, 1)
 scan_kernel(const ScanArgs a) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -929,10 +1069,12 @@ scan_kernel(const ScanArgs a) {
     // blocks; its copy runs while the block fills its tables
     unsigned long long t = static_cast<unsigned long long>(warp) * gridDim.x + blockIdx.x;
     Group g{};
+    Item it{};
     uint32_t hi = 0;
-    if (t < a.n_groups) {
-        hi = a.groups[t];
-        g = fetch_group(f, a, c, a.groups[t + 1], hi, true);
+    if (t < a.n_items) {
+        it = item_at<BANDS>(a, static_cast<uint32_t>(t));
+        hi = a.groups[it.group];
+        g = fetch_group(f, a, c, a.groups[it.group + 1], hi, true);
     }
     clear_table<QS>(f, c);
     load_matrix();
@@ -941,15 +1083,16 @@ scan_kernel(const ScanArgs a) {
     Query<QS, WT> q;
     q.ptr = a.q;
     q.len = a.qlen;
-    while (t < a.n_groups) {
-        if (!process_group(f, a, c, q, g, a.query_index)) return;
+    while (t < a.n_items) {
+        if (!process_group<QS, WT, BANDS>(f, a, c, q, g, a.query_index, it)) return;
         uint32_t lo = g.lo + f.ns;
         if (lo == hi) {
             if (lane == 0) t = atomicAdd(a.cursor, 1ull) + static_cast<unsigned long long>(gridDim.x) * (blockDim.x >> 5);
             t = __shfl_sync(kFull, t, 0);
-            if (t >= a.n_groups) break;
-            lo = a.groups[t + 1];
-            hi = a.groups[t];
+            if (t >= a.n_items) break;
+            it = item_at<BANDS>(a, static_cast<uint32_t>(t));
+            lo = a.groups[it.group + 1];
+            hi = a.groups[it.group];
         }
         g = fetch_group(f, a, c, lo, hi, true);
     }
@@ -1036,7 +1179,8 @@ scan_batch_kernel(const ScanArgs a) {
                 }
                 // after a copy that never landed: read this and every later
                 // subject from global memory (the host reports the run as failed)
-                while (!process_group(f, a, c, q, fetch_group(f, a, c, lo, hi, staging), bq.index)) staging = false;
+                while (!process_group<QS, WT, false>(f, a, c, q, fetch_group(f, a, c, lo, hi, staging), bq.index, Item{}))
+                    staging = false;
                 lo += f.ns;
             }
             __syncwarp();
@@ -1049,13 +1193,15 @@ scan_batch_kernel(const ScanArgs a) {
 
 }  // namespace
 
-ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t n_hits, uint32_t stage_bytes, size_t smem_budget, int max_warps) {
+ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t n_hits, uint32_t stage_bytes, size_t smem_budget,
+                       int max_warps, uint32_t band_entries) {
     ScanLayout l{};
-    l.diag_entries = scan_diag_entries(qlen, window);
+    const bool smem = scan_query_in_smem(qlen, window, band_entries != 0);
+    l.diag_entries = band_entries ? band_entries : scan_diag_entries(qlen, window);
     l.diag_magic = static_cast<uint32_t>((1ull << 32) / l.diag_entries + 1);
-    l.diag_bytes = scan_diag_bytes(qlen, window);
+    l.diag_bytes = (l.diag_entries * (smem ? 2u : 4u) + 15u) & ~15u;
     l.stage_bytes = stage_bytes;
-    l.query_smem_bytes = scan_query_in_smem(qlen, window) ? (static_cast<uint32_t>(qlen) + 15u) & ~15u : 0u;
+    l.query_smem_bytes = smem ? (static_cast<uint32_t>(qlen) + 15u) & ~15u : 0u;
     l.warp_smem_bytes = scan_warp_bytes(l.diag_bytes, stage_bytes);
     auto fit = [&](size_t tab) {
         const size_t fixed = kScanMatBytes + tab + l.query_smem_bytes;
@@ -1105,13 +1251,17 @@ static cudaError_t allow_full_smem(const void *kernel) {
     return e;
 }
 
-static void (*single_kernel(bool query_in_smem, bool word_table))(ScanArgs) {
-    return !query_in_smem ? scan_kernel<false, false> : word_table ? scan_kernel<true, true> : scan_kernel<true, false>;
+static void (*single_kernel(bool query_in_smem, bool word_table, bool bands))(ScanArgs) {
+    if (bands)
+        return !query_in_smem ? scan_kernel<false, false, true>
+                              : word_table ? scan_kernel<true, true, true> : scan_kernel<true, false, true>;
+    return !query_in_smem ? scan_kernel<false, false, false>
+                          : word_table ? scan_kernel<true, true, false> : scan_kernel<true, false, false>;
 }
 
 cudaError_t launch_scan(const ScanArgs &a, bool word_table, int n_blocks, int warps_per_block, size_t smem_bytes,
                         cudaStream_t st) {
-    auto kernel = single_kernel(a.query_smem_bytes != 0, word_table);
+    auto kernel = single_kernel(a.query_smem_bytes != 0, word_table, a.pieces != nullptr);
     cudaError_t e = allow_full_smem(reinterpret_cast<const void *>(kernel));
     if (e != cudaSuccess) return e;
     kernel<<<n_blocks, warps_per_block * 32, smem_bytes, st>>>(a);
@@ -1130,9 +1280,12 @@ static int max_warps_by_registers(const void *kernel) {
 }
 
 int scan_max_warps_by_registers(bool query_in_smem) {
-    const int w = max_warps_by_registers(reinterpret_cast<const void *>(single_kernel(query_in_smem, false)));
-    if (!query_in_smem) return w;
-    return std::min(w, max_warps_by_registers(reinterpret_cast<const void *>(single_kernel(true, true))));
+    int w = kScanMaxWarpsPerBlock;
+    for (bool bands : {false, true})
+        for (bool table : {false, true})
+            w = std::min(w, max_warps_by_registers(reinterpret_cast<const void *>(
+                                single_kernel(query_in_smem, table && query_in_smem, bands))));
+    return w;
 }
 
 static void (*batch_kernel(bool query_in_smem, bool word_table))(ScanArgs) {
@@ -1163,9 +1316,9 @@ int scan_batch_max_warps_by_registers(bool query_in_smem) {
     return std::min(w, max_warps_by_registers(reinterpret_cast<const void *>(batch_kernel(true, true))));
 }
 
-cudaError_t scan_occupancy(bool query_in_smem, bool word_table, int warps_per_block, size_t smem_bytes,
+cudaError_t scan_occupancy(bool query_in_smem, bool word_table, bool bands, int warps_per_block, size_t smem_bytes,
                            int *blocks_per_sm) {
-    auto kernel = single_kernel(query_in_smem, word_table);
+    auto kernel = single_kernel(query_in_smem, word_table, bands);
     cudaError_t e = allow_full_smem(reinterpret_cast<const void *>(kernel));
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel, warps_per_block * 32,
