@@ -2,13 +2,16 @@
 // 28^3 words, the query offsets whose word scores at least the threshold
 // against it, or equals it (BLAZE_ncbi/prelim_stage.cpp:135-155, :378-386).
 //
-// One thread per word walks the query, so a word's offsets come out ascending
-// and no neighbourhood lists are needed: 21,952 threads x the query's length
-// x about ten instructions, a few microseconds for a protein. One pass counts,
-// a block per query turns the counts into the tables, a second pass writes the
-// offsets. Built on the host instead, a 350-residue query's call over a proteome
-// took 542 us against 470, and 64 queries arriving at a server 29.8 ms against
-// 29.0.
+// A block takes the 28 words that begin with one pair of letters, its warps a
+// part of the query each, a lane per offset: where the pair's score leaves a
+// third letter that can reach the threshold the offset is a candidate (about one
+// in twenty at the default), and full batches of candidates are tested against
+// the 28 letters, a ballot each. So a word's offsets come out ascending and no
+// neighbourhood lists are needed. One pass counts, a block per query turns the
+// counts into the tables, a second pass writes the offsets.
+// The passes are bound by the latency of their steps, 32 offsets each: 8 and 13
+// us at 300 query residues, 31 and 65 at 12,345, where a thread per word that
+// walked the query alone took 0.5 ms a pass.
 #include <algorithm>
 #include <cstdint>
 
@@ -21,49 +24,115 @@ __device__ const int32_t g_blosum_lk[kAlphabet * kAlphabet] = {
 #include "blosum62.inc"
 };
 
-constexpr int kLookupThreads = 256;
-constexpr int kLookupTile = 512;  // query offsets staged at a time
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kLookupWarps = 8;                // per block, each with a part of the query
+constexpr int kPairs = kAlphabet * kAlphabet;  // pairs of letters, a block each
+constexpr int kRow = kAlphabet + 1;            // of the matrix in shared memory: an odd stride, so that the
+                                               // lanes' rows lie in different banks
 
-// A query offset's word as the walk reads it: its letters' rows in the matrix
-// (byte offsets) and the word itself.
-struct Pos {
-    uint32_t row0, row1, row2, word;
+struct WalkShared {
+    int32_t mat[kAlphabet * kRow];
+    int32_t best[kAlphabet];          // of a row
+    uint32_t cand[kLookupWarps][64];  // offset | third letter << 16 | starts with the pair << 31
+    int32_t cand_score[kLookupWarps][64];
+    uint32_t count[kLookupWarps][32];  // by third letter
 };
 
-// Calls hit(i) for each query offset i whose word is in the thread's cell.
+__device__ __forceinline__ void walk_setup(WalkShared &sh) {
+    for (int i = threadIdx.x; i < kPairs; i += blockDim.x)
+        sh.mat[i / kAlphabet * kRow + i % kAlphabet] = g_blosum_lk[i];
+    __syncthreads();
+    if (threadIdx.x < kAlphabet) {
+        int32_t m = sh.mat[threadIdx.x * kRow];
+        for (int k = 1; k < kAlphabet; ++k) m = max(m, sh.mat[threadIdx.x * kRow + k]);
+        sh.best[threadIdx.x] = m;
+    }
+    __syncthreads();
+}
+
+// The warp's part of the query: calls hit(c, mask, i) for each third letter c
+// and batch of candidates: the lanes in mask have the word's offset i. Every
+// lane makes every call.
 template <typename F>
-__device__ __forceinline__ void walk_query(const LookupQuery &lq, int32_t threshold, uint32_t word, F hit) {
-    __shared__ int32_t mat[kAlphabet * kAlphabet];
-    __shared__ Pos tile[kLookupTile];
-    for (int i = threadIdx.x; i < kAlphabet * kAlphabet; i += blockDim.x) mat[i] = g_blosum_lk[i];
-    const int32_t n = lq.qlen - (kWordSize - 1);
-    const uint32_t a = min(word / 784u, 27u), b = word / 28u % 28u, c = word % 28u;
-    const int32_t *m0 = mat + a, *m1 = mat + b, *m2 = mat + c;
-    for (int32_t i0 = 0; i0 < n; i0 += kLookupTile) {
-        __syncthreads();
-        const int32_t m = min(n - i0, kLookupTile);
-        for (int32_t i = threadIdx.x; i < m; i += blockDim.x) {
-            const uint8_t *q = lq.q + i0 + i;
-            const uint32_t x = q[0], y = q[1], z = q[2];
-            tile[i] = Pos{x * kAlphabet, y * kAlphabet, z * kAlphabet, x * 784u + y * 28u + z};
-        }
-        __syncthreads();
+__device__ __forceinline__ void walk_query(WalkShared &sh, const LookupQuery &lq, int32_t threshold, F hit) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t a = blockIdx.x / kAlphabet, b = blockIdx.x % kAlphabet;
+    const int32_t *mat = sh.mat;
+    uint32_t *cand = sh.cand[warp];
+    int32_t *cand_score = sh.cand_score[warp];
+    const int32_t all = max(lq.qlen - (kWordSize - 1), 0);
+    const int32_t part = ((all + kLookupWarps - 1) / kLookupWarps + 31) & ~31;
+    const int32_t from = min(part * static_cast<int32_t>(warp), all), n = min(from + part, all);
+    uint32_t have = 0;
+    auto test = [&](uint32_t m) {  // the first m candidates
+        const bool in = lane < m;
+        const uint32_t w = in ? cand[lane] : 0u;
+        const int32_t s = in ? cand_score[lane] : 0;
+        const uint32_t z = (w >> 16) & 31u;
+        const bool same = (w >> 31) != 0u;
 #pragma unroll 4
-        for (int32_t i = 0; i < m; ++i) {
-            const Pos p = tile[i];
-            if (m0[p.row0] + m1[p.row1] + m2[p.row2] >= threshold || p.word == word) hit(i0 + i);
+        for (uint32_t c = 0; c < kAlphabet; ++c) {
+            const bool h = in && (s + mat[z * kRow + c] >= threshold || (same && z == c));
+            hit(c, __ballot_sync(kFull, h), w & 0xffffu);
+        }
+    };
+    for (int32_t i0 = from; i0 < n; i0 += 32) {
+        const int32_t i = i0 + static_cast<int32_t>(lane);
+        bool is = false, same = false;
+        uint32_t z = 0;
+        int32_t s = 0;
+        if (i < n) {
+            const uint32_t x = lq.q[i], y = lq.q[i + 1];
+            z = lq.q[i + 2];
+            s = mat[x * kRow + a] + mat[y * kRow + b];
+            same = x == a && y == b;
+            is = same || s + sh.best[z] >= threshold;
+        }
+        const uint32_t m = __ballot_sync(kFull, is);
+        if (is) {
+            const uint32_t at = have + __popc(m & ((1u << lane) - 1u));
+            cand[at] = static_cast<uint32_t>(i) | (z << 16) | (same ? 0x80000000u : 0u);
+            cand_score[at] = s;
+        }
+        have += __popc(m);
+        __syncwarp();
+        if (have >= 32u) {
+            test(32u);
+            have -= 32u;
+            __syncwarp();
+            const uint32_t w = cand[32u + lane];
+            const int32_t ws = cand_score[32u + lane];
+            if (lane < have) {
+                cand[lane] = w;
+                cand_score[lane] = ws;
+            }
+            __syncwarp();
         }
     }
+    if (have) test(have);
+}
+
+// The warp's counts, by third letter.
+__device__ __forceinline__ void walk_count(WalkShared &sh, const LookupQuery &lq, int32_t threshold) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t n = 0;  // lane c: of the word with third letter c
+    walk_query(sh, lq, threshold, [&](uint32_t c, uint32_t mask, uint32_t) { n += lane == c ? __popc(mask) : 0; });
+    sh.count[threadIdx.x >> 5][lane] = n;
+    __syncthreads();
 }
 
 // Counts of every word, left in cell_start.
-__global__ void __launch_bounds__(kLookupThreads)
+__global__ void __launch_bounds__(kLookupWarps * 32)
 lookup_count_kernel(const LookupQuery one, const LookupQuery *many, int32_t threshold) {
+    __shared__ WalkShared sh;
     const LookupQuery lq = many ? many[blockIdx.y] : one;
-    const uint32_t word = blockIdx.x * kLookupThreads + threadIdx.x;
-    uint32_t n = 0;
-    walk_query(lq, threshold, word, [&](int32_t) { ++n; });
-    if (word < static_cast<uint32_t>(kWords)) lq.cell_start[word] = n;
+    walk_setup(sh);
+    walk_count(sh, lq, threshold);
+    if (threadIdx.x < kAlphabet) {
+        uint32_t n = 0;
+        for (int w = 0; w < kLookupWarps; ++w) n += sh.count[w][threadIdx.x];
+        lq.cell_start[blockIdx.x * kAlphabet + threadIdx.x] = n;
+    }
 }
 
 // One block per query: starts, packed cells (start << 8 | min(count, 255)) and
@@ -107,14 +176,23 @@ __global__ void __launch_bounds__(1024) lookup_tables_kernel(const LookupQuery o
     }
 }
 
-__global__ void __launch_bounds__(kLookupThreads)
+// The offsets; a warp counts its part first, for where the next one's begin.
+__global__ void __launch_bounds__(kLookupWarps * 32)
 lookup_write_kernel(const LookupQuery one, const LookupQuery *many, int32_t threshold) {
+    __shared__ WalkShared sh;
     const LookupQuery lq = many ? many[blockIdx.y] : one;
-    const uint32_t word = blockIdx.x * kLookupThreads + threadIdx.x;
-    uint16_t *out = lq.cell_off + (word < static_cast<uint32_t>(kWords) ? lq.cell_start[word] : 0u);
-    const bool own = word < static_cast<uint32_t>(kWords);
-    walk_query(lq, threshold, word, [&](int32_t i) {
-        if (own) *out++ = static_cast<uint16_t>(i);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    walk_setup(sh);
+    walk_count(sh, lq, threshold);
+    uint32_t to = 0;  // lane c: where the next offset of its word goes
+    if (lane < kAlphabet) {
+        to = lq.cell_start[blockIdx.x * kAlphabet + lane];
+        for (uint32_t w = 0; w < warp; ++w) to += sh.count[w][lane];
+    }
+    walk_query(sh, lq, threshold, [&](uint32_t c, uint32_t mask, uint32_t i) {
+        const uint32_t at = __shfl_sync(kFull, to, c) + __popc(mask & ((1u << lane) - 1u));
+        if ((mask >> lane) & 1u) lq.cell_off[at] = static_cast<uint16_t>(i);
+        to += lane == c ? __popc(mask) : 0;
     });
 }
 
@@ -122,14 +200,14 @@ lookup_write_kernel(const LookupQuery one, const LookupQuery *many, int32_t thre
 
 cudaError_t launch_lookup(const LookupQuery &one, const LookupQuery *many, uint32_t n, int32_t threshold,
                           cudaStream_t st) {
-    constexpr uint32_t kBlocks = (kWords + kLookupThreads - 1) / kLookupThreads;
+    constexpr uint32_t kBlocks = kPairs;
     constexpr uint32_t kMost = 32768;  // queries per launch (the grid's y extent)
     for (uint32_t i = 0; i < n; i += kMost) {
         const LookupQuery *m = many ? many + i : nullptr;
         const uint32_t k = std::min(n - i, kMost);
-        lookup_count_kernel<<<dim3(kBlocks, k), kLookupThreads, 0, st>>>(one, m, threshold);
+        lookup_count_kernel<<<dim3(kBlocks, k), kLookupWarps * 32, 0, st>>>(one, m, threshold);
         lookup_tables_kernel<<<k, 1024, 0, st>>>(one, m);
-        lookup_write_kernel<<<dim3(kBlocks, k), kLookupThreads, 0, st>>>(one, m, threshold);
+        lookup_write_kernel<<<dim3(kBlocks, k), kLookupWarps * 32, 0, st>>>(one, m, threshold);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
