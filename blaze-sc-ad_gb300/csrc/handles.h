@@ -76,6 +76,12 @@ struct DevBuf {
     }
 };
 
+// A subject's HSP list in the results' order: by query, then OID.
+struct ListKey {
+    uint64_t key;
+    uint32_t at;  // in the published lists
+};
+
 struct blaze_search {
     blaze_db *db = nullptr;
     cudaStream_t stream = nullptr;
@@ -95,6 +101,7 @@ struct blaze_search {
     size_t h_out_n = 0;
     int gapped_blocks = 0;
     unsigned long long lane_dp_slots = kLaneDpSlots;
+    std::vector<ListKey> order[2];  // the lists' order, and space to sort it
     std::vector<blaze_hsp> results;
     blaze_stats stats{};
     unsigned long long last_init_count = 0, last_work_count = 0;

@@ -100,9 +100,10 @@ static int traceback_passes(blaze_search *s, const std::vector<TbItem> &items, c
 
 // One subject's traced HSPs: purged of shared start and end points (the
 // better kept), ordered as the preliminary stage orders them, given final
-// E-values and bit scores and reaped at `evalue`; appended to `out`.
-static void traceback_finish_subject(std::vector<TbOut> g, uint32_t oid, const blaze_params &p, double evalue,
-                                     std::vector<blaze_aligned_hsp> &out) {
+// E-values and bit scores and reaped at `evalue`; appended to `out` (`g` is
+// space for them).
+static void traceback_finish_subject(const TbOut *first, const TbOut *last, uint32_t oid, const blaze_params &p,
+                                     double evalue, std::vector<TbOut> &g, std::vector<blaze_aligned_hsp> &out) {
     auto by_start = [](const TbOut &a, const TbOut &b) {
         if (a.q_start != b.q_start) return a.q_start < b.q_start;
         if (a.s_start != b.s_start) return a.s_start < b.s_start;
@@ -124,17 +125,20 @@ static void traceback_finish_subject(std::vector<TbOut> g, uint32_t oid, const b
         if (a.q_start != b.q_start) return a.q_start < b.q_start;
         return a.q_end > b.q_end;
     };
-    std::stable_sort(g.begin(), g.end(), by_start);
-    std::vector<TbOut> m;
-    for (const TbOut &o : g)
-        if (m.empty() || o.q_start != m.back().q_start || o.s_start != m.back().s_start) m.push_back(o);
-    std::stable_sort(m.begin(), m.end(), by_end);
-    std::vector<TbOut> m2;
-    for (const TbOut &o : m)
-        if (m2.empty() || o.q_end != m2.back().q_end || o.s_end != m2.back().s_end) m2.push_back(o);
-    std::stable_sort(m2.begin(), m2.end(), by_score);
+    g.assign(first, last);
+    if (g.size() > 1) {
+        std::stable_sort(g.begin(), g.end(), by_start);
+        g.erase(std::unique(g.begin(), g.end(),
+                            [](const TbOut &a, const TbOut &b) { return a.q_start == b.q_start && a.s_start == b.s_start; }),
+                g.end());
+        std::stable_sort(g.begin(), g.end(), by_end);
+        g.erase(std::unique(g.begin(), g.end(),
+                            [](const TbOut &a, const TbOut &b) { return a.q_end == b.q_end && a.s_end == b.s_end; }),
+                g.end());
+        std::stable_sort(g.begin(), g.end(), by_score);
+    }
     const double ln2 = std::log(2.0), lnK = std::log(p.K);
-    for (const TbOut &o : m2) {
+    for (const TbOut &o : g) {
         blaze_aligned_hsp h{};
         h.oid = oid;
         h.score = o.score;
@@ -180,11 +184,13 @@ extern "C" int blaze_search_traceback(blaze_search *s, const blaze_query *q, con
     if ((rc = traceback_passes(s, items, p, final_xdrop, q->d_q, q->qlen, nullptr, nullptr, q->qlen, outs)) !=
         BLAZE_OK)
         return rc;
+    std::vector<TbOut> space;
+    s->tb_results.reserve(n);
     for (size_t i = 0; i < n;) {
         size_t j = i;
         while (j < n && s->results[j].oid == s->results[i].oid) ++j;
-        traceback_finish_subject(std::vector<TbOut>(outs.begin() + i, outs.begin() + j), s->results[i].oid, *p,
-                                 evalue, s->tb_results);
+        traceback_finish_subject(outs.data() + i, outs.data() + j, s->results[i].oid, *p, evalue, space,
+                                 s->tb_results);
         i = j;
     }
     if (n_hsps) *n_hsps = s->tb_results.size();
@@ -216,14 +222,15 @@ extern "C" int blaze_search_traceback_batch(blaze_search *s, const blaze_batch *
     if ((rc = traceback_passes(s, items, &params[0], final_xdrop, nullptr, 0, s->bqptr.p, s->bqlen.p, max_qlen,
                                outs)) != BLAZE_OK)
         return rc;
+    std::vector<TbOut> space;
     std::vector<blaze_aligned_hsp> one;
+    s->tb_batch_results.reserve(n);
     for (size_t i = 0; i < n;) {
         size_t j = i;
         const uint32_t qi = s->batch_results[i].query, oid = s->batch_results[i].hsp.oid;
         while (j < n && s->batch_results[j].query == qi && s->batch_results[j].hsp.oid == oid) ++j;
         one.clear();
-        traceback_finish_subject(std::vector<TbOut>(outs.begin() + i, outs.begin() + j), oid, params[qi], evalue,
-                                 one);
+        traceback_finish_subject(outs.data() + i, outs.data() + j, oid, params[qi], evalue, space, one);
         for (const blaze_aligned_hsp &h : one) s->tb_batch_results.push_back(blaze_batch_aligned_hsp{qi, 0u, h});
         i = j;
     }
