@@ -305,6 +305,8 @@ extern "C" int blaze_search_free(blaze_search *s) {
     if (s->h_stage) cudaFreeHost(s->h_stage);
     s->tb_items.release();
     s->tb_out.release();
+    s->tb_part.release();
+    s->tb_done.release();
     s->tb_dirs.release();
     s->tb_rows.release();
     s->tb_dp.release();

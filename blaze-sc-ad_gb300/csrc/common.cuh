@@ -282,6 +282,13 @@ struct TbOut {
     int32_t cells;   // DP cells computed (left and right)
 };
 
+// One side of a traced HSP: the DP's best cell (rows, columns from the start
+// point) and the path's counts; last: the kind of its move next to the start
+// point (0 a pair, 1 and 2 gaps, -1 none). status as in TbOut.
+struct TbPart {
+    int32_t score, a, b, pairs, identities, positives, gaps, gap_opens, last, status, cells;
+};
+
 struct TracebackArgs {
     const uint8_t *res;
     const uint64_t *off;
@@ -297,8 +304,10 @@ struct TracebackArgs {
     uint32_t dp_stride;
     uint8_t *dirs;              // per warp: dir_cap direction bytes
     unsigned long long dir_cap;
-    int32_t *rows;              // per warp: 3 ints (first, end, offset) per DP row
+    int32_t *rows;              // per warp: 3 ints per DP row
     uint32_t row_cap;
+    TbPart *part;               // per item: left and right side
+    unsigned int *done;         // per item: sides done (zeroed)
     unsigned long long *cursor;
 };
 
@@ -313,6 +322,7 @@ cudaError_t launch_gapped(const GappedArgs &a, int n_blocks, cudaStream_t st,
                           int warps_per_block = kGappedWarpsPerBlock);
 cudaError_t launch_hitlist(const HitlistArgs &a, uint32_t n_select, int n_sm, cudaStream_t st);
 constexpr int kTracebackWarpsPerBlock = 4;
+constexpr int kTracebackBlocksPerSm = 5;
 cudaError_t launch_traceback(const TracebackArgs &a, int n_blocks, cudaStream_t st);
 cudaError_t launch_scan_batch(const ScanArgs &a, bool word_table, int n_blocks, int warps_per_block, size_t smem,
                               cudaStream_t st);

@@ -139,6 +139,8 @@ struct blaze_search {
     // traceback stage
     DevBuf<TbItem> tb_items;
     DevBuf<TbOut> tb_out;
+    DevBuf<TbPart> tb_part;
+    DevBuf<unsigned int> tb_done;
     DevBuf<uint8_t> tb_dirs;
     DevBuf<int32_t> tb_rows, tb_dp;
     DevBuf<unsigned long long> tb_cursor;

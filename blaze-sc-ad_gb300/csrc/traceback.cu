@@ -5,10 +5,11 @@
 // reference this is NCBI's traceback stage after the preliminary search,
 // BLAZE_ncbi/prelim_stage.cpp:1462-1498).
 //
-// One warp per HSP. The left and right X-drop DPs run row-parallel exactly as
-// in the gapped stage; every computed cell also stores a direction byte in
-// the warp's buffer (row by row over the band). Lane 0 then walks the path
-// back from the best cell.
+// One warp per side of an HSP. The X-drop DP runs row by row with its band in
+// registers, as in the gapped stage; every row's direction bytes go to the
+// warp's buffer. The warp then walks the path back from the best cell, 32 cells
+// of a diagonal at a time. Where the band outgrows the registers the rows are
+// kept in memory and one lane walks.
 #include <cstdint>
 
 #include "common.cuh"
@@ -277,7 +278,234 @@ __device__ Walk walk_back(const DirRows &d, int32_t rows, const uint8_t *A, cons
     return w;
 }
 
-__global__ void __launch_bounds__(kTracebackWarpsPerBlock * 32) traceback_kernel(const TracebackArgs a) {
+// The same DP with the band in registers: a window of 192 columns, parts of 64,
+// lane i holding H and E of columns w0 + 2i and w0 + 2i + 1 of each. A part is
+// computed only in rows whose band reaches it; the window moves right when the
+// band outgrows its first part. A row's direction bytes begin at its own w0:
+// d.rows holds w0 and where they are. H of every dead cell is -inf, and E of a
+// dead cell is at most its H was, so neither changes a live cell's direction.
+// Row letter k is Q[dir * k], column letter k is S[dir * k]. Returns false when
+// the band does not fit the window.
+//
+// Bound by instruction issue and by the chain of a row's steps. 7,756 sides of
+// 500 query residues: 1.20 ms with the rows in memory, both sides on one warp and
+// one lane walking back; 1.06 with 128 columns (many bands outgrow them), 0.62
+// with 192 and 20 warps an SM, 0.70 with 192 or 256 and 16 warps.
+constexpr int kTbParts = 3, kTbWindow = 64 * kTbParts;
+constexpr int kTbRowMost = kTbWindow + 64;  // bytes of a row: the window, moved by less than 64, holds its end
+__device__ __forceinline__ bool xdrop_dp_window_dirs(const uint8_t *__restrict__ Q, const uint8_t *__restrict__ S,
+                                                     int32_t dir, int32_t M, int32_t N, int32_t gap_open,
+                                                     int32_t gap_extend, int32_t xdrop, const int32_t *mat, DirRows &d,
+                                                     TbPart &out) {
+    const int lane = threadIdx.x & 31;
+    const int32_t goe = gap_open + gap_extend, ge = gap_extend;
+    if (xdrop < goe) xdrop = goe;
+    if (M <= 0 || N <= 0) return true;
+    int32_t bsize = 1 + min(N, (xdrop - goe) / ge + 1);
+    if (bsize > kTbWindow) return false;
+    if (static_cast<uint32_t>(M) + 1 > d.row_cap) {
+        d.overflow = true;
+        return true;
+    }
+    int2 *rows_out = reinterpret_cast<int2 *>(d.rows);
+    int32_t w0 = 0, at = 0;
+    auto letter = [&](int32_t b) { return b >= 1 && b <= N ? static_cast<int32_t>(S[dir * b]) : 0; };
+    int32_t h[2 * kTbParts], e[2 * kTbParts], l[2 * kTbParts];  // per part: the lane's two columns
+#pragma unroll
+    for (int j = 0; j < 2 * kTbParts; ++j) {
+        const int32_t b = 64 * (j >> 1) + 2 * lane + (j & 1);
+        l[j] = letter(b);
+        h[j] = b >= bsize ? kNeg : b == 0 ? 0 : -goe - (b - 1) * ge;
+        e[j] = b >= bsize ? kNeg : h[j] - goe;
+    }
+    int32_t best = 0, first = 0, ab = 0, bb = 0, n_cells = 0;
+    int32_t rows = 0;  // lane i: the matrix row of row letter (a - 1) rounded down to 32, plus i + 1
+    for (int32_t a = 1; a <= M; ++a) {
+        if (static_cast<unsigned long long>(at) + kTbRowMost > d.cap) {
+            d.overflow = true;
+            return true;
+        }
+        const int32_t ai = (a - 1) & 31;
+        if (ai == 0) rows = a + lane <= M ? kAlphabet * static_cast<int32_t>(Q[dir * (a + lane)]) : 0;
+        const int32_t *row = mat + __shfl_sync(kFull, rows, ai);
+        if (lane == 0) rows_out[a] = make_int2(w0, at);
+        uint8_t *dirs = d.dir + at - w0;  // a column's byte
+        n_cells += bsize - first;
+        int32_t carry_p = kNeg, carry_h = kNeg;  // into the next part
+        int32_t lo = INT32_MAX, hi = -1;         // the first and last live column
+        int32_t row_end = w0;                    // of the parts computed
+        auto part = [&](int s, int32_t &h0, int32_t &h1, int32_t &e0, int32_t &e1, int32_t l0, int32_t l1) {
+            const int32_t b0 = w0 + 64 * s + 2 * lane, b1 = b0 + 1, gb = ge * b0;
+            const bool in0 = b0 < bsize, in1 = b1 < bsize;
+            int32_t hprev = __shfl_up_sync(kFull, h1, 1);
+            if (lane == 0) hprev = carry_h;
+            const int32_t g0 = hprev + row[l0], g1 = h0 + row[l1];  // by the diagonal
+            const int32_t d0 = in0 ? max(g0, e0) : kNeg, d1 = in1 ? max(g1, e1) : kNeg;
+            // row gap: prefix maximum of D + ge * column over the columns before each
+            const int32_t p0 = d0 + gb, p1 = d1 + gb + ge;
+            int32_t incl = max(p0, p1);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) incl = max(incl, __shfl_up_sync(kFull, incl, o));  // lanes < o get their own
+            int32_t excl = __shfl_up_sync(kFull, incl, 1);
+            if (lane == 0) excl = kNeg;
+            excl = max(excl, carry_p);
+            const int32_t open = ge - goe - gb;
+            const int32_t f0 = excl + open, f1 = max(excl, p0) + open - ge;
+            const int32_t H0 = in0 ? max(f0, d0) : kNeg, H1 = in1 ? max(f1, d1) : kNeg;
+            const int32_t top = max(H0, H1), cm = __reduce_max_sync(kFull, top);
+            int32_t thr0 = best - xdrop, thr1 = thr0;  // live from there on
+            if (cm > best) {
+                int32_t t = top;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) t = max(t, __shfl_up_sync(kFull, t, o));
+                t = __shfl_up_sync(kFull, t, 1);
+                if (lane > 0) thr0 = max(thr0, t - xdrop);
+                thr1 = max(thr0, H0 - xdrop);
+                const unsigned m0 = __ballot_sync(kFull, H0 == cm), m1 = __ballot_sync(kFull, H1 == cm);
+                const int fl = __ffs(m0 | m1) - 1;
+                ab = a;
+                bb = w0 + 64 * s + 2 * fl + ((m0 >> fl) & 1u ? 0 : 1);
+                best = cm;
+            }
+            const bool alive0 = H0 >= thr0, alive1 = H1 >= thr1;
+            lo = min(lo, __reduce_min_sync(kFull, alive0 ? b0 : alive1 ? b1 : INT32_MAX));
+            hi = max(hi, __reduce_max_sync(kFull, alive1 ? b1 : alive0 ? b0 : -1));
+            auto direction = [&](bool alive, int32_t g, int32_t ein, int32_t f, int32_t H) {
+                uint32_t v = max(g, ein) < f ? kTbF : g < ein ? kTbE : kTbDiag;
+                if (H - goe <= ein - ge) v |= kTbEExt;
+                if (H - goe <= f - ge) v |= kTbFExt;
+                return alive ? v : static_cast<uint32_t>(kTbDead);
+            };
+            const uint32_t v0 = direction(alive0, g0, e0, f0, H0), v1 = direction(alive1, g1, e1, f1, H1);
+            *reinterpret_cast<uint16_t *>(dirs + b0) = static_cast<uint16_t>(v0 | (v1 << 8));
+            if (s + 1 < kTbParts) carry_h = __shfl_sync(kFull, h1, 31);
+            // live cells hand on; dead ones keep their E
+            if (alive0) e0 = max(H0 - goe, e0 - ge);
+            if (alive1) e1 = max(H1 - goe, e1 - ge);
+            h0 = alive0 ? H0 : kNeg;
+            h1 = alive1 ? H1 : kNeg;
+            carry_p = max(carry_p, __shfl_sync(kFull, incl, 31));
+            row_end = w0 + 64 * (s + 1);
+        };
+#pragma unroll
+        for (int s = 0; s < kTbParts; ++s)
+            if (s == 0 || bsize > w0 + 64 * s) part(s, h[2 * s], h[2 * s + 1], e[2 * s], e[2 * s + 1], l[2 * s], l[2 * s + 1]);
+        if (hi < 0) break;
+        first = lo;
+        const int32_t from = hi + 1;  // columns from here on are outside, or the row gap's
+        int32_t n_ext = 0, F = 0;
+        if (from == bsize && bsize <= N) {
+            F = carry_p - goe + ge - ge * bsize;
+            const int32_t room = F - (best - xdrop);
+            if (room >= 0) n_ext = min(N - bsize + 1, room / ge + 1);
+        }
+        bsize = from + n_ext;
+        if (bsize <= N) ++bsize;  // the next column, -inf so far
+        // move the window when the band leaves its first part (unless that
+        // gains little) or the window itself
+        const int32_t behind = first - w0, reach = bsize - w0, w_row = w0;
+        if (reach > 64 && (behind >= 16 || reach > kTbWindow || (behind >= 4 && reach - behind < 64))) {
+            const int32_t by = min(behind >> 1, 31);
+            w0 += 2 * by;
+            if (bsize - w0 > kTbWindow) return false;
+            const int src = (lane + by) & 31;
+            const bool same = lane + by < 32;
+#pragma unroll
+            for (int j = 0; j < 2 * kTbParts; ++j) {
+                const int32_t hn = j + 2 < 2 * kTbParts ? h[j + 2 < 2 * kTbParts ? j + 2 : j] : kNeg;
+                const int32_t en = j + 2 < 2 * kTbParts ? e[j + 2 < 2 * kTbParts ? j + 2 : j] : kNeg;
+                const int32_t ha = __shfl_sync(kFull, h[j], src), hb = __shfl_sync(kFull, hn, src);
+                const int32_t ea = __shfl_sync(kFull, e[j], src), eb = __shfl_sync(kFull, en, src);
+                h[j] = same ? ha : hb;
+                e[j] = same ? ea : eb;
+            }
+#pragma unroll
+            for (int j = 0; j < 2 * kTbParts; ++j) l[j] = letter(w0 + 64 * (j >> 1) + 2 * lane + (j & 1));
+        }
+        if (n_ext > 0) {
+#pragma unroll
+            for (int j = 0; j < 2 * kTbParts; ++j) {
+                const int32_t t = w0 + 64 * (j >> 1) + 2 * lane + (j & 1) - from;
+                if (t >= 0 && t < n_ext) {
+                    h[j] = F - t * ge;
+                    e[j] = h[j] - goe;
+                }
+            }
+            __syncwarp();  // the last part's bytes are there
+            for (int32_t t = lane; t < n_ext; t += 32) dirs[from + t] = static_cast<uint8_t>(kTbF | kTbFExt);
+        }
+        at += (max(row_end, bsize) - w_row + 63) & ~63;
+    }
+    out.score = best;
+    out.a = ab;
+    out.b = bb;
+    out.cells += n_cells;
+    __syncwarp();
+    return true;
+}
+
+// The path from the best cell of xdrop_dp_window_dirs back to the origin, by
+// the whole warp: lane i looks at the cell i steps up the diagonal, and the
+// leading cells that came from their diagonal are passed at once.
+__device__ __forceinline__ void walk_window(const DirRows &d, const uint8_t *__restrict__ Q,
+                                            const uint8_t *__restrict__ S, int32_t dir, const int32_t *mat,
+                                            TbPart &p) {
+    const int32_t lane = threadIdx.x & 31;
+    const int2 *rows = reinterpret_cast<const int2 *>(d.rows);
+    int32_t a = p.a, b = p.b;
+    auto byte_at = [&](int32_t ra, int32_t cb) {  // -1: not in the row
+        const int2 r = rows[ra];
+        const int32_t k = cb - r.x;
+        return k >= 0 && k < kTbRowMost ? static_cast<int32_t>(d.dir[r.y + k]) : -1;
+    };
+    p.status = 2;
+    while (a > 0) {
+        const int32_t ra = a - lane, cb = b - lane;
+        const int32_t v = ra > 0 && cb >= 0 ? byte_at(ra, cb) : -1;
+        const bool diag = cb > 0 && v >= 0 && (v & (kTbDead | 3)) == kTbDiag;
+        const unsigned m = __ballot_sync(kFull, diag);
+        const int32_t n = m == kFull ? 32 : __ffs(~m) - 1;
+        if (n > 0) {
+            const bool in = lane < n;
+            const uint32_t x = in ? Q[dir * ra] : 0u, y = in ? S[dir * cb] : 0u;
+            p.pairs += n;
+            p.identities += __popc(__ballot_sync(kFull, in && x == y));
+            p.positives += __popc(__ballot_sync(kFull, in && mat[x * kAlphabet + y] > 0));
+            p.last = 0;
+            a -= n;
+            b -= n;
+            if (n == 32 || a == 0) continue;
+        }
+        const int32_t here = __shfl_sync(kFull, v, n);
+        if (here < 0 || (here & kTbDead)) return;
+        const int32_t kind = (here & 3) == kTbE ? 1 : 2;  // a gap: down the rows, or along this row
+        if (p.last != kind) ++p.gap_opens;
+        p.last = kind;
+        for (bool on = true; on;) {
+            ++p.gaps;
+            if (kind == 1) {
+                --a;
+                const int32_t w = a > 0 ? byte_at(a, b) : 0;
+                if (w < 0) return;
+                on = (w & kTbEExt) != 0;
+            } else {
+                --b;
+                const int32_t w = b >= 0 ? byte_at(a, b) : -1;
+                if (w < 0) return;
+                on = (w & kTbFExt) != 0;
+            }
+        }
+    }
+    if (b > 0) {  // along row 0
+        if (p.last != 2) ++p.gap_opens;
+        p.last = 2;
+        p.gaps += b;
+    }
+    p.status = 0;
+}
+
+__global__ void __launch_bounds__(kTracebackWarpsPerBlock * 32, kTracebackBlocksPerSm)
+traceback_kernel(const TracebackArgs a) {
     __shared__ int32_t mat[kAlphabet * kAlphabet];
     for (int i = threadIdx.x; i < kAlphabet * kAlphabet; i += blockDim.x) mat[i] = g_blosum_tb[i];
     __syncthreads();
@@ -294,44 +522,73 @@ __global__ void __launch_bounds__(kTracebackWarpsPerBlock * 32) traceback_kernel
         unsigned long long t = 0;
         if (lane == 0) t = atomicAdd(a.cursor, 1ull);
         t = __shfl_sync(kFull, t, 0);
-        if (t >= a.n_items) break;
-        const TbItem it = a.items[t];
+        if (t >= 2ull * a.n_items) break;
+        const bool is_left = (t & 1ull) == 0;
+        const unsigned long long ti = t >> 1;
+        const TbItem it = a.items[ti];
         const uint64_t o0 = a.off[it.subject];
         const uint8_t *sub = a.res + o0;
         const int32_t slen = static_cast<int32_t>(a.off[it.subject + 1] - o0);
         const int32_t q_off = it.q_off, s_off = it.s_off;
         const uint8_t *qres = a.batch_q ? a.batch_q[it.query] : a.q;
         const int32_t qlen = a.batch_q ? a.batch_qlen[it.query] : a.qlen;
+        // row and column letter k at Q[dir * k] and S[dir * k]
+        const int32_t dir = is_left ? -1 : 1;
+        const uint8_t *Q = qres + q_off + (is_left ? 1 : 0), *S = sub + s_off + (is_left ? 1 : 0);
+        const int32_t M = is_left ? q_off + 1 : qlen - q_off - 1, N = is_left ? s_off + 1 : slen - s_off - 1;
         d.overflow = false;
-        int32_t al, bl, ar = 0, br = 0, right = 0, rows, cells = 0;
-        TbOut o{};
-        const int32_t left = xdrop_dp_dirs<true>(qres, sub, q_off + 1, s_off + 1, a.gap_open, a.gap_extend, a.xdrop,
-                                                 mat, Hb, Eb, &al, &bl, d, &rows, &cells);
-        Walk wl{0, 0, 0, 0, 0, -1, true}, wr{0, 0, 0, 0, 0, -1, true};
-        if (!d.overflow && lane == 0) wl = walk_back<true>(d, rows, qres, sub, q_off + 1, s_off + 1, al, bl, mat);
-        __syncwarp();
-        if (!d.overflow && q_off < qlen - 1 && s_off < slen - 1) {
-            right = xdrop_dp_dirs<false>(qres + q_off, sub + s_off, qlen - q_off - 1, slen - s_off - 1, a.gap_open,
-                                         a.gap_extend, a.xdrop, mat, Hb, Eb, &ar, &br, d, &rows, &cells);
-            if (!d.overflow && lane == 0)
-                wr = walk_back<false>(d, rows, qres + q_off, sub + s_off, qlen - q_off - 1, slen - s_off - 1, ar,
-                                      br, mat);
+        TbPart p{};
+        p.last = -1;
+        if (xdrop_dp_window_dirs(Q, S, dir, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, d, p)) {
+            if (!d.overflow) walk_window(d, Q, S, dir, mat, p);
+        } else {
+            __syncwarp();
+            int32_t rows;
+            Walk w{0, 0, 0, 0, 0, -1, true};
+            if (is_left) {
+                p.score = xdrop_dp_dirs<true>(qres, sub, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, Hb, Eb, &p.a,
+                                              &p.b, d, &rows, &p.cells);
+                if (!d.overflow && lane == 0) w = walk_back<true>(d, rows, qres, sub, M, N, p.a, p.b, mat);
+            } else {
+                p.score = xdrop_dp_dirs<false>(Q, S, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, Hb, Eb, &p.a, &p.b,
+                                               d, &rows, &p.cells);
+                if (!d.overflow && lane == 0) w = walk_back<false>(d, rows, Q, S, M, N, p.a, p.b, mat);
+            }
+            p.pairs = w.pairs;
+            p.identities = w.identities;
+            p.positives = w.positives;
+            p.gaps = w.gaps;
+            p.gap_opens = w.gap_opens;
+            p.last = w.last_move;
+            p.status = w.ok ? 0 : 2;
         }
+        if (d.overflow) p.status = 1;
         if (lane == 0) {
-            o.score = left + right;
-            o.q_start = q_off + 1 - al;
-            o.q_end = q_off + ar + 1;
-            o.s_start = s_off + 1 - bl;
-            o.s_end = s_off + br + 1;
-            o.identities = wl.identities + wr.identities;
-            o.positives = wl.positives + wr.positives;
-            o.gaps = wl.gaps + wr.gaps;
-            o.length = wl.pairs + wr.pairs + o.gaps;
-            o.mismatches = wl.pairs + wr.pairs - o.identities;
-            o.gap_opens = wl.gap_opens + wr.gap_opens - ((wl.last_move > 0 && wl.last_move == wr.last_move) ? 1 : 0);
-            o.status = d.overflow ? 1 : ((wl.ok && wr.ok) ? 0 : 2);
-            o.cells = cells;
-            a.out[t] = o;
+            a.part[t] = p;
+            __threadfence();  // the side before the count
+            if (atomicAdd(a.done + ti, 1u) == 1u) {  // the item's other side is done too
+                __threadfence();
+                const volatile int32_t *other = reinterpret_cast<const volatile int32_t *>(a.part + (t ^ 1ull));
+                TbPart o2;
+                for (int i = 0; i < static_cast<int>(sizeof(TbPart) / 4); ++i) reinterpret_cast<int32_t *>(&o2)[i] = other[i];
+                const TbPart &l = is_left ? p : o2, &r = is_left ? o2 : p;
+                TbOut o{};
+                o.score = l.score + r.score;
+                o.q_start = q_off + 1 - l.a;
+                o.q_end = q_off + r.a + 1;
+                o.s_start = s_off + 1 - l.b;
+                o.s_end = s_off + r.b + 1;
+                o.identities = l.identities + r.identities;
+                o.positives = l.positives + r.positives;
+                o.gaps = l.gaps + r.gaps;
+                o.length = l.pairs + r.pairs + o.gaps;
+                o.mismatches = l.pairs + r.pairs - o.identities;
+                // a gap across the start point is one
+                o.gap_opens = l.gap_opens + r.gap_opens - ((l.last > 0 && l.last == r.last) ? 1 : 0);
+                o.status = l.status == 1 || r.status == 1 ? 1 : max(l.status, r.status);
+                o.cells = l.cells + r.cells;
+                a.out[ti] = o;
+            }
         }
         __syncwarp();
     }

@@ -28,8 +28,8 @@ static int traceback_passes(blaze_search *s, const std::vector<TbItem> &items, c
     s->stats.traceback_cells = 0;
     std::vector<uint32_t> todo(n);
     for (size_t i = 0; i < n; ++i) todo[i] = static_cast<uint32_t>(i);
-    unsigned long long cap = s->tb_dir_cap;
-    const uint32_t row_cap = static_cast<uint32_t>(max_qlen) + 2u;
+    unsigned long long cap = (s->tb_dir_cap + 63) & ~63ull;  // rows of direction bytes begin at multiples of 64
+    const uint32_t row_cap = (static_cast<uint32_t>(max_qlen) + 3u) & ~1u;  // even: pairs of ints
     const uint32_t dp_stride = std::max<uint32_t>(db->max_len, 1u) + 2u;
     std::vector<TbItem> pass_items;
     std::vector<TbOut> pass_out;
@@ -37,8 +37,8 @@ static int traceback_passes(blaze_search *s, const std::vector<TbItem> &items, c
     for (int attempt = 0; !todo.empty(); ++attempt) {
         if (attempt > 12) return BLAZE_ERR_LIMIT;
         const size_t m = todo.size();
-        const int blocks = static_cast<int>(std::min<size_t>(static_cast<size_t>(s->n_sm) * 4,
-                                                             (m + kTracebackWarpsPerBlock - 1) / kTracebackWarpsPerBlock));
+        const int blocks = static_cast<int>(std::min<size_t>(static_cast<size_t>(s->n_sm) * kTracebackBlocksPerSm,
+                                                             (2 * m + kTracebackWarpsPerBlock - 1) / kTracebackWarpsPerBlock));
         const size_t warps = static_cast<size_t>(blocks) * kTracebackWarpsPerBlock;
         pass_items.resize(m);
         for (size_t k = 0; k < m; ++k) pass_items[k] = items[todo[k]];
@@ -47,6 +47,8 @@ static int traceback_passes(blaze_search *s, const std::vector<TbItem> &items, c
         if ((rc = s->tb_out.ensure(m)) != BLAZE_OK) return rc;
         if ((rc = s->tb_rows.ensure(warps * 3 * row_cap)) != BLAZE_OK) return rc;
         if ((rc = s->tb_dp.ensure(warps * 2 * dp_stride)) != BLAZE_OK) return rc;
+        if ((rc = s->tb_part.ensure(2 * m)) != BLAZE_OK) return rc;
+        if ((rc = s->tb_done.ensure(m)) != BLAZE_OK) return rc;
         if ((rc = s->tb_cursor.ensure(1)) != BLAZE_OK) return rc;
         if ((rc = s->tb_dirs.ensure(warps * cap)) != BLAZE_OK) return rc;
         BLAZE_CUDA_TRY(cudaMemcpyAsync(s->tb_items.p, pass_items.data(), sizeof(TbItem) * m, cudaMemcpyHostToDevice,
@@ -71,7 +73,10 @@ static int traceback_passes(blaze_search *s, const std::vector<TbItem> &items, c
         ta.dir_cap = cap;
         ta.rows = s->tb_rows.p;
         ta.row_cap = row_cap;
+        ta.part = s->tb_part.p;
+        ta.done = s->tb_done.p;
         ta.cursor = s->tb_cursor.p;
+        BLAZE_CUDA_TRY(cudaMemsetAsync(s->tb_done.p, 0, sizeof(unsigned int) * m, s->stream));
         BLAZE_CUDA_TRY(cudaMemsetAsync(s->tb_cursor.p, 0, sizeof(unsigned long long), s->stream));
         BLAZE_CUDA_TRY(cudaEventRecord(s->ev[1], s->stream));
         BLAZE_CUDA_TRY(launch_traceback(ta, blocks, s->stream));
