@@ -114,19 +114,25 @@ extern "C" int blaze_db_create(int device, const uint8_t *residues, const uint64
 
 int db_make_groups(blaze_db *db) {
     const std::vector<uint64_t> &off = db->h_off;
-    // at least 16 groups for each of the 152 x 32 warps of a scan, so that they
-    // end about together (256 queries against 35 M residues: 185.5 ms, and
-    // 189.6 with 4)
-    constexpr uint64_t kGroups = 16ull * 152 * 32;
-    const uint64_t most = std::min<uint64_t>(db->total / kGroups, kGroupMaxBytes);
-    db->group_bytes = static_cast<uint32_t>(most);
+    // A group holds twice a warp's share of the residues that are left (152 x 32
+    // warps), at most what a warp stages: what a group costs beyond its residues
+    // -- fetching it, its last partial batches and extensions -- is spread over
+    // more of them, and the last groups are small, so that the warps end about
+    // together. 300 query residues against 14 / 35 / 140 M: 0.183 / 0.329 / 1.013
+    // ms with 1/16 of a warp's share of all residues, 0.140 / 0.261 / 0.983 so.
+    constexpr uint64_t kWarps = 152 * 32, kLeast = 512;
+    const uint64_t least = std::min<uint64_t>(kLeast, db->total / kWarps);
+    db->group_bytes = 0;
     std::vector<uint32_t> &b = db->h_groups;
     b.assign(1, db->n);
     for (uint32_t hi = db->n; hi > 0;) {
+        const uint64_t most = std::min<uint64_t>(std::max<uint64_t>(2 * off[hi] / kWarps, least), kGroupMaxBytes);
         uint32_t lo = hi - 1;
         while (lo > 0 && hi - lo < kGroupMaxSubjects &&
                off[hi] - off[lo - 1] + kGroupSubjectBytes * (hi - lo + 1) <= most)
             --lo;
+        if (hi - lo > 1)
+            db->group_bytes = std::max(db->group_bytes, static_cast<uint32_t>(off[hi] - off[lo] + kGroupSubjectBytes * (hi - lo)));
         b.push_back(lo);
         hi = lo;
     }
@@ -134,7 +140,7 @@ int db_make_groups(blaze_db *db) {
     // residues (with what precedes it in its first 16 bytes), other groups are
     // one piece. (4,000 residues against 500 subjects: 0.21 ms with pieces of
     // 128, 0.35 of 512, 0.52 of 2,240.)
-    const uint64_t piece = std::min<uint64_t>(std::max<uint64_t>(db->total / (152 * 32), kPieceLeast), kPieceMost);
+    const uint64_t piece = std::min<uint64_t>(std::max<uint64_t>(db->total / kWarps, kPieceLeast), kPieceMost);
     std::vector<uint32_t> pieces(1, 0u);
     for (size_t g = 0; g + 1 < b.size(); ++g) {
         const uint64_t len = b[g] - b[g + 1] == 1 ? off[b[g]] - off[b[g + 1]] : 0;
@@ -749,9 +755,15 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
                                 : scan_max_warps_by_registers(scan_query_in_smem(r.q->qlen, p0->window));
     const int warp_cap = s->max_warps ? std::min(reg_cap, static_cast<int>(s->max_warps)) : reg_cap;
     // layout of one single-query scan launch
-    const uint32_t stage_bytes = std::max(s->stage_bytes, db->group_bytes);
+    const uint64_t share = db->total / (static_cast<uint64_t>(s->n_sm) * kScanMaxWarpsPerBlock);
     constexpr size_t kSmemMost = 227 * 1024 - 64;  // the opt-in limit less static shared memory
-    auto layout_for = [&](int32_t qlen, uint32_t n_hits, int warps, uint32_t band_entries = 0) {
+    auto layout_for = [&](int32_t qlen, uint32_t n_hits, int warps, bool queue, uint32_t band_entries = 0) {
+        // A warp stages a whole group, but a part of one next to a long query's
+        // table, where more warps on an SM are worth more (1,500 / 3,000 residues
+        // against 140 M: 3.79 -> 3.61 and 8.16 -> 7.81 ms) -- unless there is no
+        // more than a group for each warp (1,500 against 7 M: 0.35 -> 0.40)
+        const bool part = band_entries == 0 && qlen > kStageQuery && (queue || share > kGroupMaxBytes);
+        const uint32_t stage_bytes = part ? s->stage_bytes : std::max(s->stage_bytes, db->group_bytes);
         ScanLayout l = scan_layout(qlen, p0->window, n_hits, stage_bytes, kSmemBudget, warps, band_entries);
         // next to the longest tables only smaller groups are staged
         if (l.smem_bytes > kSmemMost)
@@ -764,7 +776,7 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     // when that fits the budget, else the whole budget (at least one warp);
     // the block runs as many warps as fit for each query
     auto batch_layout_for = [&](int32_t longest, bool word_table) {
-        ScanLayout l = layout_for(longest, UINT32_MAX, 1);
+        ScanLayout l = layout_for(longest, UINT32_MAX, 1, true);
         const size_t regions = l.smem_bytes - l.warp_smem_bytes + (word_table ? kScanWordTabBytes - kScanPresenceBytes : 0);
         l.word_table = word_table;
         l.warps_per_block = std::max(1, std::min(warp_cap, kScanMaxWarpsPerBlock));
@@ -782,8 +794,8 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
                          [&](uint32_t a, uint32_t b) { return r.b->qlen[a] < r.b->qlen[b]; });
     auto qlen_at = [&](uint32_t k) { return batched ? r.b->qlen[order[k]] : r.q->qlen; };
     std::vector<ScanPlan> plans;
-    auto query_layout = [&](uint32_t k, uint32_t band_entries = 0) {
-        return layout_for(qlen_at(k), batched ? r.b->n_off[order[k]] : r.q->n_off, warp_cap, band_entries);
+    auto query_layout = [&](uint32_t k, bool queue, uint32_t band_entries = 0) {
+        return layout_for(qlen_at(k), batched ? r.b->n_off[order[k]] : r.q->n_off, warp_cap, queue, band_entries);
     };
     // One query's launch runs in bands of diagonals
     // - where a subject is longer than a warp's share of the residues, so that
@@ -802,10 +814,9 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     // of 2,000 to 5,000 residues against 10.7 M residues with subjects of up to
     // 35,000 scan in 14.4 ms instead of 104.2. Otherwise one launch per query
     // is the faster (256 queries against 35 M residues 117.2 ms and 120.1).
-    const uint64_t share = db->total / (static_cast<uint64_t>(s->n_sm) * kScanMaxWarpsPerBlock);
     const bool per_query = batched && (s->batch_launch == 2 || (s->batch_launch == 0 && (nq == 1 || db->max_len < share)));
     const bool has_pieces = db->n_pieces + 1 > db->h_groups.size();
-    auto narrow_layout = [&](uint32_t k) { return query_layout(k, scan_band_entries(qlen_at(k))); };
+    auto narrow_layout = [&](uint32_t k) { return query_layout(k, false, scan_band_entries(qlen_at(k))); };
     auto is_narrow = [&](uint32_t k) {  // (a group's bands have to be staged as one)
         return qlen_at(k) > kBandQuery && p0->window <= kTab16Window && db->n > 0 &&
                narrow_layout(k).stage_bytes >= db->group_bytes;
@@ -814,14 +825,14 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     for (uint32_t i = 0; i < nq;) {
         uint32_t j = i + 1;
         ScanPlan pl;
-        pl.lay = query_layout(i);
         const bool narrow = is_narrow(i);
         pl.queue = batched && !per_query && (!narrow || s->batch_launch == 1);
+        pl.lay = query_layout(i, pl.queue);
         const bool banded = narrow || (has_pieces && db->max_len > share && p0->window <= kTab16Window);
         if (pl.queue) {
             const bool smem = pl.lay.query_smem_bytes != 0, table = pl.lay.word_table;
             for (; j < nq; ++j) {
-                const ScanLayout l = query_layout(j);
+                const ScanLayout l = query_layout(j, true);
                 if ((l.query_smem_bytes != 0) != smem || l.word_table != table || is_narrow(j) != narrow) break;
             }
             pl.lay = batch_layout_for(qlen_at(j - 1), table);

@@ -48,6 +48,7 @@ constexpr uint32_t kBandEntries16 = 3360, kBandEntries32 = 2240;
 static_assert(kBandEntries32 >= kGroupMaxBytes && kBandEntries16 >= kGroupMaxBytes, "a group is one piece");
 constexpr uint32_t kPieceLeast = 128, kPieceMost = kGroupMaxBytes;  // residues of a long subject's piece
 constexpr int32_t kBandQuery = 7000;         // longer queries take such tables
+constexpr int32_t kStageQuery = 1300;        // longer ones stage parts of a group
 constexpr uint32_t kScanStageBytes = 1024;   // subjects up to this length are staged
 
 inline bool scan_query_in_smem(int32_t qlen, int32_t window, bool bands = false) {

@@ -833,9 +833,9 @@ struct Group {
     bool staged;
 };
 
-// Takes the subjects [lo, hi) of a group -- or only the first, when they do
-// not fit the stage buffer or `staging` is off -- and starts their copies to
-// the stage buffer, each lane its subject's.
+// Takes the subjects [lo, hi) of a group, or as many as fit the stage buffer,
+// and starts their copies there, each lane its subject's; the first one stays in
+// global memory when not even it fits or `staging` is off.
 __device__ __forceinline__ Group fetch_group(Finder &f, const ScanArgs &a, const Ctx &c, uint32_t lo, uint32_t hi,
                                              bool staging) {
     const uint32_t lane = threadIdx.x & 31;
@@ -850,16 +850,11 @@ __device__ __forceinline__ Group fetch_group(Finder &f, const ScanArgs &a, const
     // a subject's block: what precedes it in its first 16 bytes, it, two zeros
     const uint32_t block = lane < f.ns ? (lead + len + 2u + 15u) & ~15u : 0u;
     const uint32_t to = warp_prefix(block);
-    auto fits = [&](uint32_t n) {
-        const uint32_t need = __shfl_sync(kFull, to, n - 1u);
-        return staging && need <= scan_stage_blocks(a.stage_bytes) &&
-               (n == 1u || need + static_cast<uint32_t>(c.window) * n <= kPackSpan - kChunk);
-    };
-    r.staged = fits(f.ns);
-    if (!r.staged && f.ns > 1) {
-        f.ns = 1;
-        r.staged = fits(1);
-    }
+    const bool fits = lane < f.ns && staging && to <= scan_stage_blocks(a.stage_bytes) &&
+                      (lane == 0u || to + static_cast<uint32_t>(c.window) * (lane + 1u) <= kPackSpan - kChunk);
+    const uint32_t n = __popc(__ballot_sync(kFull, fits));  // the first n subjects do
+    r.staged = n > 0u;
+    f.ns = max(n, 1u);
     const bool has = lane < f.ns;
     if (!has) len = 0u;
     f.first = has ? (r.staged ? to - block + lead : 0u) : 0x7fffffffu;
