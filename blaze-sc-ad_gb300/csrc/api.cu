@@ -811,9 +811,10 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     // A batch runs as one launch whose blocks go from query to query where a
     // query's own pass would end in a wait for its longest subjects, that is
     // where one of them is more than a warp's share of the residues: 16 queries
-    // of 2,000 to 5,000 residues against 10.7 M residues with subjects of up to
-    // 35,000 scan in 14.4 ms instead of 104.2. Otherwise one launch per query
-    // is the faster (256 queries against 35 M residues 117.2 ms and 120.1).
+    // of 2,000 to 5,000 residues against 10.5 M residues with subjects of up to
+    // 35,000 scan in 13.1 ms, with a banded launch each in 15.4. Otherwise one
+    // launch per query is the faster (256 queries against 35 M residues 100.9 ms
+    // and 103.9).
     const bool per_query = batched && (s->batch_launch == 2 || (s->batch_launch == 0 && (nq == 1 || db->max_len < share)));
     const bool has_pieces = db->n_pieces + 1 > db->h_groups.size();
     auto narrow_layout = [&](uint32_t k) { return query_layout(k, false, scan_band_entries(qlen_at(k))); };

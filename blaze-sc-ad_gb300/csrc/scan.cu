@@ -1,14 +1,14 @@
 // scan.cu -- word finder, two-hit seeding and ungapped X-drop extension of
 // the BLASTP preliminary search on GB300 (sm_103a). Integer work only.
 //
-// One warp per group of subjects; persistent warps pull groups, longest
-// subjects first, from a device cursor (batched: blocks pull (query, group
-// range) tiles, their warps the tile's groups). Per block in shared memory: the BLOSUM62 matrix
-// (int8), the query's word-presence bitset and, for queries up to
-// kQuerySmemMax, the query residues. Per warp: the diagonal table, the deferred-hit and seed
-// queues and a staging buffer that holds the whole group when it fits, so
-// the word scan and the extensions read shared memory instead of making
-// dependent global loads.
+// One warp per group of subjects (or band of its diagonals); persistent warps
+// pull groups, longest subjects first, from a device cursor (batched: one per
+// query, and blocks go from query to query). Per block in shared memory: the
+// BLOSUM62 matrix, the query's word table or word-presence bitset and, for
+// queries up to kQuerySmemMax, the query residues. Per warp: the diagonal table,
+// the deferred-hit and seed queues, the list of a chunk's words with hits and a
+// staging buffer for the group, so the word scan and the extensions read shared
+// memory instead of making dependent global loads.
 //
 // Reference counterpart: gpuBLAZE_full (BLAZE_gpu/gpuBLAZE.cu:885-1252), which
 // is a filter; this kernel produces the exact ungapped HSPs of the
@@ -344,7 +344,7 @@ struct Finder {
 };
 
 // Per-query parameters of the word finder (one query, or the query of the
-// current tile in a batch).
+// batch at hand).
 struct Ctx {
     int32_t qlen;
     const uint32_t *cell_start, *cell_pack;
@@ -426,7 +426,7 @@ __device__ __forceinline__ uint32_t claim(uint32_t entry, uint32_t here, bool ac
 // Behind a second hit that starts over as well (rare: it is `window` or more
 // from the first) the rest is brought again: true is returned for them.
 //
-// The kernel is bound by instruction issue (82 % at 300 query residues), and
+// The kernel is bound by instruction issue (85 % at 300 query residues), and
 // this function was nearly half of it. __match_any_sync in place of the claims
 // costs few instructions, but 8.4 cycles per distinct value: 270 for a batch of
 // 32 diagonals. With the claims and full batches: 139 M residues at 300 / 1,000
@@ -1126,8 +1126,8 @@ scan_kernel(const ScanArgs a) {
 // the next query that has any. Blocks start at queries spread over the launch
 // and meet at the last ones, so only the launch has an end at which warps wait
 // for its longest subjects, not each query's pass: 16 queries of 2,000 to 5,000
-// residues against 10.7 M residues with subjects of up to 35,000 take 14.4 ms in
-// one launch and 104.2 in a launch each. The block lays its warps' regions out
+// residues against 10.5 M residues with subjects of up to 35,000 take 13.1 ms in
+// one launch, and in a launch each 112, or 15.4 in bands. The block lays its warps' regions out
 // for each query: a warp's diagonal table takes the query's length plus the
 // window, so as many warps as fit (at most the block's) work on it.
 template <bool QS, bool WT>
