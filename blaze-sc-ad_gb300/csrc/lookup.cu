@@ -2,16 +2,18 @@
 // 28^3 words, the query offsets whose word scores at least the threshold
 // against it, or equals it (BLAZE_ncbi/prelim_stage.cpp:135-155, :378-386).
 //
-// A block takes the 28 words that begin with one pair of letters, its warps a
-// part of the query each, a lane per offset: where the pair's score leaves a
+// A warp takes the 28 words that begin with one pair of letters and walks the
+// query or a part of it, a lane per offset: where the pair's score leaves a
 // third letter that can reach the threshold the offset is a candidate (about one
 // in twenty at the default), and full batches of candidates are tested against
 // the 28 letters, a ballot each. So a word's offsets come out ascending and no
 // neighbourhood lists are needed. One pass counts, a block per query turns the
 // counts into the tables, a second pass writes the offsets.
-// The passes are bound by the latency of their steps, 32 offsets each: 8 and 13
-// us at 300 query residues, 31 and 65 at 12,345, where a thread per word that
-// walked the query alone took 0.5 ms a pass.
+// One query's passes are bound by the latency of their steps, 32 offsets each: 8
+// and 13 us at 300 query residues, 32 and 65 at 12,345, where a thread per word
+// that walked the query alone took 0.5 ms a pass; many queries' by issue: 256 of
+// 50 to 2,000 residues 0.62 and 1.18 ms (0.86 and 1.74 with a block and eight
+// parts for every pair and query).
 #include <algorithm>
 #include <cstdint>
 
@@ -25,10 +27,29 @@ __device__ const int32_t g_blosum_lk[kAlphabet * kAlphabet] = {
 };
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kLookupWarps = 8;                // per block, each with a part of the query
-constexpr int kPairs = kAlphabet * kAlphabet;  // pairs of letters, a block each
+constexpr int kLookupWarps = 8;                // per block: pairs of letters times parts of the query
+constexpr int kPartLeast = 256;                // offsets of a part: a test of the 28 letters costs the same for
+                                               // one candidate and 32, so parts are not cut smaller
+constexpr int kPairs = kAlphabet * kAlphabet;  // pairs of letters
 constexpr int kRow = kAlphabet + 1;            // of the matrix in shared memory: an odd stride, so that the
                                                // lanes' rows lie in different banks
+
+static_assert(kPairs % kLookupWarps == 0);
+
+// A block's work on a query with `all` offsets: the parts that the query is cut
+// in, a warp each, and so how many pairs the block takes.
+struct Split {
+    int32_t all, parts, part;
+    uint32_t pairs;
+    __device__ __forceinline__ explicit Split(int32_t qlen) : all(max(qlen - (kWordSize - 1), 0)), parts(1) {
+        while (parts < kLookupWarps && all > parts * kPartLeast) parts *= 2;
+        part = ((all + parts - 1) / parts + 31) & ~31;
+        pairs = kLookupWarps / parts;
+    }
+    __device__ __forceinline__ bool idle() const { return blockIdx.x * pairs >= kPairs; }
+    __device__ __forceinline__ uint32_t pair() const { return blockIdx.x * pairs + (threadIdx.x >> 5) / parts; }
+    __device__ __forceinline__ uint32_t mine() const { return (threadIdx.x >> 5) % parts; }  // the warp's part
+};
 
 struct WalkShared {
     int32_t mat[kAlphabet * kRow];
@@ -54,15 +75,13 @@ __device__ __forceinline__ void walk_setup(WalkShared &sh) {
 // and batch of candidates: the lanes in mask have the word's offset i. Every
 // lane makes every call.
 template <typename F>
-__device__ __forceinline__ void walk_query(WalkShared &sh, const LookupQuery &lq, int32_t threshold, F hit) {
+__device__ __forceinline__ void walk_query(WalkShared &sh, const LookupQuery &lq, const Split &sp, int32_t threshold, F hit) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t a = blockIdx.x / kAlphabet, b = blockIdx.x % kAlphabet;
+    const uint32_t a = sp.pair() / kAlphabet, b = sp.pair() % kAlphabet;
     const int32_t *mat = sh.mat;
     uint32_t *cand = sh.cand[warp];
     int32_t *cand_score = sh.cand_score[warp];
-    const int32_t all = max(lq.qlen - (kWordSize - 1), 0);
-    const int32_t part = ((all + kLookupWarps - 1) / kLookupWarps + 31) & ~31;
-    const int32_t from = min(part * static_cast<int32_t>(warp), all), n = min(from + part, all);
+    const int32_t from = min(sp.part * static_cast<int32_t>(sp.mine()), sp.all), n = min(from + sp.part, sp.all);
     uint32_t have = 0;
     auto test = [&](uint32_t m) {  // the first m candidates
         const bool in = lane < m;
@@ -112,11 +131,11 @@ __device__ __forceinline__ void walk_query(WalkShared &sh, const LookupQuery &lq
     if (have) test(have);
 }
 
-// The warp's counts, by third letter.
-__device__ __forceinline__ void walk_count(WalkShared &sh, const LookupQuery &lq, int32_t threshold) {
+// The warps' counts, by third letter.
+__device__ __forceinline__ void walk_count(WalkShared &sh, const LookupQuery &lq, const Split &sp, int32_t threshold) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t n = 0;  // lane c: of the word with third letter c
-    walk_query(sh, lq, threshold, [&](uint32_t c, uint32_t mask, uint32_t) { n += lane == c ? __popc(mask) : 0; });
+    walk_query(sh, lq, sp, threshold, [&](uint32_t c, uint32_t mask, uint32_t) { n += lane == c ? __popc(mask) : 0; });
     sh.count[threadIdx.x >> 5][lane] = n;
     __syncthreads();
 }
@@ -126,12 +145,15 @@ __global__ void __launch_bounds__(kLookupWarps * 32)
 lookup_count_kernel(const LookupQuery one, const LookupQuery *many, int32_t threshold) {
     __shared__ WalkShared sh;
     const LookupQuery lq = many ? many[blockIdx.y] : one;
+    const Split sp(lq.qlen);
+    if (sp.idle()) return;
     walk_setup(sh);
-    walk_count(sh, lq, threshold);
-    if (threadIdx.x < kAlphabet) {
+    walk_count(sh, lq, sp, threshold);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (sp.mine() == 0u && lane < kAlphabet) {
         uint32_t n = 0;
-        for (int w = 0; w < kLookupWarps; ++w) n += sh.count[w][threadIdx.x];
-        lq.cell_start[blockIdx.x * kAlphabet + threadIdx.x] = n;
+        for (int p = 0; p < sp.parts; ++p) n += sh.count[warp + p][lane];
+        lq.cell_start[sp.pair() * kAlphabet + lane] = n;
     }
 }
 
@@ -176,20 +198,23 @@ __global__ void __launch_bounds__(1024) lookup_tables_kernel(const LookupQuery o
     }
 }
 
-// The offsets; a warp counts its part first, for where the next one's begin.
+// The offsets; where there are several parts a warp counts its own first, for
+// where the next one's begin.
 __global__ void __launch_bounds__(kLookupWarps * 32)
 lookup_write_kernel(const LookupQuery one, const LookupQuery *many, int32_t threshold) {
     __shared__ WalkShared sh;
     const LookupQuery lq = many ? many[blockIdx.y] : one;
+    const Split sp(lq.qlen);
+    if (sp.idle()) return;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     walk_setup(sh);
-    walk_count(sh, lq, threshold);
+    if (sp.parts > 1) walk_count(sh, lq, sp, threshold);
     uint32_t to = 0;  // lane c: where the next offset of its word goes
     if (lane < kAlphabet) {
-        to = lq.cell_start[blockIdx.x * kAlphabet + lane];
-        for (uint32_t w = 0; w < warp; ++w) to += sh.count[w][lane];
+        to = lq.cell_start[sp.pair() * kAlphabet + lane];
+        for (uint32_t w = warp - sp.mine(); w < warp; ++w) to += sh.count[w][lane];
     }
-    walk_query(sh, lq, threshold, [&](uint32_t c, uint32_t mask, uint32_t i) {
+    walk_query(sh, lq, sp, threshold, [&](uint32_t c, uint32_t mask, uint32_t i) {
         const uint32_t at = __shfl_sync(kFull, to, c) + __popc(mask & ((1u << lane) - 1u));
         if ((mask >> lane) & 1u) lq.cell_off[at] = static_cast<uint16_t>(i);
         to += lane == c ? __popc(mask) : 0;

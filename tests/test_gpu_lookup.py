@@ -12,7 +12,7 @@ from _parity import HSP_FIELDS, compare, concat, params_for
 
 pytestmark = pytest.mark.gpu
 
-LENGTHS = [1, 2, 3, 4, 511, 512, 513, 514, 515, 1026, 1027]
+LENGTHS = [1, 2, 3, 4, 257, 258, 259, 511, 512, 513, 514, 515, 1026, 1027]
 
 
 @pytest.mark.parametrize("qlens,threshold", [(LENGTHS, 11), (LENGTHS, 40), ([32_000], 11), ([300, 2000], 0),
