@@ -1,10 +1,11 @@
 // host.cpp -- host-side pieces of libblaze103 that need no GPU: the BLOSUM62
-// table, the query word lookup and the NCBI-default search parameters.
+// table, the size of a query's word lookup and the NCBI-default search parameters.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -21,15 +22,18 @@ namespace {
 // Size of every three-letter word's neighbourhood for one threshold: the words
 // v with score(w, v) >= threshold, and w itself (BLAZE_ncbi/
 // prelim_stage.cpp:135-155 enumerates the same set; :378-383 keeps the exact
-// word). Computed once per threshold and cached.
+// word). Computed once per threshold and kept (44 KB) for a few of them.
 std::mutex g_nb_mutex;
-std::map<int32_t, std::vector<uint16_t>> g_nb_cache;
+using NeighbourhoodSizes = std::shared_ptr<const std::vector<uint16_t>>;
+std::map<int32_t, NeighbourhoodSizes> g_nb_cache;
+constexpr size_t kNbCacheMost = 32;
 
-const std::vector<uint16_t> &neighbourhood_sizes(int32_t threshold) {
+NeighbourhoodSizes neighbourhood_sizes(int32_t threshold) {
     std::lock_guard<std::mutex> lock(g_nb_mutex);
     auto it = g_nb_cache.find(threshold);
     if (it != g_nb_cache.end()) return it->second;
-    std::vector<uint16_t> size(kWords);
+    auto sizes = std::make_shared<std::vector<uint16_t>>(kWords);
+    std::vector<uint16_t> &size = *sizes;
     int32_t row_max[kAlphabet];
     for (int a = 0; a < kAlphabet; ++a)
         row_max[a] = *std::max_element(kBlosum62[a], kBlosum62[a] + kAlphabet);
@@ -47,13 +51,15 @@ const std::vector<uint16_t> &neighbourhood_sizes(int32_t threshold) {
         }
         size[w] = static_cast<uint16_t>(n);  // at most 21,952
     }
-    return g_nb_cache.emplace(threshold, std::move(size)).first->second;
+    if (g_nb_cache.size() >= kNbCacheMost) g_nb_cache.clear();
+    return g_nb_cache.emplace(threshold, std::move(sizes)).first->second;
 }
 
 }  // namespace
 
 uint32_t lookup_hits(const uint8_t *query, int32_t qlen, int32_t threshold) {
-    const std::vector<uint16_t> &size = neighbourhood_sizes(threshold);
+    const NeighbourhoodSizes sizes = neighbourhood_sizes(threshold);
+    const std::vector<uint16_t> &size = *sizes;
     uint32_t n = 0;
     for (int32_t i = 0; i + kWordSize <= qlen; ++i) n += size[query[i] * 784 + query[i + 1] * 28 + query[i + 2]];
     return n;

@@ -112,7 +112,7 @@ typedef struct blaze_stats {
     float gapped_ms; /* gapped kernel */
     float device_ms; /* first to last device operation of the run, all passes */
     uint32_t kernel_launches; /* kernels launched by the run, all passes */
-    uint64_t h2d_bytes; /* host->device bytes of the run (query tables included) */
+    uint64_t h2d_bytes; /* host->device bytes of the run (the query's residues included) */
     uint64_t d2h_bytes; /* device->host bytes of the run */
     uint32_t graph_replays; /* passes launched from an already built CUDA graph */
     uint32_t graph_builds;  /* passes that captured (or updated) the CUDA graph */
