@@ -1096,7 +1096,8 @@ __device__ __forceinline__ void finish_item(const GappedArgs &a, const Item &it,
 }
 
 // Whether the task's init hit lies inside the HSP of its item's best one, as
-// far as that is known by now: the finishing kernel then skips it.
+// far as that is known by now: the finishing warp then skips it. Other warps
+// write what it reads, so two lanes may get different answers.
 __device__ __forceinline__ bool inside_first(const GappedArgs &a, unsigned long long slot, const DpTask &k) {
     if (k.rank == 0) return false;
     const unsigned long long f = slot - static_cast<unsigned long long>(k.rank);
@@ -1149,7 +1150,9 @@ gapped_warp_dp_kernel(const GappedArgs a) {
             if (k.valid && lane == 0) atomicOr(&a.cnt->flags, kFlagBadState);
             continue;
         }
-        if (!inside_first(a, slot, k)) {
+        // one lane looks: the best one's DPs may be ending, and the warp goes one way
+        const bool skip = lane == 0 && inside_first(a, slot, k);
+        if (!__shfl_sync(kFull, skip, 0)) {
             const int4 r = warp_dp(a, q, qlen, a.res + k.s_base, k.slen, k.q_off, k.s_off, left, mat, Hb, Eb);
             if (lane == 0) {
                 volatile int32_t *o = reinterpret_cast<volatile int32_t *>(a.dres + 2 * slot + (left ? 0 : 1));
