@@ -750,13 +750,24 @@ gapped_kernel(const GappedArgs a) {
 // Every DP is independent of the others (containment only decides which
 // results are used), so the results are exactly those of gapped_kernel.
 
+// A number read by one thread for its block: other blocks may set a flag
+// meanwhile, and the number decides which warps go on and meet at the block's
+// barriers, so all of its threads hold the same. A barrier for the block.
+template <typename F>
+__device__ __forceinline__ unsigned long long block_number(F read) {
+    __shared__ unsigned long long n;
+    if (threadIdx.x == 0) n = read();
+    __syncthreads();
+    return n;
+}
+
 __global__ void __launch_bounds__(kGappedWarpsPerBlock * 32)
 gapped_prep_kernel(const GappedArgs a) {
     __shared__ int32_t mat[kAlphabet * kAlphabet];
     load_matrix(mat);
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const unsigned long long n_work = work_items(a);
+    const unsigned long long n_work = block_number([&] { return work_items(a); });
     for (;;) {
         unsigned long long t = 0;
         if (lane == 0) t = atomicAdd(&a.cnt->next_prep, 1ull);
@@ -1000,7 +1011,7 @@ __global__ void __launch_bounds__(kDpWarpsPerBlock * 32)
 gapped_dp_kernel(const GappedArgs a) {
     __shared__ int32_t mat[kAlphabet * kAlphabet];
     extern __shared__ __align__(16) uint32_t dp_smem[];
-    const unsigned long long slots = dp_slots(a), n = 2ull * slots;
+    const unsigned long long slots = block_number([&] { return dp_slots(a); }), n = 2ull * slots;
     if (slots < a.lane_slots) return;  // gapped_warp_dp_kernel takes the pass
     load_matrix(mat);
     __syncthreads();
@@ -1122,7 +1133,7 @@ __device__ __forceinline__ bool inside_first(const GappedArgs &a, unsigned long 
 __global__ void __launch_bounds__(kGappedWarpsPerBlock * 32)
 gapped_warp_dp_kernel(const GappedArgs a) {
     __shared__ int32_t mat[kAlphabet * kAlphabet];
-    const unsigned long long slots = dp_slots(a);
+    const unsigned long long slots = block_number([&] { return dp_slots(a); });
     if (slots >= a.lane_slots) return;
     load_matrix(mat);
     __syncthreads();
@@ -1185,7 +1196,7 @@ gapped_warp_dp_kernel(const GappedArgs a) {
 __global__ void __launch_bounds__(kGappedWarpsPerBlock * 32)
 gapped_finish_kernel(const GappedArgs a) {
     __shared__ int32_t mat[kAlphabet * kAlphabet];
-    if (dp_slots(a) < a.lane_slots) return;  // gapped_warp_dp_kernel finished the items
+    if (block_number([&] { return dp_slots(a); }) < a.lane_slots) return;  // gapped_warp_dp_kernel finished the items
     load_matrix(mat);
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -1193,7 +1204,7 @@ gapped_finish_kernel(const GappedArgs a) {
     DevHsp *saved = a.saved + gwarp * a.cap;
     int32_t *Hb = a.dp + gwarp * 2ull * a.dp_stride;
     int32_t *Eb = Hb + a.dp_stride;
-    const unsigned long long n_work = work_items(a);
+    const unsigned long long n_work = block_number([&] { return work_items(a); });
     unsigned long long cells = 0, n_ext = 0;
     for (;;) {
         unsigned long long t = 0;
