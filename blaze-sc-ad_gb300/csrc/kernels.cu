@@ -581,13 +581,8 @@ gapped_kernel(const GappedArgs a) {
     DevHsp *saved = a.saved + gwarp * a.cap;
     int32_t *Hb = a.dp + gwarp * 2ull * a.dp_stride;
     int32_t *Eb = Hb + a.dp_stride;
-    unsigned long long n_work = *reinterpret_cast<volatile unsigned long long *>(&a.cnt->work_count);
-    if (n_work > a.work_cap) n_work = a.work_cap;
-    // A scan that overflowed its init-hit or work array counted items it
-    // could not write; the host repeats that pass with larger arrays, so this
-    // one takes no work at all (an unwritten slot holds no valid item).
-    const unsigned scan_flags = *reinterpret_cast<volatile unsigned *>(&a.cnt->flags);
-    if (scan_flags & (kFlagInitArrayFull | kFlagWorkArrayFull | kFlagBadState)) n_work = 0;
+    // no flag stops it: they are this launch's own (a skipped item's), not a scan's
+    const unsigned long long n_work = min(a.cnt->work_count, a.work_cap);
     unsigned long long cells = 0, n_ext = 0;
     for (;;) {
         unsigned long long t = 0;
