@@ -1177,6 +1177,7 @@ gapped_warp_dp_kernel(const GappedArgs a) {
             __threadfence();
         }
         if (__shfl_sync(kFull, rest, 0) == 1u) {
+            __syncwarp();  // lane 0's fence holds for every lane's reads from here on (a shuffle orders none)
             Item it;
             if (read_item(a, k.item, it, lane)) finish_item(a, it, saved, Hb, Eb, mat, cells, n_ext);
         }

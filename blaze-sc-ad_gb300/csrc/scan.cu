@@ -957,6 +957,7 @@ __device__ __forceinline__ bool merge_bands(Finder &f, const ScanArgs &a, uint32
     }
     done = __shfl_sync(kFull, done, 0);
     if (done != n_bands) return false;
+    __syncwarp();  // lane 0's fence holds for every lane's reads from here on (a shuffle orders none)
     uint32_t n = 0;
     const InitHit *frag = a.fragments;
     for (uint32_t next = __ldcg(&st->head); next != 0u;) {
