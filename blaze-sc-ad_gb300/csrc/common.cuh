@@ -51,6 +51,19 @@ constexpr int32_t kBandQuery = 7000;         // longer queries take such tables
 constexpr int32_t kStageQuery = 1300;        // longer ones stage parts of a group
 constexpr uint32_t kScanStageBytes = 1024;   // subjects up to this length are staged
 
+// Whether the register-window DPs of `rows` rows (gapped stage, traceback) stay
+// inside int32 and below -inf's distance. They compute the columns behind the
+// band as well, up to a window of them: those hold -inf, which an X-drop of 2^30
+// would call live, and enter the row gap's prefix maximum as -inf plus gap_extend
+// times their column. A band's last column is at most rows + (11 rows + xdrop) /
+// gap_extend + 2 (11: the matrix's largest score). Other DPs take the form with
+// their rows in memory.
+__device__ __forceinline__ bool dp_window_exact(int32_t rows, int32_t gap_open, int32_t gap_extend, int32_t xdrop) {
+    constexpr long long kBehind = 256;
+    const long long ge = gap_extend, goe = ge + gap_open, drop = xdrop > goe ? xdrop : goe;
+    return ge * (rows + kBehind) + 2 * drop + 22ll * rows <= -static_cast<long long>(kNeg);
+}
+
 inline bool scan_query_in_smem(int32_t qlen, int32_t window, bool bands = false) {
     return qlen <= (bands ? kBandQuerySmemMax : kQuerySmemMax) && window <= kTab16Window;
 }

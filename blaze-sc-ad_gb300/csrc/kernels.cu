@@ -1045,15 +1045,16 @@ gapped_dp_kernel(const GappedArgs a) {
 }
 
 // The left or right DP from a gapped start point by the whole warp: the band
-// in registers, or in the warp's DP rows when it outgrows them (best, row,
-// column, cells).
+// in registers, or in the warp's DP rows when it outgrows them or the gap costs
+// or the X-drop are too large for them (best, row, column, cells).
 __device__ __forceinline__ int4 warp_dp(const GappedArgs &a, const uint8_t *q, int32_t qlen, const uint8_t *s,
                                         int32_t slen, int32_t q_off, int32_t s_off, bool left, const int32_t *mat,
                                         int32_t *Hb, int32_t *Eb) {
     int4 r;
     const uint8_t *Q = q + q_off + (left ? 1 : 0), *S = s + s_off + (left ? 1 : 0);
     const int32_t M = left ? q_off + 1 : qlen - q_off - 1, N = left ? s_off + 1 : slen - s_off - 1;
-    if (!xdrop_dp_window(Q, S, left ? -1 : 1, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, &r.x, &r.y, &r.z, &r.w)) {
+    if (!dp_window_exact(M, a.gap_open, a.gap_extend, a.xdrop) ||
+        !xdrop_dp_window(Q, S, left ? -1 : 1, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, &r.x, &r.y, &r.z, &r.w)) {
         unsigned long long cells = 0;
         r.x = left ? xdrop_dp<true>(q, s, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, Hb, Eb, &r.y, &r.z, &cells)
                    : xdrop_dp<false>(Q, S, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, Hb, Eb, &r.y, &r.z, &cells);

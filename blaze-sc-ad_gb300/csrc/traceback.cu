@@ -8,8 +8,9 @@
 // One warp per side of an HSP. The X-drop DP runs row by row with its band in
 // registers, as in the gapped stage; every row's direction bytes go to the
 // warp's buffer. The warp then walks the path back from the best cell, 32 cells
-// of a diagonal at a time. Where the band outgrows the registers the rows are
-// kept in memory and one lane walks.
+// of a diagonal at a time. Where the band outgrows the registers, or the gap
+// costs or the X-drop are too large for them, the rows are kept in memory and
+// one lane walks.
 #include <cstdint>
 
 #include "common.cuh"
@@ -539,7 +540,8 @@ traceback_kernel(const TracebackArgs a) {
         d.overflow = false;
         TbPart p{};
         p.last = -1;
-        if (xdrop_dp_window_dirs(Q, S, dir, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, d, p)) {
+        if (dp_window_exact(M, a.gap_open, a.gap_extend, a.xdrop) &&
+            xdrop_dp_window_dirs(Q, S, dir, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, d, p)) {
             if (!d.overflow) walk_window(d, Q, S, dir, mat, p);
         } else {
             __syncwarp();
