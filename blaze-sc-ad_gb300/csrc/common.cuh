@@ -172,7 +172,8 @@ struct BatchQuery {
 
 // A query's word lookup on the device: where its residues are and its tables
 // go (cell_start: kWords + 1 prefix offsets; cell_pack: start << 8 | min(count,
-// 255), 255 sends the kernel to cell_start; presence: kPresenceWords; cell_off:
+// 255), a count of 255 sends the kernel to cell_start for both, and stands for
+// every cell whose start is 2^24 or more; presence: kPresenceWords; cell_off:
 // lookup_hits query offsets).
 struct LookupQuery {
     const uint8_t *q;
@@ -198,7 +199,7 @@ struct ScanArgs {
     const uint8_t *q;          // query residues
     int32_t qlen;
     const uint32_t *cell_start;  // kWords + 1
-    const uint32_t *cell_pack;   // kWords: start << 8 | min(count, 255)
+    const uint32_t *cell_pack;   // kWords: as LookupQuery
     const uint32_t *presence;    // kPresenceWords: bit w set when word w has hits
     const uint16_t *cell_off;    // query offsets per cell, ascending
     int32_t window, xdrop, cutoff;

@@ -157,7 +157,8 @@ lookup_count_kernel(const LookupQuery one, const LookupQuery *many, int32_t thre
     }
 }
 
-// One block per query: starts, packed cells (start << 8 | min(count, 255)) and
+// One block per query: starts, packed cells (start << 8 | min(count, 255), or 255
+// where the start takes more than 24 bits: 4,900 residues at word threshold 0) and
 // the presence bitset from the counts. A warp takes 22 rows of 32 consecutive
 // words, so every access is coalesced and a row's presence is a ballot (a run
 // of words per thread instead took 38 us for one query).
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(1024) lookup_tables_kernel(const LookupQuery o
         const uint32_t bits = __ballot_sync(0xffffffffu, n[k] != 0u);
         if (w < kWords) {
             lq.cell_start[w] = at;
-            lq.cell_pack[w] = (at << 8) | min(n[k], 255u);
+            lq.cell_pack[w] = at < (1u << 24) ? (at << 8) | min(n[k], 255u) : 255u;
         }
         if (lane == 0u && w / 32u < kPresenceWords) lq.presence[w / 32u] = bits;
         start += __shfl_sync(0xffffffffu, incl, 31);

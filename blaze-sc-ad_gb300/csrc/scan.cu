@@ -700,7 +700,10 @@ __device__ __forceinline__ void scan_span(Finder &f, const ScanArgs &a, const Ct
                 const uint32_t pk = present ? __ldg(c.cell_pack + w) : 0u;
                 cs[j] = pk >> 8;
                 cnt[j] = pk & 0xffu;
-                if (cnt[j] == 0xffu) cnt[j] = __ldg(c.cell_start + w + 1) - cs[j];
+                if (cnt[j] == 0xffu) {  // the count or the start does not fit the packed cell
+                    cs[j] = __ldg(c.cell_start + w);
+                    cnt[j] = __ldg(c.cell_start + w + 1) - cs[j];
+                }
             }
         }
         if (BANDS && !band.all) clip_cells(c, band, v0, cs, cnt);
