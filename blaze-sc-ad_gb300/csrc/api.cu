@@ -376,7 +376,7 @@ struct ScanLaunch {
     int blocks, warps_per_block;
     size_t smem_bytes;
     bool queue;  // the batched kernel, else the single-query one
-    bool word_table;
+    Words words;
 };
 
 struct PassLaunch {
@@ -399,8 +399,8 @@ static cudaError_t enqueue_pass(blaze_search *s, const PassLaunch &pl, unsigned 
         if (e == cudaSuccess && l.sa.pieces)
             e = cudaMemsetAsync(s->band_state.p, 0, sizeof(BandState) * l.sa.n_groups, s->stream);
         if (e != cudaSuccess) break;
-        e = l.queue ? launch_scan_batch(l.sa, l.word_table, l.blocks, l.warps_per_block, l.smem_bytes, s->stream)
-                       : launch_scan(l.sa, l.word_table, l.blocks, l.warps_per_block, l.smem_bytes, s->stream);
+        e = l.queue ? launch_scan_batch(l.sa, l.words, l.blocks, l.warps_per_block, l.smem_bytes, s->stream)
+                       : launch_scan(l.sa, l.words, l.blocks, l.warps_per_block, l.smem_bytes, s->stream);
     }
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(s->ev[2], s->stream, event_flags);
     if (e == cudaSuccess) e = launch_gapped_split(*pl.ga, s->gapped_blocks, s->n_sm, s->stream);
@@ -432,7 +432,8 @@ static int launch_pass_graph(blaze_search *s, const PassLaunch &pl) {
     put(head, sizeof(head));
     for (const ScanLaunch &l : pl.scans) {
         put(&l.sa, sizeof(ScanArgs));
-        const int64_t shape[4] = {l.blocks, l.warps_per_block, static_cast<int64_t>(l.smem_bytes), l.word_table};
+        const int64_t shape[4] = {l.blocks, l.warps_per_block, static_cast<int64_t>(l.smem_bytes),
+                                  static_cast<int64_t>(l.words)};
         put(shape, sizeof(shape));
     }
     put(pl.ga, sizeof(GappedArgs));
@@ -529,7 +530,7 @@ static int run_pass(blaze_search *s, const RunSpec &r, const std::vector<ScanPla
         ScanLaunch l;
         ScanArgs &sa = l.sa;
         std::memset(&sa, 0, sizeof(sa));  // whole bytes: the graph key compares them
-        l.word_table = lay.word_table;
+        l.words = lay.words;
         l.blocks = plan.blocks;
         l.warps_per_block = lay.warps_per_block;
         l.smem_bytes = lay.smem_bytes;
@@ -769,16 +770,20 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
         if (l.smem_bytes > kSmemMost)
             l = scan_layout(qlen, p0->window, n_hits, std::max(s->stage_bytes, 576u) - 576u, kSmemBudget, warps,
                             band_entries);
+        // and next to the very longest only the shortest subjects, and no bitset:
+        // query and window may have 56,688 residues together, with the bitset
+        // 55,888 to 56,000
+        if (l.smem_bytes > kSmemMost) l = scan_layout(qlen, p0->window, n_hits, 0, kSmemBudget, warps, band_entries, true);
         return l;
     };
     // layout of one batched scan launch over queries of up to `longest`
     // residues: shared memory for all the block's warps at the longest query
     // when that fits the budget, else the whole budget (at least one warp);
     // the block runs as many warps as fit for each query
-    auto batch_layout_for = [&](int32_t longest, bool word_table) {
+    auto batch_layout_for = [&](int32_t longest, Words words) {
         ScanLayout l = layout_for(longest, UINT32_MAX, 1, true);
-        const size_t regions = l.smem_bytes - l.warp_smem_bytes + (word_table ? kScanWordTabBytes - kScanPresenceBytes : 0);
-        l.word_table = word_table;
+        const size_t regions = l.smem_bytes - l.warp_smem_bytes - words_bytes(l.words) + words_bytes(words);
+        l.words = words;
         l.warps_per_block = std::max(1, std::min(warp_cap, kScanMaxWarpsPerBlock));
         l.smem_bytes = std::max(std::min(kSmemBudget, regions + static_cast<size_t>(l.warps_per_block) * l.warp_smem_bytes),
                                 regions + l.warp_smem_bytes);
@@ -831,12 +836,13 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
         pl.lay = query_layout(i, pl.queue);
         const bool banded = narrow || (has_pieces && db->max_len > share && p0->window <= kTab16Window);
         if (pl.queue) {
-            const bool smem = pl.lay.query_smem_bytes != 0, table = pl.lay.word_table;
+            const bool smem = pl.lay.query_smem_bytes != 0;
+            const Words words = pl.lay.words;
             for (; j < nq; ++j) {
                 const ScanLayout l = query_layout(j, true);
-                if ((l.query_smem_bytes != 0) != smem || l.word_table != table || is_narrow(j) != narrow) break;
+                if ((l.query_smem_bytes != 0) != smem || l.words != words || is_narrow(j) != narrow) break;
             }
-            pl.lay = batch_layout_for(qlen_at(j - 1), table);
+            pl.lay = batch_layout_for(qlen_at(j - 1), words);
         } else if (banded) {
             if (narrow) {
                 pl.lay = narrow_layout(i);
@@ -852,10 +858,10 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
         if (pl.lay.smem_bytes > kSmemMost) return BLAZE_ERR_LIMIT;
         int per_sm = 0;
         if (pl.queue) {
-            BLAZE_CUDA_TRY(scan_batch_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.word_table, pl.lay.warps_per_block,
+            BLAZE_CUDA_TRY(scan_batch_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.words, pl.lay.warps_per_block,
                                                 pl.lay.smem_bytes, &per_sm));
         } else {
-            BLAZE_CUDA_TRY(scan_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.word_table, pl.bands,
+            BLAZE_CUDA_TRY(scan_occupancy(pl.lay.query_smem_bytes != 0, pl.lay.words, pl.bands,
                                           pl.lay.warps_per_block, pl.lay.smem_bytes, &per_sm));
         }
         if (per_sm < 1) return BLAZE_ERR_LIMIT;

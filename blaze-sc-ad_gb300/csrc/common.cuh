@@ -36,6 +36,13 @@ constexpr int kPresenceWords = (kWords + 31) / 32;                     // 686
 constexpr size_t kScanMatBytes = kAlphabet * kAlphabet * 4;           // matrix, 3,136
 constexpr size_t kScanPresenceBytes = (kPresenceWords * 4 + 15) & ~15; // 2752
 constexpr size_t kScanWordTabBytes = ((kWords + 1) * 2 + 15) & ~15;    // 43,920
+// Where the scan looks a word up: in a table of the hit lists' starts in shared
+// memory, in the packed cells of words whose bit is set in a bitset there, or in
+// the packed cells alone, which leaves the longest diagonal tables the most room.
+enum class Words { kBitset, kTable, kPacked };
+__host__ __device__ constexpr uint32_t words_bytes(Words w) {
+    return static_cast<uint32_t>(w == Words::kTable ? kScanWordTabBytes : w == Words::kBitset ? kScanPresenceBytes : 0);
+}
 constexpr uint32_t kScanWordTabHits = 65535;  // hit-list entries a 16-bit word table can number
 constexpr int32_t kQuerySmemMax = 11776;      // queries up to this length live in shared memory,
 constexpr int32_t kBandQuerySmemMax = 14336;  // in bands this one,
@@ -278,7 +285,7 @@ struct HitlistArgs {
 // Shared-memory layout of the scan kernel for one query.
 struct ScanLayout {
     uint32_t diag_entries, diag_magic, diag_bytes, stage_bytes, query_smem_bytes, warp_smem_bytes;
-    bool word_table;  // the 16-bit word table in shared memory instead of the presence bitset
+    Words words;
     int warps_per_block;
     size_t smem_bytes;
 };
@@ -328,10 +335,10 @@ struct TracebackArgs {
 
 // Launchers (scan.cu, kernels.cu, traceback.cu).
 ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t n_hits, uint32_t stage_bytes, size_t smem_budget,
-                       int max_warps, uint32_t band_entries = 0);
-cudaError_t launch_scan(const ScanArgs &a, bool word_table, int n_blocks, int warps_per_block, size_t smem,
+                       int max_warps, uint32_t band_entries = 0, bool least = false);
+cudaError_t launch_scan(const ScanArgs &a, Words words, int n_blocks, int warps_per_block, size_t smem,
                         cudaStream_t st);
-cudaError_t scan_occupancy(bool query_in_smem, bool word_table, bool bands, int warps_per_block, size_t smem, int *blocks_per_sm);
+cudaError_t scan_occupancy(bool query_in_smem, Words words, bool bands, int warps_per_block, size_t smem, int *blocks_per_sm);
 int scan_max_warps_by_registers(bool query_in_smem);
 cudaError_t launch_gapped(const GappedArgs &a, int n_blocks, cudaStream_t st,
                           int warps_per_block = kGappedWarpsPerBlock);
@@ -339,9 +346,9 @@ cudaError_t launch_hitlist(const HitlistArgs &a, uint32_t n_select, int n_sm, cu
 constexpr int kTracebackWarpsPerBlock = 4;
 constexpr int kTracebackBlocksPerSm = 5;
 cudaError_t launch_traceback(const TracebackArgs &a, int n_blocks, cudaStream_t st);
-cudaError_t launch_scan_batch(const ScanArgs &a, bool word_table, int n_blocks, int warps_per_block, size_t smem,
+cudaError_t launch_scan_batch(const ScanArgs &a, Words words, int n_blocks, int warps_per_block, size_t smem,
                               cudaStream_t st);
-cudaError_t scan_batch_occupancy(bool query_in_smem, bool word_table, int warps_per_block, size_t smem,
+cudaError_t scan_batch_occupancy(bool query_in_smem, Words words, int warps_per_block, size_t smem,
                                  int *blocks_per_sm);
 int scan_batch_max_warps_by_registers(bool query_in_smem);
 cudaError_t gapped_occupancy(int *blocks_per_sm);

@@ -4,11 +4,12 @@
 // One warp per group of subjects (or band of its diagonals); persistent warps
 // pull groups, longest subjects first, from a device cursor (batched: one per
 // query, and blocks go from query to query). Per block in shared memory: the
-// BLOSUM62 matrix, the query's word table or word-presence bitset and, for
-// queries up to kQuerySmemMax, the query residues. Per warp: the diagonal table,
-// the deferred-hit and seed queues, the list of a chunk's words with hits and a
-// staging buffer for the group, so the word scan and the extensions read shared
-// memory instead of making dependent global loads.
+// BLOSUM62 matrix, the query's word table or word-presence bitset (neither next
+// to the very longest diagonal tables) and, for queries up to kQuerySmemMax, the
+// query residues. Per warp: the diagonal table, the deferred-hit and seed queues,
+// the list of a chunk's words with hits and a staging buffer for the group, so
+// the word scan and the extensions read shared memory instead of making
+// dependent global loads.
 //
 // Reference counterpart: gpuBLAZE_full (BLAZE_gpu/gpuBLAZE.cu:885-1252), which
 // is a filter; this kernel produces the exact ungapped HSPs of the
@@ -47,8 +48,8 @@ __device__ __forceinline__ uint32_t fast_mod(uint32_t idx, uint32_t L, uint32_t 
 
 constexpr uint32_t kMatOff = 0;
 constexpr uint32_t kTabOff = kScanMatBytes;  // the word table, or the word-presence bitset
-template <bool WT>
-constexpr uint32_t kQueryOff = kTabOff + (WT ? kScanWordTabBytes : kScanPresenceBytes);
+template <Words W>
+constexpr uint32_t kQueryOff = kTabOff + words_bytes(W);
 // a warp's region, from Finder::w
 constexpr uint32_t kBarAt = 0;                                // the stage buffer's mbarrier
 constexpr uint32_t kDeferAt = 16;                             // two buffers of deferred hits
@@ -146,12 +147,12 @@ struct Subject {
 };
 
 // The query: in shared memory for queries up to kQuerySmemMax, else global.
-template <bool QSMEM, bool WT>
+template <bool QSMEM, Words W>
 struct Query {
     const uint8_t *ptr;
     int32_t len;
     __device__ __forceinline__ uint32_t at(int32_t i) const {
-        if (QSMEM) return smem[kQueryOff<WT> + i];
+        if (QSMEM) return smem[kQueryOff<W> + i];
         return __ldg(ptr + i);
     }
 };
@@ -495,8 +496,8 @@ __device__ __forceinline__ bool queues_full(const Finder &f) {
 // a seed, so the loop ends. Seeds of all the group's subjects share a flush: a
 // walk takes as many warp instructions a step whether one lane or 32 take it,
 // so what an extension costs falls with the seeds it shares its flush with.
-template <bool QS, bool WT, bool BANDS, bool ST>
-__device__ __forceinline__ void flush(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, WT> &q,
+template <bool QS, Words W, bool BANDS, bool ST>
+__device__ __forceinline__ void flush(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, W> &q,
                                       const Span<ST> &span, bool empty) {
     const uint32_t lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();
@@ -652,8 +653,8 @@ __device__ __forceinline__ void clip_cells(const Ctx &c, const Band &band, int32
 // its word by a population count. A chunk's last hits, too few for a batch,
 // wait in front of the next chunk's, so batches are full (at 300 query
 // residues a chunk brings 79 hits).
-template <bool QS, bool WT, bool BANDS, bool ST>
-__device__ __forceinline__ void scan_span(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, WT> &q,
+template <bool QS, Words W, bool BANDS, bool ST>
+__device__ __forceinline__ void scan_span(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, W> &q,
                                           const Span<ST> &span, bool long_one, const Band &band) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t list = f.w + kListAt;
@@ -690,13 +691,13 @@ __device__ __forceinline__ void scan_span(Finder &f, const ScanArgs &a, const Ct
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const bool in = ST || p0 + j < xend;  // (zeros follow the staged residues)
-            if (WT) {
+            if (W == Words::kTable) {
                 const uint32_t t = kTabOff + (in ? r[j] * 1568u + r[j + 1] * 56u + r[j + 2] * 2u : 0u);
                 cs[j] = lds16(t);
                 cnt[j] = lds16(t + 2u) - cs[j];
             } else {
                 const uint32_t w = in ? r[j] * 784u + r[j + 1] * 28u + r[j + 2] : 0u;
-                const bool present = (lds32(kTabOff + 4u * (w >> 5)) >> (w & 31u)) & 1u;
+                const bool present = W == Words::kPacked ? in : (lds32(kTabOff + 4u * (w >> 5)) >> (w & 31u)) & 1u;
                 const uint32_t pk = present ? __ldg(c.cell_pack + w) : 0u;
                 cs[j] = pk >> 8;
                 cnt[j] = pk & 0xffu;
@@ -749,7 +750,7 @@ __device__ __forceinline__ void scan_span(Finder &f, const ScanArgs &a, const Ct
                 m = begins_from(k0);
             }
             const bool done = empty && k0 >= total;
-            if (queues_full(f) || done) flush<QS, WT, BANDS>(f, a, c, q, span, done);
+            if (queues_full(f) || done) flush<QS, W, BANDS>(f, a, c, q, span, done);
             if (done || !batch) break;
         } while (true);
         // the hits left wait: their words move to the front of the list, counted from k0
@@ -1000,8 +1001,8 @@ __device__ __forceinline__ Item item_at(const ScanArgs &a, uint32_t t) {
 
 // The fetched subjects for the query of `c`: finds the item's init hits and
 // publishes each subject's. False when a staging copy never landed.
-template <bool QS, bool WT, bool BANDS>
-__device__ __forceinline__ bool process_group(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, WT> &q,
+template <bool QS, Words W, bool BANDS>
+__device__ __forceinline__ bool process_group(Finder &f, const ScanArgs &a, const Ctx &c, const Query<QS, W> &q,
                                               const Group &g, uint32_t query_index, const Item &it) {
     f.n_init = 0;
     f.vb = 0;
@@ -1021,12 +1022,12 @@ __device__ __forceinline__ bool process_group(Finder &f, const ScanArgs &a, cons
         span.off = f.w + kDiagAt + c.diag_bytes;
         span.ptr = nullptr;
         clear_margins(f, span.off);
-        scan_span<QS, WT, BANDS>(f, a, c, q, span, long_one, b);
+        scan_span<QS, W, BANDS>(f, a, c, q, span, long_one, b);
     } else {  // one subject
         Span<false> span;
         span.off = 0;
         span.ptr = a.res + g.o0;
-        scan_span<QS, WT, BANDS>(f, a, c, q, span, long_one, b);
+        scan_span<QS, W, BANDS>(f, a, c, q, span, long_one, b);
     }
     if (b.all || merge_bands(f, a, it.group, it.n_bands)) {
         if (f.n_init > a.scratch_cap) scratch_overflow(a, f.n_init);
@@ -1056,23 +1057,23 @@ __device__ __forceinline__ void load_matrix() {
 
 // A query's tables in shared memory: its word table or word-presence bitset,
 // and its residues.
-template <bool QS, bool WT>
+template <bool QS, Words W>
 __device__ __forceinline__ void load_query_tables(const uint32_t *cell_start, const uint32_t *presence,
                                                   const uint8_t *q, int32_t qlen) {
-    if (WT) {
+    if (W == Words::kTable) {
         uint16_t *tab = reinterpret_cast<uint16_t *>(smem + kTabOff);
         for (uint32_t i = threadIdx.x; i <= kWords; i += blockDim.x) tab[i] = static_cast<uint16_t>(cell_start[i]);
-    } else {
+    } else if (W == Words::kBitset) {
         for (uint32_t i = threadIdx.x; i < kPresenceWords; i += blockDim.x) sts32(kTabOff + 4u * i, presence[i]);
     }
     if (QS)
-        for (int i = threadIdx.x; i < qlen; i += blockDim.x) smem[kQueryOff<WT> + i] = q[i];
+        for (int i = threadIdx.x; i < qlen; i += blockDim.x) smem[kQueryOff<W> + i] = q[i];
 }
 
 // One query against the whole database: the query's word table (or its
 // word-presence bitset) and the query itself when short enough live in shared
 // memory; warps pull groups, longest subjects first.
-template <bool QS, bool WT, bool BANDS>
+template <bool QS, Words W, bool BANDS>
 __global__ void __launch_bounds__(kScanMaxWarpsPerBlock * 32, 1)
 scan_kernel(const ScanArgs a) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1089,7 +1090,7 @@ scan_kernel(const ScanArgs a) {
     c.cutoff = a.cutoff;
     c.seed_span = seed_span(a.window);
     Finder f{};
-    start_region(f, kQueryOff<WT> + a.query_smem_bytes + warp * a.warp_smem_bytes);
+    start_region(f, kQueryOff<W> + a.query_smem_bytes + warp * a.warp_smem_bytes);
     // each warp's first group is its own, the longest subjects spread over the
     // blocks; its copy runs while the block fills its tables
     unsigned long long t = static_cast<unsigned long long>(warp) * gridDim.x + blockIdx.x;
@@ -1103,13 +1104,13 @@ scan_kernel(const ScanArgs a) {
     }
     clear_table<QS>(f, c);
     load_matrix();
-    load_query_tables<QS, WT>(a.cell_start, a.presence, a.q, a.qlen);
+    load_query_tables<QS, W>(a.cell_start, a.presence, a.q, a.qlen);
     __syncthreads();
-    Query<QS, WT> q;
+    Query<QS, W> q;
     q.ptr = a.q;
     q.len = a.qlen;
     while (t < a.n_items) {
-        if (!process_group<QS, WT, BANDS>(f, a, c, q, g, a.query_index, it)) return;
+        if (!process_group<QS, W, BANDS>(f, a, c, q, g, a.query_index, it)) return;
         uint32_t lo = g.lo + f.ns;
         if (lo == hi) {
             if (lane == 0) t = atomicAdd(a.cursor, 1ull) + static_cast<unsigned long long>(gridDim.x) * (blockDim.x >> 5);
@@ -1134,13 +1135,13 @@ scan_kernel(const ScanArgs a) {
 // one launch, and in a launch each 112, or 15.4 in bands. The block lays its warps' regions out
 // for each query: a warp's diagonal table takes the query's length plus the
 // window, so as many warps as fit (at most the block's) work on it.
-template <bool QS, bool WT>
+template <bool QS, Words W>
 __global__ void __launch_bounds__(kScanMaxWarpsPerBlock * 32, 1)
 scan_batch_kernel(const ScanArgs a) {
     __shared__ uint32_t s_next;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     load_matrix();
-    const uint32_t regions = kQueryOff<WT> + a.query_smem_bytes;
+    const uint32_t regions = kQueryOff<W> + a.query_smem_bytes;
     const uint32_t start = static_cast<uint32_t>(static_cast<unsigned long long>(blockIdx.x) * a.n_queries / gridDim.x);
     Finder f{};
     bool staging = true;  // false after a bulk copy that never landed (kFlagBadState is set)
@@ -1171,7 +1172,7 @@ scan_batch_kernel(const ScanArgs a) {
         if (from == a.n_queries) break;
         const uint32_t qi = (start + from) % a.n_queries;
         const BatchQuery bq = a.queries[qi];
-        load_query_tables<QS, WT>(bq.cell_start, bq.presence, bq.q, bq.qlen);
+        load_query_tables<QS, W>(bq.cell_start, bq.presence, bq.q, bq.qlen);
         __syncthreads();
         const uint32_t warp_bytes = scan_warp_bytes(bq.diag_bytes, a.stage_bytes);
         const uint32_t active = min(blockDim.x >> 5, (a.smem_bytes - regions) / warp_bytes);  // >= 1 (host)
@@ -1190,7 +1191,7 @@ scan_batch_kernel(const ScanArgs a) {
             c.seed_span = seed_span(a.window);
             start_region(f, regions + warp * warp_bytes);
             clear_table<QS>(f, c);
-            Query<QS, WT> q;
+            Query<QS, W> q;
             q.ptr = bq.q;
             q.len = bq.qlen;
             for (uint32_t lo = 0, hi = 0;;) {
@@ -1204,7 +1205,7 @@ scan_batch_kernel(const ScanArgs a) {
                 }
                 // after a copy that never landed: read this and every later
                 // subject from global memory (the host reports the run as failed)
-                while (!process_group<QS, WT, false>(f, a, c, q, fetch_group(f, a, c, lo, hi, staging), bq.index, Item{}))
+                while (!process_group<QS, W, false>(f, a, c, q, fetch_group(f, a, c, lo, hi, staging), bq.index, Item{}))
                     staging = false;
                 lo += f.ns;
             }
@@ -1219,7 +1220,7 @@ scan_batch_kernel(const ScanArgs a) {
 }  // namespace
 
 ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t n_hits, uint32_t stage_bytes, size_t smem_budget,
-                       int max_warps, uint32_t band_entries) {
+                       int max_warps, uint32_t band_entries, bool least) {
     ScanLayout l{};
     const bool smem = scan_query_in_smem(qlen, window, band_entries != 0);
     l.diag_entries = band_entries ? band_entries : scan_diag_entries(qlen, window);
@@ -1235,9 +1236,9 @@ ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t n_hits, uint32_t s
         l.warps_per_block = w;
         l.smem_bytes = fixed + static_cast<size_t>(w) * l.warp_smem_bytes;
     };
-    fit(kScanPresenceBytes);
+    l.words = least && !smem ? Words::kPacked : Words::kBitset;
+    fit(words_bytes(l.words));
     const int w0 = l.warps_per_block;
-    l.word_table = false;
     // the word table in shared memory where its 16 bits can number the hits and
     // it costs few warps: 139 M residues at 300 query residues 1.43 -> 1.30 ms
     // and at 1,000 (29 warps of 32) 3.56 -> 3.47, but at 1,500 (22 of 28) 5.05
@@ -1245,8 +1246,8 @@ ScanLayout scan_layout(int32_t qlen, int32_t window, uint32_t n_hits, uint32_t s
     constexpr int kWordTabWarps = 28;
     if (l.query_smem_bytes && n_hits <= kScanWordTabHits) {
         fit(kScanWordTabBytes);
-        l.word_table = l.warps_per_block >= std::min(w0, kWordTabWarps);
-        if (!l.word_table) fit(kScanPresenceBytes);
+        if (l.warps_per_block >= std::min(w0, kWordTabWarps)) l.words = Words::kTable;
+        else fit(kScanPresenceBytes);
     }
     return l;
 }
@@ -1276,17 +1277,19 @@ static cudaError_t allow_full_smem(const void *kernel) {
     return e;
 }
 
-static void (*single_kernel(bool query_in_smem, bool word_table, bool bands))(ScanArgs) {
+static void (*single_kernel(bool query_in_smem, Words words, bool bands))(ScanArgs) {
+    constexpr Words kBitset = Words::kBitset, kTable = Words::kTable;
     if (bands)
-        return !query_in_smem ? scan_kernel<false, false, true>
-                              : word_table ? scan_kernel<true, true, true> : scan_kernel<true, false, true>;
-    return !query_in_smem ? scan_kernel<false, false, false>
-                          : word_table ? scan_kernel<true, true, false> : scan_kernel<true, false, false>;
+        return !query_in_smem ? scan_kernel<false, kBitset, true>
+                              : words == kTable ? scan_kernel<true, kTable, true> : scan_kernel<true, kBitset, true>;
+    if (words == Words::kPacked) return scan_kernel<false, Words::kPacked, false>;
+    return !query_in_smem ? scan_kernel<false, kBitset, false>
+                          : words == kTable ? scan_kernel<true, kTable, false> : scan_kernel<true, kBitset, false>;
 }
 
-cudaError_t launch_scan(const ScanArgs &a, bool word_table, int n_blocks, int warps_per_block, size_t smem_bytes,
+cudaError_t launch_scan(const ScanArgs &a, Words words, int n_blocks, int warps_per_block, size_t smem_bytes,
                         cudaStream_t st) {
-    auto kernel = single_kernel(a.query_smem_bytes != 0, word_table, a.pieces != nullptr);
+    auto kernel = single_kernel(a.query_smem_bytes != 0, words, a.pieces != nullptr);
     cudaError_t e = allow_full_smem(reinterpret_cast<const void *>(kernel));
     if (e != cudaSuccess) return e;
     kernel<<<n_blocks, warps_per_block * 32, smem_bytes, st>>>(a);
@@ -1307,43 +1310,45 @@ static int max_warps_by_registers(const void *kernel) {
 int scan_max_warps_by_registers(bool query_in_smem) {
     int w = kScanMaxWarpsPerBlock;
     for (bool bands : {false, true})
-        for (bool table : {false, true})
+        for (Words words : {Words::kBitset, Words::kTable})
             w = std::min(w, max_warps_by_registers(reinterpret_cast<const void *>(
-                                single_kernel(query_in_smem, table && query_in_smem, bands))));
+                                single_kernel(query_in_smem, words, bands))));
     return w;
 }
 
-static void (*batch_kernel(bool query_in_smem, bool word_table))(ScanArgs) {
-    return !query_in_smem ? scan_batch_kernel<false, false>
-                          : word_table ? scan_batch_kernel<true, true> : scan_batch_kernel<true, false>;
+static void (*batch_kernel(bool query_in_smem, Words words))(ScanArgs) {
+    constexpr Words kBitset = Words::kBitset, kTable = Words::kTable;
+    if (words == Words::kPacked) return scan_batch_kernel<false, Words::kPacked>;
+    return !query_in_smem ? scan_batch_kernel<false, kBitset>
+                          : words == kTable ? scan_batch_kernel<true, kTable> : scan_batch_kernel<true, kBitset>;
 }
 
-cudaError_t launch_scan_batch(const ScanArgs &a, bool word_table, int n_blocks, int warps_per_block, size_t smem_bytes,
+cudaError_t launch_scan_batch(const ScanArgs &a, Words words, int n_blocks, int warps_per_block, size_t smem_bytes,
                               cudaStream_t st) {
-    auto kernel = batch_kernel(a.query_smem_bytes != 0, word_table);
+    auto kernel = batch_kernel(a.query_smem_bytes != 0, words);
     cudaError_t e = allow_full_smem(reinterpret_cast<const void *>(kernel));
     if (e != cudaSuccess) return e;
     kernel<<<n_blocks, warps_per_block * 32, smem_bytes, st>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t scan_batch_occupancy(bool query_in_smem, bool word_table, int warps_per_block, size_t smem_bytes,
+cudaError_t scan_batch_occupancy(bool query_in_smem, Words words, int warps_per_block, size_t smem_bytes,
                                  int *blocks_per_sm) {
-    auto kernel = batch_kernel(query_in_smem, word_table);
+    auto kernel = batch_kernel(query_in_smem, words);
     cudaError_t e = allow_full_smem(reinterpret_cast<const void *>(kernel));
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel, warps_per_block * 32, smem_bytes);
 }
 
 int scan_batch_max_warps_by_registers(bool query_in_smem) {
-    const int w = max_warps_by_registers(reinterpret_cast<const void *>(batch_kernel(query_in_smem, false)));
+    const int w = max_warps_by_registers(reinterpret_cast<const void *>(batch_kernel(query_in_smem, Words::kBitset)));
     if (!query_in_smem) return w;
-    return std::min(w, max_warps_by_registers(reinterpret_cast<const void *>(batch_kernel(true, true))));
+    return std::min(w, max_warps_by_registers(reinterpret_cast<const void *>(batch_kernel(true, Words::kTable))));
 }
 
-cudaError_t scan_occupancy(bool query_in_smem, bool word_table, bool bands, int warps_per_block, size_t smem_bytes,
+cudaError_t scan_occupancy(bool query_in_smem, Words words, bool bands, int warps_per_block, size_t smem_bytes,
                            int *blocks_per_sm) {
-    auto kernel = single_kernel(query_in_smem, word_table, bands);
+    auto kernel = single_kernel(query_in_smem, words, bands);
     cudaError_t e = allow_full_smem(reinterpret_cast<const void *>(kernel));
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel, warps_per_block * 32,
