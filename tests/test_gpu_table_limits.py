@@ -1,5 +1,7 @@
 """The largest diagonal tables, against the oracle: query and window lengths up to
-the most that shared memory holds, in the plain and both batched forms."""
+the most that shared memory holds, in the plain and both batched forms, and the
+16-bit table at its longest query, with subjects long enough that it has to be
+moved down and a match along nearly the whole query."""
 import numpy as np
 import pytest
 
@@ -56,5 +58,26 @@ def test_beyond_the_longest_table():
     p, _ = params_for(len(q), db.tot_len, 1, window=24_689)
     with pytest.raises(blaze103.BlazeError):
         ps.run(q, p)
+    ps.close()
+    db.close()
+
+
+@pytest.mark.parametrize("qlen", [11_776, 11_777])
+def test_longest_16_bit_table(qlen):
+    rng = np.random.default_rng(qlen)
+    q = synth.random_residues(rng, qlen)
+    seqs = [synth.random_residues(rng, int(L)) for L in (1, 300, 2240, 16_383, 16_384, 33_000)]
+    seqs[4][3000:3000 + qlen - 60] = q[30:qlen - 30]  # along a diagonal, within a moved table
+    seqs[5][20_000:20_000 + qlen] = q
+    seqs.append(q.copy())
+    seqs.append(np.concatenate([q[5000:], q[:5000]]))
+    res, off = concat(seqs)
+    over = dict(window=256)
+    db = blaze103.SeqSrc(res, off)
+    ps = blaze103.PrelimSearch(db, autotune=False)
+    want, _, _ = compare(q, res, off, seq_src=db, search=ps, **over)
+    assert len(want) >= 4
+    for mode in (1, 2):
+        _batched(db, ps, [q], mode, [want], **over)
     ps.close()
     db.close()
