@@ -22,7 +22,9 @@ namespace {
 // Size of every three-letter word's neighbourhood for one threshold: the words
 // v with score(w, v) >= threshold, and w itself (BLAZE_ncbi/
 // prelim_stage.cpp:135-155 enumerates the same set; :378-383 keeps the exact
-// word). Computed once per threshold and kept (44 KB) for a few of them.
+// word). No v has the letter 0, whatever the threshold: residues are 1 and up,
+// and the scan takes zeros around its subjects for words without hits. Computed
+// once per threshold and kept (44 KB) for a few of them.
 std::mutex g_nb_mutex;
 using NeighbourhoodSizes = std::shared_ptr<const std::vector<uint16_t>>;
 std::map<int32_t, NeighbourhoodSizes> g_nb_cache;
@@ -40,16 +42,16 @@ NeighbourhoodSizes neighbourhood_sizes(int32_t threshold) {
     for (int w = 0; w < kWords; ++w) {
         const int x = w / 784, y = (w / 28) % 28, z = w % 28;
         uint32_t n = kBlosum62[x][x] + kBlosum62[y][y] + kBlosum62[z][z] < threshold ? 1 : 0;
-        for (int a = 0; a < kAlphabet; ++a) {
+        for (int a = 1; a < kAlphabet; ++a) {
             const int32_t s0 = kBlosum62[x][a];
             if (s0 + row_max[y] + row_max[z] < threshold) continue;
-            for (int b = 0; b < kAlphabet; ++b) {
+            for (int b = 1; b < kAlphabet; ++b) {
                 const int32_t s1 = s0 + kBlosum62[y][b];
                 if (s1 + row_max[z] < threshold) continue;
-                for (int c = 0; c < kAlphabet; ++c) n += s1 + kBlosum62[z][c] >= threshold ? 1u : 0u;
+                for (int c = 1; c < kAlphabet; ++c) n += s1 + kBlosum62[z][c] >= threshold ? 1u : 0u;
             }
         }
-        size[w] = static_cast<uint16_t>(n);  // at most 21,952
+        size[w] = static_cast<uint16_t>(n);  // at most 27^3
     }
     if (g_nb_cache.size() >= kNbCacheMost) g_nb_cache.clear();
     return g_nb_cache.emplace(threshold, std::move(sizes)).first->second;

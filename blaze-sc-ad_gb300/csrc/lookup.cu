@@ -71,7 +71,7 @@ __device__ __forceinline__ void walk_setup(WalkShared &sh) {
     __syncthreads();
 }
 
-// The warp's part of the query: calls hit(c, mask, i) for each third letter c
+// The warp's part of the query: calls hit(c, mask, i) for each third letter c from 1
 // and batch of candidates: the lanes in mask have the word's offset i. Every
 // lane makes every call.
 template <typename F>
@@ -81,7 +81,8 @@ __device__ __forceinline__ void walk_query(WalkShared &sh, const LookupQuery &lq
     const int32_t *mat = sh.mat;
     uint32_t *cand = sh.cand[warp];
     int32_t *cand_score = sh.cand_score[warp];
-    const int32_t from = min(sp.part * static_cast<int32_t>(sp.mine()), sp.all), n = min(from + sp.part, sp.all);
+    const int32_t from = min(sp.part * static_cast<int32_t>(sp.mine()), sp.all);
+    const int32_t n = a > 0u && b > 0u ? min(from + sp.part, sp.all) : from;  // no word with the letter 0 has hits
     uint32_t have = 0;
     auto test = [&](uint32_t m) {  // the first m candidates
         const bool in = lane < m;
@@ -90,7 +91,7 @@ __device__ __forceinline__ void walk_query(WalkShared &sh, const LookupQuery &lq
         const uint32_t z = (w >> 16) & 31u;
         const bool same = (w >> 31) != 0u;
 #pragma unroll 4
-        for (uint32_t c = 0; c < kAlphabet; ++c) {
+        for (uint32_t c = 1; c < kAlphabet; ++c) {
             const bool h = in && (s + mat[z * kRow + c] >= threshold || (same && z == c));
             hit(c, __ballot_sync(kFull, h), w & 0xffffu);
         }

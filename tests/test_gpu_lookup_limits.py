@@ -1,5 +1,6 @@
-"""Queries whose word lookup has more list entries than 24 bits number, against
-the oracle: the packed cells cannot hold where the later words' lists begin."""
+"""The word lookup at its limits, against the oracle: queries with more list entries
+than 24 bits number (the packed cells cannot hold where the later words' lists
+begin), and thresholds low enough for words with the letter 0."""
 import numpy as np
 import pytest
 
@@ -37,5 +38,29 @@ def test_lists_beyond_24_bits(qlen, threshold, fits):
     for f in ["oid"] + HSP_FIELDS:
         assert np.array_equal(one[f], want[f])
         assert np.array_equal(got[f], want[f])
+    ps.close()
+    db.close()
+
+
+# a word with one letter 0 scores -32,746 at most; no residue is 0
+@pytest.mark.parametrize("threshold", [-32_745, -32_746, -40_000, -100_000, -(2**31), 2**31 - 1])
+@pytest.mark.parametrize("stage_bytes", [0, 128])
+def test_thresholds_that_the_letter_0_reaches(threshold, stage_bytes):
+    rng = np.random.default_rng(23)
+    qs = [synth.random_residues(rng, L) for L in (2, 12, 300)]
+    seqs = [synth.random_residues(rng, int(L)) for L in rng.integers(0, 90, 50)]
+    seqs += [np.concatenate([synth.random_residues(rng, 9), q[:60]]) for q in qs] + [synth.random_residues(rng, 3000)]
+    res, off = concat(seqs)
+    over = dict(word_threshold=threshold, ungapped_cutoff=12)
+    db = blaze103.SeqSrc(res, off)
+    ps = blaze103.PrelimSearch(db, autotune=False)
+    ps.set_tuning(stage_bytes=stage_bytes)
+    batch = blaze103.QueryBatch(db, qs, threshold)
+    got = ps.run_batch(batch, [params_for(len(q), db.tot_len, db.num_seqs, **over)[0] for q in qs])
+    batch.close()
+    for i, q in enumerate(qs):
+        want, _, _ = compare(q, res, off, seq_src=db, search=ps, **over)
+        for f in ["oid"] + HSP_FIELDS:
+            assert np.array_equal(got[got["query"] == i][f], want[f])
     ps.close()
     db.close()
