@@ -1210,13 +1210,24 @@ extern "C" int blaze_prelim_search(blaze_search *s, const uint8_t *query, int32_
     std::memset(s->h_stage + length, 0, t.res_bytes - static_cast<size_t>(length));
     if ((rc = s->qt.ensure(t.bytes)) != BLAZE_OK) return rc;
     t.point(q, s->qt.p);
+    // A search that is refused waits for nothing: then the copy has to end here,
+    // since the next call overwrites the staging, and other residues under the
+    // lookup's kernels could have more hits than the tables have room for.
+    struct StreamWait {
+        cudaStream_t st;
+        bool on = true;
+        ~StreamWait() {
+            if (on) cudaStreamSynchronize(st);
+        }
+    } wait{s->stream};
     BLAZE_CUDA_TRY(cudaMemcpyAsync(q.d_q, s->h_stage, t.res_bytes, cudaMemcpyHostToDevice, s->stream));
     BLAZE_CUDA_TRY(build_lookup(q, s->stream));
     RunSpec r;
     r.q = &q;
     r.p = p;
-    rc = run_search(s, r, n_hsps);  // synchronises the stream before it returns
+    rc = run_search(s, r, n_hsps);
     s->stats.h2d_bytes += q.upload_bytes;
     if (rc != BLAZE_OK) return rc;
+    wait.on = false;  // the search has waited
     return blaze_search_results(s, out, capacity, n_hsps);
 } BLAZE_ABI_CATCH
