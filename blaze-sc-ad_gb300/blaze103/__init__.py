@@ -298,8 +298,8 @@ class PrelimSearch:
                    launch_mode: int = 0, batch_launch: int = 0):
         """Launch shape (0 = library default for each); launch_mode 0: CUDA
         graph for batched runs, 1: direct launches, 2: CUDA graph always;
-        batch_launch 0: by the longest subject, 1: many queries per
-        launch, 2: one scan launch per query."""
+        batch_launch 0: by the database's residues and its longest subject,
+        1: many queries per launch, 2: one scan launch per query."""
         self._auto = False
         self._set_tuning(stage_bytes, tile_residues, max_warps_per_block, launch_mode, batch_launch)
 

@@ -8,7 +8,7 @@ block -- checks that every setting returns the same HSPs, and writes the fastest
 setting per shape to ``tuning.json`` beside this file. ``lookup`` returns the
 entry of the nearest shape; ``PrelimSearch`` applies it to batched runs unless
 a tuning was set explicitly. The batched launch mode stays automatic: it goes
-by the database's longest subject, which a shape does not tell.
+by the database's residues and its longest subject, which a shape does not tell.
 
 Run on the GPU:  python blaze-sc-ad_gb300/blaze103/autotune.py [--quick]
 """

@@ -813,14 +813,23 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     //   residues against 140 M: 42.0 -> 37.5, 172 -> 62 and 1,520 -> 230 ms; at
     //   5,000 (14 warps without) 19.9 -> 24.0, since every band looks up its
     //   words again. Such queries of a batch have launches of their own too.
-    // A batch runs as one launch whose blocks go from query to query where a
-    // query's own pass would end in a wait for its longest subjects, that is
-    // where one of them is more than a warp's share of the residues: 16 queries
-    // of 2,000 to 5,000 residues against 10.5 M residues with subjects of up to
-    // 35,000 scan in 13.1 ms, with a banded launch each in 15.4. Otherwise one
-    // launch per query is the faster (256 queries against 35 M residues 100.9 ms
-    // and 103.9).
-    const bool per_query = batched && (s->batch_launch == 2 || (s->batch_launch == 0 && (nq == 1 || db->max_len < share)));
+    // A batch runs as one launch whose blocks go from query to query
+    // - where a query's own pass would end in a wait for its longest subjects,
+    //   that is where one of them is more than a warp's share of the residues: 16
+    //   queries of 2,000 to 5,000 residues against 10.5 M residues with subjects
+    //   of up to 35,000 scan in 13.1 ms, with a banded launch each in 15.4;
+    // - where a query's own pass is mostly its start and its end: against fewer
+    //   than 2^23 residues. 64 queries of 20 to 60 residues against 0.3 / 3 / 8 M
+    //   residues of peptides in one launch 0.50 / 1.21 / 2.60 ms, in one each 1.11
+    //   / 1.71 / 3.04; 64 of 50 to 500 against 3 / 8 M of proteins up to 300 2.02 /
+    //   4.84 and 2.64 / 5.30.
+    // Otherwise one launch per query is the faster (4 queries of 50 to 500 residues
+    // against 12 M 0.593 and 0.604 ms, 17 of 1,000 to 5,000 18.2 and 18.6, 256 against
+    // 35 M 100.9 and 103.9).
+    constexpr uint64_t kOneLaunchResidues = 1ull << 23;
+    const bool per_query = batched && (s->batch_launch == 2 ||
+                                       (s->batch_launch == 0 &&
+                                        (nq == 1 || (db->max_len < share && db->total >= kOneLaunchResidues))));
     const bool has_pieces = db->n_pieces + 1 > db->h_groups.size();
     auto narrow_layout = [&](uint32_t k) { return query_layout(k, false, scan_band_entries(qlen_at(k))); };
     auto is_narrow = [&](uint32_t k) {  // (a group's bands have to be staged as one)

@@ -307,10 +307,11 @@ typedef struct blaze_tuning {
      * The graph is captured once and replayed while the launch arguments stay
      * the same (updated in place when they change). */
     uint32_t launch_mode;
-    /* Batched runs: 0: automatic (one scan launch for the whole batch where a
-     * subject is longer than a warp's share of the database, so that the
-     * queries do not wait for their longest subjects one after another; one
-     * launch per query otherwise); 1: one launch for the batch always; 2: one
+    /* Batched runs: 0: automatic (one scan launch for the whole batch against
+     * fewer than 2^23 residues, where a launch per query would be mostly its
+     * start and its end, and where a subject is longer than a warp's share of
+     * the database, so that the queries do not wait for their longest subjects
+     * one after another; one launch per query otherwise); 1: one launch for the batch always; 2: one
      * launch per query always. Results are identical either way. */
     uint32_t batch_launch;
 } blaze_tuning;
