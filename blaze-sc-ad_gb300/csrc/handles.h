@@ -33,6 +33,10 @@ struct blaze_db {
     // the word finder's groups, from the longest subjects down (ScanArgs::groups)
     std::vector<uint32_t> h_groups;
     uint32_t *d_groups = nullptr;
+    // groups that are not cut below 512 bytes on small databases, for launches of
+    // many queries (behind d_groups; null: those are such)
+    uint32_t *d_batch_groups = nullptr;
+    uint32_t n_batch_groups = 0;
     uint32_t *d_pieces = nullptr;  // prefix sums of the groups' pieces (ScanArgs::pieces)
     uint32_t n_pieces = 0;
     uint32_t group_bytes = 0;      // the most that the blocks of a group of several subjects take
