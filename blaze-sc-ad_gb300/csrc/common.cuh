@@ -344,8 +344,21 @@ cudaError_t launch_gapped(const GappedArgs &a, int n_blocks, cudaStream_t st,
                           int warps_per_block = kGappedWarpsPerBlock);
 cudaError_t launch_hitlist(const HitlistArgs &a, uint32_t n_select, int n_sm, cudaStream_t st);
 constexpr int kTracebackWarpsPerBlock = 4;
-constexpr int kTracebackBlocksPerSm = 5;
-cudaError_t launch_traceback(const TracebackArgs &a, int n_blocks, cudaStream_t st);
+constexpr int kTracebackBlocksPerSm = 5;      // with the band in registers
+constexpr int kTracebackRowsBlocksPerSm = 8;  // with the rows in memory
+constexpr int32_t kTbParts = 3, kTbWindow = 64 * kTbParts;  // columns that the registers hold
+// Whether an X-drop's bands fit the registers: they reach about three times the
+// columns of their first row's gap. Of 4,000 alignments of 300 residues at gap
+// costs 11/1 none outgrows them at X-drop 68 (0.47 ms, 0.82 with the rows in
+// memory), at 72 so many do that the other form is no slower, and from 95 on it is
+// the faster (1.03 and 1.01, at 140 2.54 and 2.24); of 2,300 of 450 residues with
+// subjects of up to 20,000 1.54 and 1.04 ms at 75. A band has one column more than
+// its subject at most.
+inline bool traceback_in_window(int32_t gap_open, int32_t gap_extend, int32_t xdrop, uint32_t longest) {
+    const int64_t first_gap = (static_cast<int64_t>(xdrop) - gap_open - gap_extend) / gap_extend;
+    return 3 * first_gap + 16 <= kTbWindow || longest + 1u <= static_cast<uint32_t>(kTbWindow);
+}
+cudaError_t launch_traceback(const TracebackArgs &a, bool window, int n_blocks, cudaStream_t st);
 cudaError_t launch_scan_batch(const ScanArgs &a, Words words, int n_blocks, int warps_per_block, size_t smem,
                               cudaStream_t st);
 cudaError_t scan_batch_occupancy(bool query_in_smem, Words words, int warps_per_block, size_t smem,

@@ -10,7 +10,7 @@
 // warp's buffer. The warp then walks the path back from the best cell, 32 cells
 // of a diagonal at a time. Where the band outgrows the registers, or the gap
 // costs or the X-drop are too large for them, the rows are kept in memory and
-// one lane walks.
+// one lane walks; X-drops with such bands go there at once.
 #include <cstdint>
 
 #include "common.cuh"
@@ -292,7 +292,6 @@ __device__ Walk walk_back(const DirRows &d, int32_t rows, const uint8_t *A, cons
 // 500 query residues: 1.20 ms with the rows in memory, both sides on one warp and
 // one lane walking back; 1.06 with 128 columns (many bands outgrow them), 0.62
 // with 192 and 20 warps an SM, 0.70 with 192 or 256 and 16 warps.
-constexpr int kTbParts = 3, kTbWindow = 64 * kTbParts;
 constexpr int kTbRowMost = kTbWindow + 64;  // bytes of a row: the window, moved by less than 64, holds its end
 __device__ __forceinline__ bool xdrop_dp_window_dirs(const uint8_t *__restrict__ Q, const uint8_t *__restrict__ S,
                                                      int32_t dir, int32_t M, int32_t N, int32_t gap_open,
@@ -505,7 +504,13 @@ __device__ __forceinline__ void walk_window(const DirRows &d, const uint8_t *__r
     p.status = 0;
 }
 
-__global__ void __launch_bounds__(kTracebackWarpsPerBlock * 32, kTracebackBlocksPerSm)
+// Sides whose bands are expected to outgrow the registers (traceback_in_window)
+// have a kernel without them: it needs fewer and runs more warps. 2,300 alignments
+// of 450 residues at X-drop 105 / 215: 3.02 / 5.08 ms as the other form's way out,
+// 2.36 / 4.11 so (2.40 / 4.35 with both sides on one warp).
+template <bool WINDOW>
+__global__ void
+__launch_bounds__(kTracebackWarpsPerBlock * 32, WINDOW ? kTracebackBlocksPerSm : kTracebackRowsBlocksPerSm)
 traceback_kernel(const TracebackArgs a) {
     __shared__ int32_t mat[kAlphabet * kAlphabet];
     for (int i = threadIdx.x; i < kAlphabet * kAlphabet; i += blockDim.x) mat[i] = g_blosum_tb[i];
@@ -540,7 +545,7 @@ traceback_kernel(const TracebackArgs a) {
         d.overflow = false;
         TbPart p{};
         p.last = -1;
-        if (dp_window_exact(M, a.gap_open, a.gap_extend, a.xdrop) &&
+        if (WINDOW && dp_window_exact(M, a.gap_open, a.gap_extend, a.xdrop) &&
             xdrop_dp_window_dirs(Q, S, dir, M, N, a.gap_open, a.gap_extend, a.xdrop, mat, d, p)) {
             if (!d.overflow) walk_window(d, Q, S, dir, mat, p);
         } else {
@@ -598,8 +603,9 @@ traceback_kernel(const TracebackArgs a) {
 
 }  // namespace
 
-cudaError_t launch_traceback(const TracebackArgs &a, int n_blocks, cudaStream_t st) {
-    traceback_kernel<<<n_blocks, kTracebackWarpsPerBlock * 32, 0, st>>>(a);
+cudaError_t launch_traceback(const TracebackArgs &a, bool window, int n_blocks, cudaStream_t st) {
+    auto kernel = window ? traceback_kernel<true> : traceback_kernel<false>;
+    kernel<<<n_blocks, kTracebackWarpsPerBlock * 32, 0, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -31,13 +31,17 @@ static int traceback_passes(blaze_search *s, const std::vector<TbItem> &items, c
     unsigned long long cap = (s->tb_dir_cap + 63) & ~63ull;  // rows of direction bytes begin at multiples of 64
     const uint32_t row_cap = (static_cast<uint32_t>(max_qlen) + 3u) & ~1u;  // even: pairs of ints
     const uint32_t dp_stride = std::max<uint32_t>(db->max_len, 1u) + 2u;
+    const bool window = traceback_in_window(p->gap_open, p->gap_extend, final_xdrop, db->max_len);
     std::vector<TbItem> pass_items;
     std::vector<TbOut> pass_out;
     int rc;
     for (int attempt = 0; !todo.empty(); ++attempt) {
         if (attempt > 12) return BLAZE_ERR_LIMIT;
         const size_t m = todo.size();
-        const int blocks = static_cast<int>(std::min<size_t>(static_cast<size_t>(s->n_sm) * kTracebackBlocksPerSm,
+        // fewer warps next to large direction buffers or DP rows
+        const bool large = cap > (1u << 20) || dp_stride > (1u << 17);
+        const int per_sm = large ? 4 : window ? kTracebackBlocksPerSm : kTracebackRowsBlocksPerSm;
+        const int blocks = static_cast<int>(std::min<size_t>(static_cast<size_t>(s->n_sm) * per_sm,
                                                              (2 * m + kTracebackWarpsPerBlock - 1) / kTracebackWarpsPerBlock));
         const size_t warps = static_cast<size_t>(blocks) * kTracebackWarpsPerBlock;
         pass_items.resize(m);
@@ -79,7 +83,7 @@ static int traceback_passes(blaze_search *s, const std::vector<TbItem> &items, c
         BLAZE_CUDA_TRY(cudaMemsetAsync(s->tb_done.p, 0, sizeof(unsigned int) * m, s->stream));
         BLAZE_CUDA_TRY(cudaMemsetAsync(s->tb_cursor.p, 0, sizeof(unsigned long long), s->stream));
         BLAZE_CUDA_TRY(cudaEventRecord(s->ev[1], s->stream));
-        BLAZE_CUDA_TRY(launch_traceback(ta, blocks, s->stream));
+        BLAZE_CUDA_TRY(launch_traceback(ta, window, blocks, s->stream));
         BLAZE_CUDA_TRY(cudaEventRecord(s->ev[2], s->stream));
         s->stats.kernel_launches += 1;
         BLAZE_CUDA_TRY(cudaMemcpyAsync(pass_out.data(), s->tb_out.p, sizeof(TbOut) * m, cudaMemcpyDeviceToHost,
