@@ -273,6 +273,8 @@ extern "C" int blaze_search_create(blaze_db *db, blaze_search **out) try {
         return BLAZE_ERR_CUDA;
     }
     s->gapped_blocks = s->n_sm * std::min(std::max(per_sm, 1), 8);
+    for (int smem = 0; smem < 2; ++smem) s->reg_warps[smem] = scan_max_warps_by_registers(smem != 0);
+    s->batch_reg_warps = std::min(scan_batch_max_warps_by_registers(true), scan_batch_max_warps_by_registers(false));
     s->init_cap = std::max<unsigned long long>(1ull << 20, db->n / 8);
     s->work_cap = std::max<unsigned long long>(1ull << 20, db->n / 4);
     s->out_cap = std::max<unsigned long long>(1ull << 20, db->n / 16);
@@ -763,9 +765,7 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
     if (n_hsps) *n_hsps = 0;
 
     constexpr size_t kSmemBudget = 220 * 1024;
-    const int reg_cap = batched ? std::min(scan_batch_max_warps_by_registers(true),
-                                           scan_batch_max_warps_by_registers(false))
-                                : scan_max_warps_by_registers(scan_query_in_smem(r.q->qlen, p0->window));
+    const int reg_cap = batched ? s->batch_reg_warps : s->reg_warps[scan_query_in_smem(r.q->qlen, p0->window)];
     const int warp_cap = s->max_warps ? std::min(reg_cap, static_cast<int>(s->max_warps)) : reg_cap;
     // layout of one single-query scan launch
     const uint64_t share = db->total / (static_cast<uint64_t>(s->n_sm) * kScanMaxWarpsPerBlock);

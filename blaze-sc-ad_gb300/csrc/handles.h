@@ -90,6 +90,9 @@ struct blaze_search {
     blaze_db *db = nullptr;
     cudaStream_t stream = nullptr;
     int n_sm = 0;
+    // warps that registers allow in a scan block: by whether a single query is in
+    // shared memory, and of batched runs (fixed per kernel, asked once)
+    int reg_warps[2] = {0, 0}, batch_reg_warps = 0;
     // per-run capacities
     uint32_t scratch_cap = kInitialScratchCap;
     unsigned long long init_cap = 0, out_cap = 0;
