@@ -815,11 +815,17 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
         return layout_for(qlen_at(k), batched ? r.b->n_off[order[k]] : r.q->n_off, warp_cap, queue, band_entries);
     };
     // One query's launch runs in bands of diagonals
-    // - where a subject is longer than a warp's share of the residues, so that
-    //   the launch would end in a wait for it: such subjects are cut in pieces.
-    //   300 and 4,999 residues against 17.5 M with subjects of up to 35,000:
-    //   0.81 -> 0.29 and 10.46 -> 2.83 ms; but 103 against 140 M, longest 5,000
-    //   (a share is 28,700), 0.62 -> 0.70;
+    // - where a subject is so long that the launch would end in a wait for it:
+    //   such subjects are cut in pieces. A warp alone on its SM takes a residue in
+    //   4 ns plus 0.05 per query residue, 2.5 times as fast as next to 31 others,
+    //   so the wait is for what a subject has beyond 2.5 shares of the residues (a
+    //   share: all of them over 152 x 32 warps); bands cost 10 to 15 us (a buffer
+    //   to clear, merging) and look words up again. 300 and 4,999 residues against
+    //   17.5 M with subjects of up to 35,000: 0.81 -> 0.29 and 10.46 -> 2.83 ms; of
+    //   uniform lengths up to 35,000, 100 residues against 34 / 85 / 131 M (5 / 2 /
+    //   1.3 shares): 0.50 -> 0.32, 0.61 -> 0.58, 0.72 -> 0.83, 3,000 residues 6.4 ->
+    //   4.5, 8.1 -> 10.2, 10.1 -> 15.3; up to 1,000, 31 residues against 0.25 / 1.6 M
+    //   84 -> 86 and 80 -> 95 us;
     // - for the longest queries, with a table of one band's diagonals: tables of
     //   a whole query would leave few warps an SM. 8,000 / 12,345 / 30,000
     //   residues against 140 M: 42.0 -> 37.5, 172 -> 62 and 1,520 -> 230 ms; at
@@ -843,6 +849,10 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
                                        (s->batch_launch == 0 &&
                                         (nq == 1 || (db->max_len < share && db->total >= kOneLaunchResidues))));
     const bool has_pieces = db->n_pieces + 1 > db->h_groups.size();
+    auto waits_for_longest = [&](int32_t qlen) {
+        const uint64_t passed = share * 5 / 2;
+        return db->max_len > passed && (db->max_len - passed) * (static_cast<uint64_t>(qlen) + 80) >= 240000;
+    };
     auto narrow_layout = [&](uint32_t k) { return query_layout(k, false, scan_band_entries(qlen_at(k))); };
     auto is_narrow = [&](uint32_t k) {  // (a group's bands have to be staged as one)
         return qlen_at(k) > kBandQuery && p0->window <= kTab16Window && db->n > 0 &&
@@ -855,7 +865,7 @@ static int run_search(blaze_search *s, const RunSpec &spec, uint64_t *n_hsps) {
         const bool narrow = is_narrow(i);
         pl.queue = batched && !per_query && (!narrow || s->batch_launch == 1);
         pl.lay = query_layout(i, pl.queue);
-        const bool banded = narrow || (has_pieces && db->max_len > share && p0->window <= kTab16Window);
+        const bool banded = narrow || (has_pieces && waits_for_longest(qlen_at(i)) && p0->window <= kTab16Window);
         if (pl.queue) {
             const bool smem = pl.lay.query_smem_bytes != 0;
             const Words words = pl.lay.words;
