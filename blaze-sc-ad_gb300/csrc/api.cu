@@ -1267,6 +1267,7 @@ extern "C" int blaze_prelim_search(blaze_search *s, const uint8_t *query, int32_
     r.p = p;
     rc = run_search(s, r, n_hsps);
     s->stats.h2d_bytes += q.upload_bytes;
+    s->stats.kernel_launches += kLookupKernels;
     if (rc != BLAZE_OK) return rc;
     wait.on = false;  // the search has waited
     return blaze_search_results(s, out, capacity, n_hsps);

@@ -370,6 +370,7 @@ cudaError_t gapped_occupancy(int *blocks_per_sm);
 cudaError_t launch_gapped_split(const GappedArgs &a, int n_blocks, int n_sm, cudaStream_t st);
 
 // The lookups of n queries: `many` (a device array), or `one` when it is null.
+constexpr uint32_t kLookupKernels = 3;  // of a launch
 cudaError_t launch_lookup(const LookupQuery &one, const LookupQuery *many, uint32_t n, int32_t threshold,
                           cudaStream_t st);
 

@@ -111,7 +111,7 @@ typedef struct blaze_stats {
     float scan_ms;   /* word finder + ungapped kernel */
     float gapped_ms; /* gapped kernel */
     float device_ms; /* first to last device operation of the run, all passes */
-    uint32_t kernel_launches; /* kernels launched by the run, all passes */
+    uint32_t kernel_launches; /* kernels launched by the run, all passes (blaze_prelim_search: its lookup too) */
     uint64_t h2d_bytes; /* host->device bytes of the run (the query's residues included) */
     uint64_t d2h_bytes; /* device->host bytes of the run */
     uint32_t graph_replays; /* passes launched from an already built CUDA graph */
