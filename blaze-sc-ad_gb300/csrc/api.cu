@@ -114,19 +114,22 @@ extern "C" int blaze_db_create(int device, const uint8_t *residues, const uint64
 
 int db_make_groups(blaze_db *db) {
     const std::vector<uint64_t> &off = db->h_off;
-    // A group holds twice a warp's share of the residues that are left (152 x 32
-    // warps), at most what a warp stages: what a group costs beyond its residues
+    // A group holds twice a warp's share of the residues that are left (32 warps
+    // an SM), at most what a warp stages: what a group costs beyond its residues
     // -- fetching it, its last partial batches and extensions -- is spread over
     // more of them, and the last groups are small, so that the warps end about
     // together. 300 query residues against 14 / 35 / 140 M: 0.183 / 0.329 / 1.013
     // ms with 1/16 of a warp's share of all residues, 0.140 / 0.261 / 0.983 so.
-    constexpr uint64_t kWarps = 152 * 32, kLeast = 512;
-    const uint64_t least = std::min<uint64_t>(kLeast, db->total / kWarps);
+    constexpr uint64_t kLeast = 512;
+    int n_sm = 0;
+    BLAZE_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, db->device));
+    const uint64_t warps = static_cast<uint64_t>(n_sm) * kScanMaxWarpsPerBlock;
+    const uint64_t least = std::min<uint64_t>(kLeast, db->total / warps);
     auto cut = [&](uint64_t at_least, std::vector<uint32_t> &b) {  // returns the bytes of the largest group of several
         uint32_t largest = 0;
         b.assign(1, db->n);
         for (uint32_t hi = db->n; hi > 0;) {
-            const uint64_t most = std::min<uint64_t>(std::max<uint64_t>(2 * off[hi] / kWarps, at_least), kGroupMaxBytes);
+            const uint64_t most = std::min<uint64_t>(std::max<uint64_t>(2 * off[hi] / warps, at_least), kGroupMaxBytes);
             uint32_t lo = hi - 1;
             while (lo > 0 && hi - lo < kGroupMaxSubjects &&
                    off[hi] - off[lo - 1] + kGroupSubjectBytes * (hi - lo + 1) <= most)
@@ -145,7 +148,7 @@ int db_make_groups(blaze_db *db) {
     // residues (with what precedes it in its first 16 bytes), other groups are
     // one piece. (4,000 residues against 500 subjects: 0.21 ms with pieces of
     // 128, 0.35 of 512, 0.52 of 2,240.)
-    const uint64_t piece = std::min<uint64_t>(std::max<uint64_t>(db->total / kWarps, kPieceLeast), kPieceMost);
+    const uint64_t piece = std::min<uint64_t>(std::max<uint64_t>(db->total / warps, kPieceLeast), kPieceMost);
     std::vector<uint32_t> pieces(1, 0u);
     for (size_t g = 0; g + 1 < b.size(); ++g) {
         const uint64_t len = b[g] - b[g + 1] == 1 ? off[b[g]] - off[b[g + 1]] : 0;
@@ -381,7 +384,6 @@ struct RunSpec {
     std::vector<uint32_t> border;  // batched: query indices in launch (length) order
 };
 
-// One pass of both stages; fills s->h_cnt.
 // One pass's launch sequence: counter reset, scan kernel, gapped kernel and
 // the counter read-back, with the timing events between them.
 struct ScanLaunch {
