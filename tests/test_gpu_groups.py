@@ -1,8 +1,9 @@
 """The word finder's groups of subjects and its two kinds of diagonal table,
 against the oracle: subject lengths at the edges of the staging blocks and of
 the scanned chunks, groups of the most subjects, subjects long enough that a
-16-bit table has to be moved down, query lengths and windows on both sides of
-the 16-bit limit, and the batched launch chosen by the longest subject."""
+16-bit table has to be moved down, windows on both sides of the 16-bit limit
+(query lengths at it: test_gpu_table_limits.py), queries in bands, and the batched
+launch chosen by the longest subject."""
 import numpy as np
 import pytest
 

@@ -1,5 +1,5 @@
 """The word lookup built on the device, against the oracle: query lengths around
-a word and around the staged tile, the longest query, thresholds from "nearly
+a word and around the parts of 256 offsets, the longest query, thresholds from "nearly
 every word" (cells of more than 255 offsets) to "the exact word only", in the
 plain, one-call and batched forms."""
 import numpy as np

@@ -200,7 +200,8 @@ def test_invalid_inputs_rejected():
 
 
 def test_query_longer_than_shared_copy():
-    # queries above 8192 residues are read from global memory by the word finder
+    # a long query: in bands with a table of one band's diagonals (above 14,336
+    # residues, where the query is read from global memory: test_gpu_bands.py)
     rng = np.random.default_rng(9000)
     q = synth.random_residues(rng, 9000)
     seqs = [synth.random_residues(rng, int(L)) for L in synth.lognormal_lengths(rng, 300, 250, 0.82, 30, 3000)]

@@ -30,7 +30,7 @@ def make_case(rng):
         qlen = int(np.clip(rng.lognormal(np.log(300), 0.7), 12, 3000))
     elif r < 0.95:
         qlen = int(rng.integers(3000, 8200))
-    else:  # longer than the shared-memory copy of the query
+    else:  # in bands with a table of one band's diagonals
         qlen = int(rng.integers(8193, 12000))
     q = synth.random_residues(rng, qlen)
     n = int(rng.choice([1, 2, 7, 50, 300, 1500]))

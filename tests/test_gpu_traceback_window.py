@@ -1,8 +1,10 @@
 """The traceback stage's DP with its band in registers, and where it gives way to
 the one with rows in memory, against the oracle: query lengths around the 32
-cells that the walk back takes at once, X-drops whose first row just fits the
-256 columns of registers and just does not, alignments with long gaps, and
-direction buffers of odd and tiny sizes."""
+cells that the walk back takes at once, X-drops whose first row (X-drop - 10
+columns at gap costs 11/1) just fits the 192 columns of registers and just does
+not, alignments with long gaps, and direction buffers of odd and tiny sizes. Which
+form a call takes first goes by the X-drop; both sides of that line are in
+test_gpu_traceback_forms.py."""
 import numpy as np
 import pytest
 
